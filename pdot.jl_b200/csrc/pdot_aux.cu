@@ -15,38 +15,26 @@ namespace pdot {
 namespace {
 
 constexpr int kAuxThreads = 256;
-constexpr int kColChunk = 64;  // columns per CTA of the strided (row) sums
+constexpr int kAuxWarps = kAuxThreads / 32;
+constexpr int kColChunk = 64;  // columns per CTA of a warm-start plan's row sums
 
-// Row sums, stage one: CTA (rb, cb) sums columns [cb*kColChunk, ...) for rows
-// rb*256 + t; partial[cb * m + i]. Consecutive threads read consecutive rows.
-__global__ void k_row_partials(int64_t m, int64_t n, const double* __restrict__ X, double* __restrict__ part) {
-  const int64_t i = (int64_t)blockIdx.x * kAuxThreads + threadIdx.x;
-  const int64_t j0 = (int64_t)blockIdx.y * kColChunk;
-  const int64_t j1 = (j0 + kColChunk < n) ? j0 + kColChunk : n;
-  if (i >= m) return;
-  double s = 0.0;
-  for (int64_t j = j0; j < j1; ++j) s += X[i + j * m];
-  part[(int64_t)blockIdx.y * m + i] = s;
-}
-
-// Column sums: one CTA per column, a fixed-order tree over the contiguous rows.
-__global__ void k_col_sums(int64_t m, const double* __restrict__ X, double* __restrict__ out) {
-  __shared__ double sh[kAuxThreads];
-  const int64_t j = blockIdx.x;
-  double s = 0.0;
-  for (int64_t i = threadIdx.x; i < m; i += kAuxThreads) s += X[i + j * m];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = kAuxThreads / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[j] = sh[0];
+__device__ __forceinline__ double aux_warp_sum(double x) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
 }
 
 __device__ __forceinline__ double row_sum(const double* part, int64_t m, int chunks, int64_t i) {
   double s = 0.0;
-  for (int c = 0; c < chunks; ++c) s += part[(int64_t)c * m + i];
+  int c = 0;
+  for (; c + 8 <= chunks; c += 8) {  // eight loads in flight ahead of the ordered additions
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = part[(int64_t)(c + k) * m + i];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s += v[k];
+  }
+  for (; c < chunks; ++c) s += part[(int64_t)c * m + i];
   return s;
 }
 
@@ -57,97 +45,325 @@ __device__ __forceinline__ double scale_of(double dist, double sum) {
   return t < 1.0 ? t : 1.0;
 }
 
-__global__ void k_row_scales(int64_t m, int chunks, const double* __restrict__ part, const double* __restrict__ a,
-                             double* __restrict__ scale) {
-  const int64_t i = (int64_t)blockIdx.x * kAuxThreads + threadIdx.x;
-  if (i < m) scale[i] = scale_of(a[i], row_sum(part, m, chunks, i));
+// ---- rounding ----------------------------------------------------------------
+// The scaled plans are never stored: each pass recomputes rs_i * X and
+// cs_j * (rs_i * X) from X, rounding each product as the stored form would, so
+// rounding streams the plan four times in and once out (40 B per entry: the row
+// sums, the column sums of the row-scaled plan, both sums of the scaled plan,
+// the write). With the scaled plans written back in place it was 80 B per entry
+// and 11 launches: 10000 x 10000 took 1.75 ms of device time on B200, now the
+// four passes take 0.64 ms of their 0.61 ms at the copy peak (measured below).
+//
+// CTA (p, c) of a summing pass covers panel p (kRoundRows rows) of column chunk c; a
+// warp takes whole columns of the panel, lane rows in R-wide loads, so a column
+// partial is one shuffle tree and row partials stay in registers until the chunk ends.
+constexpr int kRoundRows = 256;
+enum { kRoundRow = 1, kRoundCol = 2, kRoundRowScaled = 4, kRoundColScaled = 8 };
+
+template <int R>
+__device__ __forceinline__ void load_rows(const double* p, double (&v)[R]) {
+  if constexpr (R == 2) {
+    const double2 t = *reinterpret_cast<const double2*>(p);
+    v[0] = t.x;
+    v[1] = t.y;
+  } else {
+    v[0] = *p;
+  }
+}
+template <int R>
+__device__ __forceinline__ void store_rows(double* p, const double (&v)[R]) {
+  if constexpr (R == 2)
+    *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+  else
+    *p = v[0];
 }
 
-__global__ void k_col_scales(int64_t n, const double* __restrict__ sums, const double* __restrict__ b,
-                             double* __restrict__ scale) {
-  const int64_t j = (int64_t)blockIdx.x * kAuxThreads + threadIdx.x;
-  if (j < n) scale[j] = scale_of(b[j], sums[j]);
-}
-
-// X_ij *= row_scale_i (by_row) or col_scale_j
-__global__ void k_scale(int64_t m, int64_t n, double* __restrict__ X, const double* __restrict__ scale, int by_row) {
-  const int64_t N = m * n;
-  for (int64_t e = (int64_t)blockIdx.x * kAuxThreads + threadIdx.x; e < N; e += (int64_t)gridDim.x * kAuxThreads) {
-    const int64_t j = e / m, i = e - j * m;
-    X[e] = __dmul_rn(by_row ? scale[i] : scale[j], X[e]);
+template <int R, int MODE>
+__global__ void __launch_bounds__(kAuxThreads, 3)
+    k_round_sums(int64_t m, int64_t n, int64_t chunk, const double* __restrict__ X, const double* __restrict__ rscale,
+                 const double* __restrict__ cscale, double* __restrict__ rowpart, double* __restrict__ colpart) {
+  constexpr int RPL = kRoundRows / (32 * R);
+  __shared__ double red[(MODE & kRoundRow) ? kAuxWarps : 1][(MODE & kRoundRow) ? kRoundRows : 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t row0 = (int64_t)blockIdx.x * kRoundRows;
+  const int64_t j0 = (int64_t)blockIdx.y * chunk, j1 = (j0 + chunk < n) ? j0 + chunk : n;
+  double acc[RPL][R], rs[RPL][R];
+  bool ok[RPL];
+#pragma unroll
+  for (int k = 0; k < RPL; ++k) {
+    const int64_t i = row0 + k * 32 * R + lane * R;
+    ok[k] = i < m;  // R divides m on the R-wide path
+#pragma unroll
+    for (int e = 0; e < R; ++e) {
+      acc[k][e] = 0.0;
+      rs[k][e] = ((MODE & kRoundRowScaled) && ok[k]) ? rscale[i + e] : 1.0;
+    }
+  }
+  for (int64_t j = j0 + warp; j < j1; j += kAuxWarps) {
+    const double cs = (MODE & kRoundColScaled) ? cscale[j] : 1.0;
+    double x[RPL][R];
+#pragma unroll
+    for (int k = 0; k < RPL; ++k)
+      if (ok[k]) load_rows<R>(X + j * m + row0 + k * 32 * R + lane * R, x[k]);
+    double col = 0.0;
+#pragma unroll
+    for (int k = 0; k < RPL; ++k)
+      if (ok[k]) {
+#pragma unroll
+        for (int e = 0; e < R; ++e) {
+          double y = x[k][e];
+          if (MODE & kRoundRowScaled) y = __dmul_rn(rs[k][e], y);
+          if (MODE & kRoundColScaled) y = __dmul_rn(cs, y);
+          if (MODE & kRoundRow) acc[k][e] += y;
+          if (MODE & kRoundCol) col += y;
+        }
+      }
+    if (MODE & kRoundCol) {
+      col = aux_warp_sum(col);
+      if (lane == 0) colpart[(int64_t)blockIdx.x * n + j] = col;
+    }
+  }
+  if constexpr ((MODE & kRoundRow) != 0) {
+#pragma unroll
+    for (int k = 0; k < RPL; ++k)
+#pragma unroll
+      for (int e = 0; e < R; ++e) red[warp][k * 32 * R + lane * R + e] = acc[k][e];
+    __syncthreads();
+    const int64_t i = row0 + threadIdx.x;
+    if (i < m) {
+      double s = red[0][threadIdx.x];
+#pragma unroll
+      for (int w = 1; w < kAuxWarps; ++w) s += red[w][threadIdx.x];
+      rowpart[(int64_t)blockIdx.y * m + i] = s;
+    }
   }
 }
 
-// err_r = a - rowsum
-__global__ void k_err_rows(int64_t m, int chunks, const double* __restrict__ part, const double* __restrict__ a,
-                           double* __restrict__ er) {
+// scale_i = min(1, dist_i / sum of the `parts` partials of i)
+__global__ void k_round_scales(int64_t count, int parts, const double* __restrict__ part,
+                               const double* __restrict__ dist, double* __restrict__ scale) {
   const int64_t i = (int64_t)blockIdx.x * kAuxThreads + threadIdx.x;
-  if (i < m) er[i] = __dsub_rn(a[i], row_sum(part, m, chunks, i));
+  if (i < count) scale[i] = scale_of(dist[i], row_sum(part, count, parts, i));
 }
 
-// ||err_r||_1 in one CTA (fixed order)
-__global__ void k_norm1(int64_t m, const double* __restrict__ er, double* __restrict__ norm1) {
+// err_r = a - rowsum and err_c = b - colsum of the scaled plan; block `bid` of the
+// row blocks also leaves its share of ||err_r||_1 (a fixed-order tree).
+__global__ void k_round_errors(int64_t m, int64_t n, int row_blocks, int chunks, int panels,
+                               const double* __restrict__ rowpart, const double* __restrict__ colpart,
+                               const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ er,
+                               double* __restrict__ ec, double* __restrict__ normpart) {
+  if ((int)blockIdx.x >= row_blocks) {
+    const int64_t j = (int64_t)(blockIdx.x - row_blocks) * kAuxThreads + threadIdx.x;
+    if (j < n) ec[j] = __dsub_rn(b[j], row_sum(colpart, n, panels, j));
+    return;
+  }
   __shared__ double sh[kAuxThreads];
-  double s = 0.0;
-  for (int64_t i = threadIdx.x; i < m; i += kAuxThreads) s += fabs(er[i]);
-  sh[threadIdx.x] = s;
+  const int64_t i = (int64_t)blockIdx.x * kAuxThreads + threadIdx.x;
+  double e = 0.0;
+  if (i < m) er[i] = e = __dsub_rn(a[i], row_sum(rowpart, m, chunks, i));
+  sh[threadIdx.x] = fabs(e);
   __syncthreads();
   for (int w = kAuxThreads / 2; w > 0; w >>= 1) {
     if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *norm1 = sh[0];
+  if (threadIdx.x == 0) normpart[blockIdx.x] = sh[0];
 }
 
-// X += (err_r / ||err_r||_1) * (b - colsum)^T
-__global__ void k_rank_one(int64_t m, int64_t n, double* __restrict__ X, const double* __restrict__ er,
-                           const double* __restrict__ norm1, const double* __restrict__ colsum,
-                           const double* __restrict__ b) {
-  const double nrm = *norm1;
-  const int64_t N = m * n;
-  for (int64_t e = (int64_t)blockIdx.x * kAuxThreads + threadIdx.x; e < N; e += (int64_t)gridDim.x * kAuxThreads) {
-    const int64_t j = e / m, i = e - j * m;
-    const double r = nrm != 0.0 ? __ddiv_rn(er[i], nrm) : er[i];
-    const double c = __dsub_rn(b[j], colsum[j]);
-    X[e] = __dadd_rn(X[e], __dmul_rn(r, c));
+// X = cs_j * (rs_i * X) + (err_r / ||err_r||_1) * err_c^T. A thread keeps R rows and
+// walks the columns of its chunk, four loads in flight.
+template <int R>
+__global__ void __launch_bounds__(kAuxThreads)
+    k_round_write(int64_t m, int64_t n, int64_t chunk, double* __restrict__ X, const double* __restrict__ rscale,
+                  const double* __restrict__ cscale, const double* __restrict__ er, const double* __restrict__ ec,
+                  const double* __restrict__ normpart, int norm_blocks) {
+  __shared__ double norm;
+  if (threadIdx.x < 32) {
+    double s = 0.0;
+    for (int k = threadIdx.x; k < norm_blocks; k += 32) s += normpart[k];
+    s = aux_warp_sum(s);
+    if (threadIdx.x == 0) norm = s;
+  }
+  __syncthreads();
+  const double nrm = norm;
+  const int64_t i = ((int64_t)blockIdx.x * kAuxThreads + threadIdx.x) * R;
+  if (i >= m) return;
+  double rs[R], r[R];
+#pragma unroll
+  for (int e = 0; e < R; ++e) {
+    rs[e] = rscale[i + e];
+    r[e] = nrm != 0.0 ? __ddiv_rn(er[i + e], nrm) : er[i + e];
+  }
+  const int64_t j0 = (int64_t)blockIdx.y * chunk, j1 = (j0 + chunk < n) ? j0 + chunk : n;
+  constexpr int U = 4;
+  for (int64_t j = j0; j < j1; j += U) {
+    double x[U][R];
+#pragma unroll
+    for (int k = 0; k < U; ++k)
+      if (j + k < j1) load_rows<R>(X + (j + k) * m + i, x[k]);
+#pragma unroll
+    for (int k = 0; k < U; ++k)
+      if (j + k < j1) {
+        const double cs = cscale[j + k], c = ec[j + k];
+#pragma unroll
+        for (int e = 0; e < R; ++e)
+          x[k][e] = __dadd_rn(__dmul_rn(cs, __dmul_rn(rs[e], x[k][e])), __dmul_rn(r[e], c));
+        store_rows<R>(X + (j + k) * m + i, x[k]);
+      }
   }
 }
 
-// C_ij = ||x_i - y_j||^2 in FP64, then divided by its maximum when `normalise`.
-__global__ void k_sqeuclid(int64_t m, int64_t n, int dim, const double* __restrict__ xs,
-                           const double* __restrict__ ys, double* __restrict__ C) {
-  const int64_t N = m * n;
-  for (int64_t e = (int64_t)blockIdx.x * kAuxThreads + threadIdx.x; e < N; e += (int64_t)gridDim.x * kAuxThreads) {
-    const int64_t j = e / m, i = e - j * m;
-    double s = 0.0;
-    for (int d = 0; d < dim; ++d) {
-      const double t = __dsub_rn(xs[i * dim + d], ys[j * dim + d]);
+// ---- the squared-Euclidean cost ------------------------------------------------
+// C_ij = ||x_i - y_j||^2 in FP64, divided by its maximum when `normalise`. The
+// maximum is taken from the points, nothing stored, and the cost is then written
+// once (8 B per entry); stored first, scanned and divided in place it took 32 B per
+// entry: 0.93 ms at 10000 x 10000 in three dimensions on B200.
+//
+// DIM 1..4 are compiled in, 0 is any dimension (coordinates from global memory).
+constexpr int kCostRows = 2;  // rows per thread of the write
+template <int DIM>
+__device__ __forceinline__ double sq_distance(const double* xi, const double* yj, int dim) {
+  double s = 0.0;
+  if constexpr (DIM > 0) {
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      const double t = __dsub_rn(xi[d], yj[d]);
       s = __dadd_rn(s, __dmul_rn(t, t));
     }
-    C[e] = s;
+  } else {
+    for (int d = 0; d < dim; ++d) {
+      const double t = __dsub_rn(xi[d], yj[d]);
+      s = __dadd_rn(s, __dmul_rn(t, t));
+    }
   }
+  return s;
 }
 
-__global__ void k_max_partials(int64_t N, const double* __restrict__ C, double* __restrict__ part) {
-  __shared__ double sh[kAuxThreads];
-  double mx = 0.0;
-  for (int64_t e = (int64_t)blockIdx.x * kAuxThreads + threadIdx.x; e < N; e += (int64_t)gridDim.x * kAuxThreads)
-    mx = fmax(mx, C[e]);
-  sh[threadIdx.x] = mx;
+// v / mx rounded to nearest for one divisor and many v. With y the correctly rounded
+// 1 / mx and q a quotient within one ulp, q + (v - q mx) y, its residual exact by one
+// fused multiply-add, is the correctly rounded quotient (Markstein, IBM J. Res. Dev.
+// 34, 1990). v y can be 1.5 ulp off, so a first such correction makes it a q within
+// one ulp and a second takes the theorem. The bounds on mx and v keep every term in
+// the normal range; v = 0 gives 0, and everything else, NaNs among it, takes the
+// division itself. Five operations in place of a division an entry.
+struct DivideBy {
+  double mx, y;
+  bool usable;
+  __device__ __forceinline__ explicit DivideBy(double m) : mx(m) {
+    usable = m >= 0x1p-400 && m <= 0x1p+400;
+    y = usable ? __drcp_rn(m) : 0.0;
+  }
+  __device__ __forceinline__ double operator()(double v) const {
+    if (usable && (v == 0.0 || (v >= 0x1p-500 && v <= mx))) {
+      double q = __dmul_rn(v, y);
+      q = __fma_rn(__fma_rn(-q, mx, v), y, q);
+      return __fma_rn(__fma_rn(-q, mx, v), y, q);
+    }
+    return __ddiv_rn(v, mx);
+  }
+};
+
+// The largest entry (NaNs ignored), at least 0, by an atomicMax on its bits
+// (non-negative doubles order as their bits do).
+template <int DIM>
+__global__ void __launch_bounds__(kAuxThreads)
+    k_sqeuclid_max(int64_t m, int64_t n, int dim, int64_t chunk, const double* __restrict__ xs,
+                   const double* __restrict__ ys, unsigned long long* __restrict__ out) {
+  constexpr int Q = 4;  // rows per thread: a column's coordinates serve four distances
+  constexpr int D = DIM > 0 ? DIM : 1;
+  const int64_t i0 = (int64_t)blockIdx.x * kAuxThreads * Q + threadIdx.x;
+  double x[Q][D], mx[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    mx[q] = 0.0;
+    if constexpr (DIM > 0) {
+      const int64_t i = i0 + q * kAuxThreads;
+#pragma unroll
+      for (int d = 0; d < D; ++d) x[q][d] = i < m ? xs[i * DIM + d] : 0.0;
+    }
+  }
+  const int64_t j0 = (int64_t)blockIdx.y * chunk, j1 = (j0 + chunk < n) ? j0 + chunk : n;
+#pragma unroll 2
+  for (int64_t j = j0; j < j1; ++j) {
+    if constexpr (DIM > 0) {
+      double y[D];
+#pragma unroll
+      for (int d = 0; d < D; ++d) y[d] = __ldg(ys + j * DIM + d);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) mx[q] = fmax(mx[q], sq_distance<DIM>(x[q], y, dim));
+    } else {
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int64_t i = i0 + q * kAuxThreads;
+        if (i < m) mx[q] = fmax(mx[q], sq_distance<0>(xs + i * dim, ys + j * dim, dim));
+      }
+    }
+  }
+  double best = 0.0;
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+    if (i0 + q * kAuxThreads < m) best = fmax(best, mx[q]);
+  __shared__ double sh[kAuxWarps];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) best = fmax(best, __shfl_xor_sync(0xffffffffu, best, o));
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = best;
   __syncthreads();
-  for (int w = kAuxThreads / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sh[threadIdx.x] = fmax(sh[threadIdx.x], sh[threadIdx.x + w]);
-    __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < kAuxWarps; ++w) best = fmax(best, sh[w]);
+    atomicMax(out, (unsigned long long)__double_as_longlong(best));
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-__global__ void k_divide_by_max(int64_t N, double* __restrict__ C, const double* __restrict__ part, int parts) {
-  double mx = 0.0;
-  for (int k = 0; k < parts; ++k) mx = fmax(mx, part[k]);
-  if (!(mx > 0.0)) return;
-  for (int64_t e = (int64_t)blockIdx.x * kAuxThreads + threadIdx.x; e < N; e += (int64_t)gridDim.x * kAuxThreads)
-    C[e] = __ddiv_rn(C[e], mx);
+// The cost's entries of a CTA's rows and column chunk, divided by *top when it is
+// given and positive. Entry 0, where *top lies, is left to k_sqeuclid_first.
+template <int DIM, int R>
+__global__ void __launch_bounds__(kAuxThreads)
+    k_sqeuclid_write(int64_t m, int64_t n, int dim, int64_t chunk, const double* __restrict__ xs,
+                     const double* __restrict__ ys, const double* top, double* C) {
+  constexpr int D = DIM > 0 ? DIM : 1;
+  const double mx = top ? *top : 0.0;
+  const DivideBy by(mx);
+  const int64_t i = ((int64_t)blockIdx.x * kAuxThreads + threadIdx.x) * R;
+  if (i >= m) return;
+  double x[R][D];
+  if constexpr (DIM > 0) {
+#pragma unroll
+    for (int e = 0; e < R; ++e)
+#pragma unroll
+      for (int d = 0; d < D; ++d) x[e][d] = xs[(i + e) * DIM + d];
+  }
+  const int64_t j0 = (int64_t)blockIdx.y * chunk, j1 = (j0 + chunk < n) ? j0 + chunk : n;
+#pragma unroll 2
+  for (int64_t j = j0; j < j1; ++j) {
+    double v[R];
+    if constexpr (DIM > 0) {
+      double y[D];
+#pragma unroll
+      for (int d = 0; d < D; ++d) y[d] = __ldg(ys + j * DIM + d);
+#pragma unroll
+      for (int e = 0; e < R; ++e) v[e] = sq_distance<DIM>(x[e], y, dim);
+    } else {
+#pragma unroll
+      for (int e = 0; e < R; ++e) v[e] = sq_distance<0>(xs + (i + e) * dim, ys + j * dim, dim);
+    }
+    if (mx > 0.0) {
+#pragma unroll
+      for (int e = 0; e < R; ++e) v[e] = by(v[e]);
+    }
+    if (top && i == 0 && j == 0) {
+      if constexpr (R == 2) C[1] = v[1];
+    } else {
+      store_rows<R>(C + j * m + i, v);
+    }
+  }
+}
+
+// Entry 0 in the place of the maximum that it held.
+__global__ void k_sqeuclid_first(int dim, const double* __restrict__ xs, const double* __restrict__ ys,
+                                 double* C) {
+  const double mx = C[0], v = sq_distance<0>(xs, ys, dim);
+  C[0] = mx > 0.0 ? __ddiv_rn(v, mx) : v;
 }
 
 // Row and column sums of a plan in storage type TX (the sums of a warm-start
@@ -184,41 +400,98 @@ __global__ void k_plan_row_totals(int64_t m, int chunks, const double* __restric
   if (i < m) r[i] = row_sum(part, m, chunks, i);
 }
 
-int grid_for(int64_t count) {
-  int64_t g = (count + kAuxThreads - 1) / kAuxThreads;
-  return (int)(g < 1 ? 1 : (g > 148 * 16 ? 148 * 16 : g));
+// Columns per CTA so that `strips` row strips times the chunks make about `target` CTAs,
+// each with at least `least` columns.
+int64_t column_chunk(int64_t n, int64_t strips, int64_t target, int64_t least) {
+  const int64_t want = (target + strips - 1) / strips;
+  const int64_t chunk = (n + want - 1) / want;
+  const int64_t c = chunk < least ? least : chunk;
+  return (n + c - 1) / c <= 65535 ? c : (n + 65534) / 65535;
+}
+
+struct RoundShape {
+  int64_t panels, chunk, chunks, strips, wchunk;
+  int rb, cb;
+};
+// About 16 CTAs per SM of the summing passes (3 resident): the ragged last
+// panel's short CTAs then even out. A chunk has at least 4 columns per warp, so
+// that the row partials stay below 1/32 of the plan.
+RoundShape round_shape(int64_t m, int64_t n, int R) {
+  RoundShape g;
+  g.panels = (m + kRoundRows - 1) / kRoundRows;
+  g.chunk = column_chunk(n, g.panels, 148 * 16, 32);
+  g.chunks = (n + g.chunk - 1) / g.chunk;
+  g.strips = (m + kAuxThreads * R - 1) / (kAuxThreads * R);
+  g.wchunk = column_chunk(n, g.strips, 148 * 32, 8);
+  g.rb = (int)((m + kAuxThreads - 1) / kAuxThreads);
+  g.cb = (int)((n + kAuxThreads - 1) / kAuxThreads);
+  return g;
+}
+
+template <int R>
+cudaError_t rounding_passes(int64_t m, int64_t n, const double* a, const double* b, double* X, double* work,
+                            cudaStream_t s) {
+  const RoundShape g = round_shape(m, n, R);
+  double* rowpart = work;
+  double* colpart = rowpart + (size_t)g.chunks * m;
+  double* rscale = colpart + (size_t)g.panels * n;
+  double* cscale = rscale + m;
+  double* er = cscale + n;
+  double* ec = er + m;
+  double* normpart = ec + n;
+  const dim3 grid((unsigned)g.panels, (unsigned)g.chunks);
+  const dim3 wgrid((unsigned)g.strips, (unsigned)((n + g.wchunk - 1) / g.wchunk));
+  k_round_sums<R, kRoundRow><<<grid, kAuxThreads, 0, s>>>(m, n, g.chunk, X, nullptr, nullptr, rowpart, colpart);
+  k_round_scales<<<g.rb, kAuxThreads, 0, s>>>(m, (int)g.chunks, rowpart, a, rscale);
+  k_round_sums<R, kRoundCol | kRoundRowScaled>
+      <<<grid, kAuxThreads, 0, s>>>(m, n, g.chunk, X, rscale, nullptr, rowpart, colpart);
+  k_round_scales<<<g.cb, kAuxThreads, 0, s>>>(n, (int)g.panels, colpart, b, cscale);
+  k_round_sums<R, kRoundRow | kRoundCol | kRoundRowScaled | kRoundColScaled>
+      <<<grid, kAuxThreads, 0, s>>>(m, n, g.chunk, X, rscale, cscale, rowpart, colpart);
+  k_round_errors<<<g.rb + g.cb, kAuxThreads, 0, s>>>(m, n, g.rb, (int)g.chunks, (int)g.panels, rowpart, colpart, a, b,
+                                                     er, ec, normpart);
+  k_round_write<R><<<wgrid, kAuxThreads, 0, s>>>(m, n, g.wchunk, X, rscale, cscale, er, ec, normpart, g.rb);
+  return cudaGetLastError();
+}
+
+template <int DIM>
+cudaError_t sqeuclid_passes(int64_t m, int64_t n, int dim, const double* xs, const double* ys, int normalise, double* C,
+                            cudaStream_t s) {
+  double* top = nullptr;
+  if (normalise) {
+    top = C;
+    cudaError_t e = cudaMemsetAsync(top, 0, sizeof(double), s);
+    if (e != cudaSuccess) return e;
+    const int64_t strips = (m + kAuxThreads * 4 - 1) / (kAuxThreads * 4);
+    const int64_t chunk = column_chunk(n, strips, 148 * 16, 16);
+    k_sqeuclid_max<DIM><<<dim3((unsigned)strips, (unsigned)((n + chunk - 1) / chunk)), kAuxThreads, 0, s>>>(
+        m, n, dim, chunk, xs, ys, reinterpret_cast<unsigned long long*>(top));
+  }
+  const bool wide = m % kCostRows == 0 && (reinterpret_cast<uintptr_t>(C) & 15u) == 0;
+  const int R = wide ? kCostRows : 1;
+  const int64_t strips = (m + kAuxThreads * R - 1) / (kAuxThreads * R);
+  const int64_t chunk = column_chunk(n, strips, 148 * 32, 8);
+  const dim3 grid((unsigned)strips, (unsigned)((n + chunk - 1) / chunk));
+  if (wide)
+    k_sqeuclid_write<DIM, kCostRows><<<grid, kAuxThreads, 0, s>>>(m, n, dim, chunk, xs, ys, top, C);
+  else
+    k_sqeuclid_write<DIM, 1><<<grid, kAuxThreads, 0, s>>>(m, n, dim, chunk, xs, ys, top, C);
+  if (normalise) k_sqeuclid_first<<<1, 1, 0, s>>>(dim, xs, ys, C);
+  return cudaGetLastError();
 }
 
 }  // namespace
 
 size_t rounding_workspace_doubles(int64_t m, int64_t n) {
-  const int64_t chunks = (n + kColChunk - 1) / kColChunk;
-  return (size_t)chunks * m + 2 * (size_t)m + 2 * (size_t)n + 1;
+  const RoundShape g = round_shape(m, n, 1);  // the sums' shape does not depend on the load width
+  return (size_t)g.chunks * m + (size_t)g.panels * n + 2 * (size_t)m + 2 * (size_t)n + g.rb;
 }
 
 cudaError_t launch_rounding(int64_t m, int64_t n, const double* a, const double* b, double* X, double* work,
                             cudaStream_t s) {
-  const int chunks = (int)((n + kColChunk - 1) / kColChunk);
-  double* part = work;
-  double* rscale = part + (size_t)chunks * m;  // row scales, later err_r
-  double* colsum = rscale + m;                 // column sums
-  double* cscale = colsum + n;
-  double* norm1 = cscale + n;
-  const dim3 rgrid((unsigned)((m + kAuxThreads - 1) / kAuxThreads), (unsigned)chunks);
-  const int rb = (int)((m + kAuxThreads - 1) / kAuxThreads), cbk = (int)((n + kAuxThreads - 1) / kAuxThreads);
-  const int eg = grid_for(m * n);
-  k_row_partials<<<rgrid, kAuxThreads, 0, s>>>(m, n, X, part);
-  k_row_scales<<<rb, kAuxThreads, 0, s>>>(m, chunks, part, a, rscale);
-  k_scale<<<eg, kAuxThreads, 0, s>>>(m, n, X, rscale, 1);
-  k_col_sums<<<(unsigned)n, kAuxThreads, 0, s>>>(m, X, colsum);
-  k_col_scales<<<cbk, kAuxThreads, 0, s>>>(n, colsum, b, cscale);
-  k_scale<<<eg, kAuxThreads, 0, s>>>(m, n, X, cscale, 0);
-  k_row_partials<<<rgrid, kAuxThreads, 0, s>>>(m, n, X, part);
-  k_err_rows<<<rb, kAuxThreads, 0, s>>>(m, chunks, part, a, rscale);
-  k_norm1<<<1, kAuxThreads, 0, s>>>(m, rscale, norm1);
-  k_col_sums<<<(unsigned)n, kAuxThreads, 0, s>>>(m, X, colsum);
-  k_rank_one<<<eg, kAuxThreads, 0, s>>>(m, n, X, rscale, norm1, colsum, b);
-  return cudaGetLastError();
+  // 16-byte loads where every column starts on a 16-byte boundary
+  if (m % 2 == 0 && (reinterpret_cast<uintptr_t>(X) & 15u) == 0) return rounding_passes<2>(m, n, a, b, X, work, s);
+  return rounding_passes<1>(m, n, a, b, X, work, s);
 }
 
 size_t plan_sums_workspace_doubles(int64_t m, int64_t n) {
@@ -241,19 +514,15 @@ cudaError_t launch_plan_sums(int64_t m, int64_t n, const void* X, int plan_f32, 
   return cudaGetLastError();
 }
 
-size_t sqeuclid_workspace_doubles() { return 148 * 4; }
-
 cudaError_t launch_sqeuclid_cost(int64_t m, int64_t n, int dim, const double* xs, const double* ys, int normalise,
-                                 double* C, double* work, cudaStream_t s) {
-  const int64_t N = m * n;
-  const int eg = grid_for(N);
-  k_sqeuclid<<<eg, kAuxThreads, 0, s>>>(m, n, dim, xs, ys, C);
-  if (normalise) {
-    const int parts = 148 * 4;
-    k_max_partials<<<parts, kAuxThreads, 0, s>>>(N, C, work);
-    k_divide_by_max<<<eg, kAuxThreads, 0, s>>>(N, C, work, parts);
+                                 double* C, cudaStream_t s) {
+  switch (dim) {
+    case 1: return sqeuclid_passes<1>(m, n, dim, xs, ys, normalise, C, s);
+    case 2: return sqeuclid_passes<2>(m, n, dim, xs, ys, normalise, C, s);
+    case 3: return sqeuclid_passes<3>(m, n, dim, xs, ys, normalise, C, s);
+    case 4: return sqeuclid_passes<4>(m, n, dim, xs, ys, normalise, C, s);
+    default: return sqeuclid_passes<0>(m, n, dim, xs, ys, normalise, C, s);
   }
-  return cudaGetLastError();
 }
 
 }  // namespace pdot

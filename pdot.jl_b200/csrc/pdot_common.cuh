@@ -228,9 +228,8 @@ cudaError_t launch_plan_sums(int64_t m, int64_t n, const void* X, int plan_f32, 
 size_t rounding_workspace_doubles(int64_t m, int64_t n);
 cudaError_t launch_rounding(int64_t m, int64_t n, const double* a, const double* b, double* X, double* work,
                             cudaStream_t s);
-size_t sqeuclid_workspace_doubles();
 cudaError_t launch_sqeuclid_cost(int64_t m, int64_t n, int dim, const double* xs, const double* ys, int normalise,
-                                 double* C, double* work, cudaStream_t s);
+                                 double* C, cudaStream_t s);
 
 // A warm-start plan recovered from warm duals (pdot_warmplan.cu), for one
 // instance or the concatenated instances of the batched solver.

@@ -16,6 +16,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <stdexcept>
 #include <string>
@@ -245,6 +246,52 @@ struct DeviceTemp {
     return static_cast<T*>(p);
   }
 };
+
+// Stream-ordered scratch of the device-level calls, from a pool of this library on
+// the current device that keeps at most kPoolKeep bytes between calls. The
+// device's default pool gives its memory back at every synchronisation unless
+// the program asked otherwise, so that a call after one paid for mapping its
+// scratch again: 0.5 ms and more, where a small rounding takes 0.03 ms. The
+// allocation is ordered on the stream like any other, so calls of several threads
+// and streams never share a block in use. While a stream is captured the
+// allocation belongs to the graph, as one of cudaMallocAsync does.
+constexpr int kPoolDevices = 64;
+constexpr uint64_t kPoolKeep = uint64_t(32) << 20;
+
+struct ScratchPools {
+  std::mutex mu;
+  cudaMemPool_t pool[kPoolDevices] = {};
+};
+
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
+  static ScratchPools* pools = new ScratchPools;  // never destroyed: the driver may be gone by then
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(s, &capture);
+  if (e != cudaSuccess) return e;
+  int device = 0;
+  if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;
+  if (capture != cudaStreamCaptureStatusNone || device >= kPoolDevices) return cudaMallocAsync(p, bytes, s);
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(pools->mu);
+    pool = pools->pool[device];
+    if (!pool) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.handleTypes = cudaMemHandleTypeNone;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = device;
+      if ((e = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return e;
+      uint64_t keep = kPoolKeep;
+      if ((e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+        cudaMemPoolDestroy(pool);
+        return e;
+      }
+      pools->pool[device] = pool;
+    }
+  }
+  return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
 
 int64_t pass_workspace_bytes(const pdot::Geometry& g) {
   return (int64_t)(pdot::pass_scratch_doubles(g) * sizeof(double));
@@ -1006,7 +1053,7 @@ int pdot_rounding_f64(int64_t m, int64_t n, const double* source, const double* 
     if (!source || !target || !plan) fail(PDOT_ERR_INVALID_ARGUMENT, "null pointer argument");
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
     double* work = nullptr;
-    CK(cudaMallocAsync(reinterpret_cast<void**>(&work), pdot::rounding_workspace_doubles(m, n) * sizeof(double), s));
+    CK(scratch_alloc(reinterpret_cast<void**>(&work), pdot::rounding_workspace_doubles(m, n) * sizeof(double), s));
     const cudaError_t e = pdot::launch_rounding(m, n, source, target, plan, work, s);
     const cudaError_t e2 = cudaFreeAsync(work, s);
     CK(e);
@@ -1046,13 +1093,8 @@ int pdot_sqeuclid_cost_f64(int64_t m, int64_t n, int32_t dim, const double* sour
   return guarded([&] {
     if (m < 1 || n < 1 || dim < 1) fail(PDOT_ERR_INVALID_ARGUMENT, "empty problem");
     if (!source_points || !target_points || !cost) fail(PDOT_ERR_INVALID_ARGUMENT, "null pointer argument");
-    const cudaStream_t s = static_cast<cudaStream_t>(stream);
-    double* work = nullptr;
-    CK(cudaMallocAsync(reinterpret_cast<void**>(&work), pdot::sqeuclid_workspace_doubles() * sizeof(double), s));
-    const cudaError_t e = pdot::launch_sqeuclid_cost(m, n, dim, source_points, target_points, normalise, cost, work, s);
-    const cudaError_t e2 = cudaFreeAsync(work, s);
-    CK(e);
-    CK(e2);
+    CK(pdot::launch_sqeuclid_cost(m, n, dim, source_points, target_points, normalise, cost,
+                                  static_cast<cudaStream_t>(stream)));
   });
 }
 

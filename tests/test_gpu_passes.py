@@ -1,0 +1,124 @@
+"""The device passes beside a solve at the sizes where they can go wrong: tiles and
+chunks that end inside a column or a row, the smallest sizes, unaligned buffers, and
+values that leave the range their fast paths take.
+
+Tolerances: the cost builder and the two passes over point pairs give the FP64 result
+bit for bit (products and sums of each entry in one order, and a maximum or minimum has
+no order). The rounded plan's entries are sums of at most m + n terms in another order,
+64-bit: 1e-12 relative, as for the host entry."""
+import numpy as np
+import oracle
+import pytest
+
+from pdot import _abi, instances, multiscale
+
+pytestmark = pytest.mark.gpu
+
+
+def _cost(x, y, normalise=True):
+    C = np.zeros((x.shape[0], y.shape[0]))
+    for k in range(x.shape[1]):
+        C += (x[:, k : k + 1] - y[None, :, k]) ** 2
+    with np.errstate(invalid="ignore"):
+        mx = np.fmax.reduce(C, axis=None, initial=0.0)
+        return C / mx if normalise and mx > 0 else C
+
+
+def _device_cost(cuda, x, y, normalise, shift=0):
+    import torch
+
+    (m, d), n = x.shape, y.shape[0]
+    lib = _abi.load()
+    dx, dy = torch.from_numpy(x).to(cuda), torch.from_numpy(y).to(cuda)
+    buf = torch.full((m * n + shift,), -1.0, dtype=torch.float64, device=cuda)
+    _abi.check(lib, lib.pdot_sqeuclid_cost_f64(m, n, d, dx.data_ptr(), dy.data_ptr(), normalise,
+                                               buf.data_ptr() + 8 * shift, None), "pdot_sqeuclid_cost_f64")
+    torch.cuda.synchronize()
+    return buf[shift:].cpu().numpy().reshape(n, m).T
+
+
+@pytest.mark.parametrize("normalise", [0, 1])
+@pytest.mark.parametrize("m,n,d", [(1, 1, 1), (2, 1, 2), (3, 2, 3), (512, 17, 4), (513, 300, 2), (1026, 33, 5), (2047, 1, 7)])
+def test_cost_builder_is_exact(cuda, m, n, d, normalise):
+    rng = np.random.default_rng(m + n)
+    x, y = rng.normal(size=(m, d)), rng.normal(size=(n, d))
+    for shift in (0, 1):
+        assert np.array_equal(_device_cost(cuda, x, y, normalise, shift), _cost(x, y, normalise))
+
+
+@pytest.mark.parametrize("scale", [0.0, 1e-160, 1e-90, 1e90, 1e150, 1e154])
+def test_cost_builder_is_exact_at_the_ends_of_the_range(cuda, scale):
+    """All points equal, squares below and above the range of the fast quotient, and infinities."""
+    rng = np.random.default_rng(5)
+    x, y = scale * rng.uniform(1, 2, (70, 2)), scale * rng.uniform(-2, -1, (41, 2))
+    x[3], y[4] = 0.0, 0.0
+    with np.errstate(over="ignore", invalid="ignore"):
+        want = _cost(x, y)
+        np.testing.assert_array_equal(_device_cost(cuda, x, y, 1), want)
+        x[5, 1] = np.nan
+        want = _cost(x, y)
+    np.testing.assert_array_equal(_device_cost(cuda, x, y, 1), want)
+
+
+def test_cost_quotients_are_correctly_rounded(cuda):
+    """Many quotients by one divisor, of all magnitudes below it: one-dimensional points against the origin."""
+    rng = np.random.default_rng(6)
+    x = np.sqrt(np.exp2(rng.uniform(-300, 0, (1_000_000, 1))) * rng.uniform(1, 2, (1_000_000, 1)))
+    x[:500_000] = rng.uniform(0.5, 1.4, (500_000, 1))
+    y = np.zeros((1, 1))
+    assert np.array_equal(_device_cost(cuda, x, y, 1), _cost(x, y))
+
+
+@pytest.mark.parametrize("m,n,shift", [(1, 1, 0), (2, 300, 0), (255, 31, 0), (256, 33, 0), (514, 65, 1), (513, 129, 0),
+                                       (4098, 7, 0), (6, 5000, 0)])
+def test_rounding_on_device_buffers(cuda, m, n, shift):
+    import torch
+
+    rng = np.random.default_rng(m * n)
+    prob = instances.uniform_sqeuclid(m, n, seed=m)
+    X = np.outer(prob.source_distribution, prob.target_distribution) * rng.uniform(0, 2, (m, n)) * (rng.random((m, n)) < 0.5)
+    X[m // 2] = 0.0  # an empty row: its ratio is a / 0
+    lib = _abi.load()
+    a, b = (torch.from_numpy(v).to(cuda) for v in (prob.source_distribution, prob.target_distribution))
+    buf = torch.zeros(m * n + shift, dtype=torch.float64, device=cuda)
+    buf[shift:] = torch.from_numpy(np.ascontiguousarray(X.T)).to(cuda).view(-1)
+    _abi.check(lib, lib.pdot_rounding_f64(m, n, a.data_ptr(), b.data_ptr(), buf.data_ptr() + 8 * shift, None), "pdot_rounding_f64")
+    torch.cuda.synchronize()
+    ref = np.asfortranarray(X)
+    oracle.rounding(prob, ref)
+    np.testing.assert_allclose(buf[shift:].cpu().numpy().reshape(n, m).T, ref, rtol=1e-12, atol=1e-18)
+
+
+def _sq(p, q):
+    out = np.zeros((p.shape[0], q.shape[0]))
+    for k in range(p.shape[1]):
+        out += (p[:, k : k + 1] - q[None, :, k]) ** 2
+    return out
+
+
+@pytest.mark.parametrize("offset,spread", [(0.0, 1.0), (1e4, 1e-3), (0.0, 1e-25), (0.0, 1e25)])
+@pytest.mark.parametrize("m,n,d", [(1, 1, 1), (513, 1, 2), (700, 257, 3), (1, 4100, 2), (1025, 2049, 1)])
+def test_pair_passes_are_exact(cuda, m, n, d, offset, spread):
+    """Bit for bit, also where FP32 tells no pairs apart (an offset, far above the spread) and where its
+    squares underflow or overflow."""
+    rng = np.random.default_rng(m + 7 * n + d)
+    x, y = ((offset + spread * rng.normal(size=(k, d))).astype(np.float32) for k in (m, n))
+    x64, y64 = x.astype(np.float64), y.astype(np.float64)
+    assert multiscale.max_sq_distance(x, y) == _sq(x64, y64).max()
+    centres = offset + spread * rng.normal(size=(n, d))
+    dual = spread**2 * rng.normal(size=n)
+    got = multiscale.c_transform(x, centres, dual, 0.7)
+    assert np.array_equal(got, (0.7 * _sq(x64, centres) - dual[None, :]).min(axis=1))
+
+
+def test_pair_passes_ignore_what_is_not_a_number(cuda):
+    rng = np.random.default_rng(9)
+    x, y = rng.normal(size=(600, 2)).astype(np.float32), rng.normal(size=(500, 2)).astype(np.float32)
+    centres, dual = rng.normal(size=(500, 2)), rng.normal(size=500)
+    y[3, 0], centres[7, 1], dual[9] = np.nan, np.nan, np.nan
+    dual[11], dual[12], x[5] = -np.inf, 1e300, np.nan
+    with np.errstate(invalid="ignore"):
+        far = np.fmax.reduce(_sq(x.astype(np.float64), y.astype(np.float64)), axis=None)
+        near = np.fmin.reduce(0.7 * _sq(x.astype(np.float64), centres) - dual[None, :], axis=1, initial=np.inf)
+    assert multiscale.max_sq_distance(x, y) == far
+    np.testing.assert_array_equal(multiscale.c_transform(x, centres, dual, 0.7), near)
