@@ -4,9 +4,19 @@
 // semi-discrete c-transform that extends duals known on coarse cells to every
 // point, u_i = min_J (scale * ||x_i - c_J||^2 - V_J).
 //
-// Both are brute force over pairs with the second set staged through shared
-// memory in tiles: at 20000 x 15000 points that is 3e8 pairs, a fraction of a
-// millisecond, where the same loops on the host took over a second.
+// Both visit every pair, but only pairs that can decide the result are computed in
+// FP64. A pass over a tile of the second set in FP32 finds what the tile holds for a
+// point, to a known error; where that cannot beat the best value so far by more than
+// the error, the tile is done, and else the FP64 values of the pairs within the error
+// are taken. The results are those of FP64 throughout, bit for bit (a maximum and a
+// minimum do not depend on the pairs that are left out). FP64 arithmetic was what
+// bounded them: B200 does two FP32 operations for one in FP64, and none of the FP32
+// ones needs the conversions.
+//
+// The second set is split over CTAs too, so that 20000 points, 79 CTAs of 256, fill
+// the 148 SMs: the maximum by atomicMax, the minimum by a cluster's shared memory.
+#include <cooperative_groups.h>
+
 #include <cfloat>
 #include <cmath>
 
@@ -15,37 +25,87 @@
 namespace pdot {
 namespace {
 
-constexpr int kTile = 256;  // points of the second set per shared-memory tile (= threads per CTA)
+constexpr int kTile = 256;      // points of the second set per shared-memory tile (= threads per CTA)
+constexpr int kPointsPer = 2;   // points of the first set per thread: a tile entry read once serves both
+constexpr int kSplit = 8;       // CTAs of a cluster, each with a share of the centres
+constexpr float kUnit = 5.9604645e-8f;  // 2^-24, the relative error of one FP32 rounding
 
-// Thread i keeps max_j ||x_i - y_j||^2 (FP64 from FP32 coordinates); a CTA
-// reduces its threads and one atomicMax on the bit pattern combines the CTAs
-// (non-negative doubles order like their bit patterns).
+// Threads keep max_j ||x_i - y_j||^2 of their points (FP64 from FP32 coordinates) over a
+// share of the y_j; a CTA reduces its threads and one atomicMax on the bit pattern
+// combines the CTAs (non-negative doubles order like their bit patterns).
+//
+// The FP32 distance of FP32 points has a relative error below (D + 3) 2^-24, and below
+// 1e-36 from underflow, so a tile's FP32 maximum t holds an FP64 distance of at least
+// t (1 - 2e-6) - 1e-30 and none above t (1 + 2e-6) + 1e-30. Threads whose upper bound
+// stays below the CTA's largest lower bound (or below the result so far) are done with
+// the tile; the others take its FP64 distances. Which threads those are can differ
+// from run to run, the maximum cannot.
 template <int D>
-__global__ void __launch_bounds__(kTile) k_max_sqdist(int64_t m, int64_t n, const float* __restrict__ xs,
+__global__ void __launch_bounds__(kTile) k_max_sqdist(int64_t m, int64_t n, int64_t share, const float* __restrict__ xs,
                                                       const float* __restrict__ ys,
                                                       unsigned long long* __restrict__ out_bits) {
   __shared__ float ty[kTile * D];
   __shared__ double red[kTile / 32];
-  const int64_t i = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  double xi[D];
+  __shared__ float sbest;  // a lower bound of the result
+  float xi[kPointsPer][D];
+  bool ok[kPointsPer];
 #pragma unroll
-  for (int d = 0; d < D; ++d) xi[d] = i < m ? (double)xs[i * D + d] : 0.0;
+  for (int q = 0; q < kPointsPer; ++q) {
+    const int64_t i = ((int64_t)blockIdx.x * kPointsPer + q) * kTile + threadIdx.x;
+    ok[q] = i < m;
+#pragma unroll
+    for (int d = 0; d < D; ++d) xi[q][d] = ok[q] ? xs[i * D + d] : 0.0f;
+  }
   double best = 0.0;
-  for (int64_t j0 = 0; j0 < n; j0 += kTile) {
-    const int64_t cnt = (n - j0) < kTile ? (n - j0) : kTile;
+  if (threadIdx.x == 0)
+    sbest = __double2float_rd(__longlong_as_double((long long)*reinterpret_cast<volatile unsigned long long*>(out_bits)));
+  const int64_t jb = (int64_t)blockIdx.y * share, je = (jb + share < n) ? jb + share : n;
+  for (int64_t j0 = jb; j0 < je; j0 += kTile) {
+    const int cnt = (int)((je - j0) < kTile ? (je - j0) : kTile);
     __syncthreads();
     for (int t = threadIdx.x; t < cnt * D; t += kTile) ty[t] = ys[j0 * D + t];
     __syncthreads();
-    if (i < m)
-      for (int t = 0; t < cnt; ++t) {
-        double s = 0.0;
+    float top[kPointsPer];
+#pragma unroll
+    for (int q = 0; q < kPointsPer; ++q) top[q] = -1.0f;
+#pragma unroll 4
+    for (int t = 0; t < cnt; ++t) {
+#pragma unroll
+      for (int q = 0; q < kPointsPer; ++q) {
+        float s = 0.0f;
 #pragma unroll
         for (int d = 0; d < D; ++d) {
-          const double e = xi[d] - (double)ty[t * D + d];
-          s += e * e;
+          const float e = xi[q][d] - ty[t * D + d];
+          s = d == 0 ? e * e : __fmaf_rn(e, e, s);
         }
-        best = s > best ? s : best;
+        top[q] = fmaxf(top[q], s);
       }
+    }
+    // the bits of non-negative floats order as the floats do
+    float lower = 0.0f;
+#pragma unroll
+    for (int q = 0; q < kPointsPer; ++q)
+      if (ok[q] && top[q] < INFINITY) lower = fmaxf(lower, top[q] * 0.999998f - 1e-30f);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) lower = fmaxf(lower, __shfl_xor_sync(0xffffffffu, lower, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int*>(&sbest), __float_as_int(lower));
+    __syncthreads();
+    const float lim = sbest;
+#pragma unroll
+    for (int q = 0; q < kPointsPer; ++q) {
+      // a tile of NaNs leaves top at -1 and has nothing to offer
+      if (ok[q] && top[q] >= 0.0f && !(top[q] * 1.000002f + 1e-30f < lim)) {
+        for (int t = 0; t < cnt; ++t) {
+          double s = 0.0;
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            const double e = (double)xi[q][d] - (double)ty[t * D + d];
+            s += e * e;
+          }
+          best = s > best ? s : best;
+        }
+      }
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -61,39 +121,141 @@ __global__ void __launch_bounds__(kTile) k_max_sqdist(int64_t m, int64_t n, cons
   }
 }
 
-// out_i = min_J (scale * ||p_i - c_J||^2 - dual_J), p in FP32, centres and
-// duals in FP64, arithmetic in FP64.
+// out_i = min_J (scale * ||p_i - c_J||^2 - dual_J), p in FP32, centres and duals in
+// FP64, arithmetic in FP64. The CTAs of a cluster take the centres of a point block in
+// equal shares; the cluster's first CTA reads the others' minima from their shared
+// memory.
+//
+// The FP32 value of a pair (centre, dual and scale rounded to FP32) is within
+//   E = 16 * 2^-24 * (2 |scale| D A^2 + V),  A = |p|_max + |c|_max,  V = |dual|_max
+// of the FP64 one over a tile (each coordinate difference is at most A and errs by at
+// most 2 * 2^-24 A, a square by 5 * 2^-24 A^2, their sum, the product and the
+// difference by a rounding each; 16 covers D <= 3). A pair whose FP32 value exceeds
+// min(best so far, tile's FP32 minimum + E) + E cannot be the minimum. Where a bound
+// is not finite no pair is left out.
 template <int D>
-__global__ void __launch_bounds__(kTile) k_c_transform(int64_t np, int64_t nc, const float* __restrict__ pts,
-                                                       const double* __restrict__ centres,
-                                                       const double* __restrict__ duals, double scale,
-                                                       double* __restrict__ out) {
+__global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kTile)
+    k_c_transform(int64_t np, int64_t nc, const float* __restrict__ pts, const double* __restrict__ centres,
+                  const double* __restrict__ duals, double scale, double* __restrict__ out) {
   __shared__ double tc[kTile * D];
   __shared__ double tv[kTile];
-  const int64_t i = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  double p[D];
+  __shared__ float fc[kTile * D];
+  __shared__ float fv[kTile];
+  __shared__ int bound_c, bound_v;  // bits of the tile's |c|_max and |dual|_max
+  __shared__ double part[kTile * kPointsPer];
+  float p[kPointsPer][D], reach[kPointsPer];
+  double best[kPointsPer];
+  bool ok[kPointsPer];
 #pragma unroll
-  for (int d = 0; d < D; ++d) p[d] = i < np ? (double)pts[i * D + d] : 0.0;
-  double best = INFINITY;
-  for (int64_t j0 = 0; j0 < nc; j0 += kTile) {
-    const int64_t cnt = (nc - j0) < kTile ? (nc - j0) : kTile;
+  for (int q = 0; q < kPointsPer; ++q) {
+    const int64_t i = ((int64_t)blockIdx.x * kPointsPer + q) * kTile + threadIdx.x;
+    ok[q] = i < np;
+    best[q] = INFINITY;
+    reach[q] = 0.0f;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      p[q][d] = ok[q] ? pts[i * D + d] : 0.0f;
+      reach[q] = fmaxf(reach[q], fabsf(p[q][d]));
+    }
+  }
+  const float sc = (float)scale;
+  const int64_t share = (nc + kSplit - 1) / kSplit;
+  const int64_t jb = (int64_t)blockIdx.y * share, je = (jb + share < nc) ? jb + share : nc;
+  for (int64_t j0 = jb; j0 < je; j0 += kTile) {
+    const int cnt = (int)((je - j0) < kTile ? (je - j0) : kTile);
     __syncthreads();
-    for (int t = threadIdx.x; t < cnt * D; t += kTile) tc[t] = centres[j0 * D + t];
-    for (int t = threadIdx.x; t < cnt; t += kTile) tv[t] = duals[j0 + t];
+    if (threadIdx.x == 0) bound_c = bound_v = 0;
     __syncthreads();
-    if (i < np)
-      for (int t = 0; t < cnt; ++t) {
-        double s = 0.0;
+    float mc = 0.0f, mv = 0.0f;
+    bool odd = false;  // a value that FP32 cannot hold or that is not a number
+    for (int t = threadIdx.x; t < cnt * D; t += kTile) {
+      const double c = centres[j0 * D + t];
+      tc[t] = c;
+      fc[t] = (float)c;
+      mc = fmaxf(mc, fabsf(fc[t]));
+      odd |= !(fabsf(fc[t]) < INFINITY);
+    }
+    for (int t = threadIdx.x; t < cnt; t += kTile) {
+      const double v = duals[j0 + t];
+      tv[t] = v;
+      fv[t] = (float)v;
+      mv = fmaxf(mv, fabsf(fv[t]));
+      odd |= !(fabsf(fv[t]) < INFINITY);
+    }
+    if (odd) mc = INFINITY;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      mc = fmaxf(mc, __shfl_xor_sync(0xffffffffu, mc, o));
+      mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+      atomicMax(&bound_c, __float_as_int(mc));
+      atomicMax(&bound_v, __float_as_int(mv));
+    }
+    __syncthreads();
+    float low[kPointsPer];
+#pragma unroll
+    for (int q = 0; q < kPointsPer; ++q) low[q] = INFINITY;
+#pragma unroll 4
+    for (int t = 0; t < cnt; ++t) {
+#pragma unroll
+      for (int q = 0; q < kPointsPer; ++q) {
+        float s = 0.0f;
 #pragma unroll
         for (int d = 0; d < D; ++d) {
-          const double e = p[d] - tc[t * D + d];
-          s += e * e;
+          const float e = p[q][d] - fc[t * D + d];
+          s = d == 0 ? e * e : __fmaf_rn(e, e, s);
         }
-        const double val = scale * s - tv[t];
-        best = val < best ? val : best;
+        low[q] = fminf(low[q], __fmaf_rn(sc, s, -fv[t]));
       }
+    }
+#pragma unroll
+    for (int q = 0; q < kPointsPer; ++q) {
+      const float A = reach[q] + __int_as_float(bound_c);
+      const float E = 16.0f * kUnit * (2.0f * fabsf(sc) * (float)D * A * A + __int_as_float(bound_v)) + fabsf(sc) * 1e-38f + 1e-30f;
+      const float have = __double2float_ru(best[q]);
+      const float lim = (low[q] + E < have ? low[q] + E : have) + E;
+      const bool all = !(E < INFINITY) || !(fabsf(sc) < INFINITY) || !(fabsf(lim) < INFINITY);
+      if (ok[q] && (all || !(low[q] > lim))) {
+        for (int t = 0; t < cnt; ++t) {
+          if (!all) {
+            float s = 0.0f;
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+              const float e = p[q][d] - fc[t * D + d];
+              s = d == 0 ? e * e : __fmaf_rn(e, e, s);
+            }
+            if (__fmaf_rn(sc, s, -fv[t]) > lim) continue;
+          }
+          double s = 0.0;
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            const double e = (double)p[q][d] - tc[t * D + d];
+            s += e * e;
+          }
+          const double val = scale * s - tv[t];
+          best[q] = val < best[q] ? val : best[q];
+        }
+      }
+    }
   }
-  if (i < np) out[i] = best;
+#pragma unroll
+  for (int q = 0; q < kPointsPer; ++q) part[q * kTile + threadIdx.x] = best[q];
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  cluster.sync();
+  if (cluster.block_rank() == 0) {
+#pragma unroll
+    for (int q = 0; q < kPointsPer; ++q) {
+      double b = best[q];
+      for (int r = 1; r < kSplit; ++r) {
+        const double o = *cluster.map_shared_rank(part + q * kTile + threadIdx.x, r);
+        b = o < b ? o : b;
+      }
+      const int64_t i = ((int64_t)blockIdx.x * kPointsPer + q) * kTile + threadIdx.x;
+      if (ok[q]) out[i] = b;
+    }
+  }
+  cluster.sync();  // no CTA leaves while its shared memory is read
 }
 
 int report(int code, const char* msg) {
@@ -114,14 +276,19 @@ extern "C" int pdot_points_max_sqdist(int64_t m, int64_t n, int32_t dim, const f
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaMemsetAsync(out, 0, sizeof(double), s);
   if (e != cudaSuccess) return report(PDOT_ERR_CUDA, cudaGetErrorString(e));
-  const unsigned blocks = (unsigned)((m + kTile - 1) / kTile);
+  const int64_t blocks = (m + kTile * kPointsPer - 1) / (kTile * kPointsPer);
+  // the second set in shares so that some 8 CTAs per SM run, none below a tile
+  int64_t shares = (148 * 8 + blocks - 1) / blocks;
+  shares = shares < (n + kTile - 1) / kTile ? shares : (n + kTile - 1) / kTile;
+  const int64_t share = (n + shares - 1) / shares;
+  const dim3 grid((unsigned)blocks, (unsigned)((n + share - 1) / share));
   auto* bits = reinterpret_cast<unsigned long long*>(out);
   if (dim == 1)
-    k_max_sqdist<1><<<blocks, kTile, 0, s>>>(m, n, source_points, target_points, bits);
+    k_max_sqdist<1><<<grid, kTile, 0, s>>>(m, n, share, source_points, target_points, bits);
   else if (dim == 2)
-    k_max_sqdist<2><<<blocks, kTile, 0, s>>>(m, n, source_points, target_points, bits);
+    k_max_sqdist<2><<<grid, kTile, 0, s>>>(m, n, share, source_points, target_points, bits);
   else
-    k_max_sqdist<3><<<blocks, kTile, 0, s>>>(m, n, source_points, target_points, bits);
+    k_max_sqdist<3><<<grid, kTile, 0, s>>>(m, n, share, source_points, target_points, bits);
   e = cudaGetLastError();
   if (e != cudaSuccess) return report(PDOT_ERR_CUDA, cudaGetErrorString(e));
   return PDOT_OK;
@@ -137,7 +304,7 @@ extern "C" int pdot_points_c_transform(int64_t num_points, int64_t num_centres, 
   if (!points || !centres || !duals || !out) return report(PDOT_ERR_INVALID_ARGUMENT, "null pointer argument");
   if (!std::isfinite(scale)) return report(PDOT_ERR_INVALID_ARGUMENT, "scale must be finite");
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const unsigned blocks = (unsigned)((num_points + kTile - 1) / kTile);
+  const dim3 blocks((unsigned)((num_points + kTile * kPointsPer - 1) / (kTile * kPointsPer)), kSplit);
   if (dim == 1)
     k_c_transform<1><<<blocks, kTile, 0, s>>>(num_points, num_centres, points, centres, duals, scale, out);
   else if (dim == 2)
