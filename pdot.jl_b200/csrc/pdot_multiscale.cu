@@ -193,9 +193,14 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kTile)
       atomicMax(&bound_v, __float_as_int(mv));
     }
     __syncthreads();
-    float low[kPointsPer];
+    // the tile's smallest and second smallest FP32 value and where the smallest is
+    float low[kPointsPer], next[kPointsPer];
+    int at[kPointsPer];
 #pragma unroll
-    for (int q = 0; q < kPointsPer; ++q) low[q] = INFINITY;
+    for (int q = 0; q < kPointsPer; ++q) {
+      low[q] = next[q] = INFINITY;
+      at[q] = 0;
+    }
 #pragma unroll 4
     for (int t = 0; t < cnt; ++t) {
 #pragma unroll
@@ -206,35 +211,46 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kTile)
           const float e = p[q][d] - fc[t * D + d];
           s = d == 0 ? e * e : __fmaf_rn(e, e, s);
         }
-        low[q] = fminf(low[q], __fmaf_rn(sc, s, -fv[t]));
+        const float v = __fmaf_rn(sc, s, -fv[t]);
+        next[q] = fminf(next[q], fmaxf(v, low[q]));
+        at[q] = v < low[q] ? t : at[q];
+        low[q] = fminf(low[q], v);
       }
     }
 #pragma unroll
     for (int q = 0; q < kPointsPer; ++q) {
       const float A = reach[q] + __int_as_float(bound_c);
-      const float E = 16.0f * kUnit * (2.0f * fabsf(sc) * (float)D * A * A + __int_as_float(bound_v)) + fabsf(sc) * 1e-38f + 1e-30f;
+      const float E = 16.0f * kUnit * (2.0f * fabsf(sc) * (float)D * A * A + __int_as_float(bound_v)) +
+                      fabsf(sc) * 1e-38f + 1e-30f;
       const float have = __double2float_ru(best[q]);
       const float lim = (low[q] + E < have ? low[q] + E : have) + E;
       const bool all = !(E < INFINITY) || !(fabsf(sc) < INFINITY) || !(fabsf(lim) < INFINITY);
+      auto take = [&](int t) {
+        double s = 0.0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          const double e = (double)p[q][d] - tc[t * D + d];
+          s += e * e;
+        }
+        const double val = scale * s - tv[t];
+        best[q] = val < best[q] ? val : best[q];
+      };
       if (ok[q] && (all || !(low[q] > lim))) {
-        for (int t = 0; t < cnt; ++t) {
-          if (!all) {
-            float s = 0.0f;
+        if (!all && next[q] > lim) {
+          take(at[q]);  // the only pair within the error
+        } else {
+          for (int t = 0; t < cnt; ++t) {
+            if (!all) {
+              float s = 0.0f;
 #pragma unroll
-            for (int d = 0; d < D; ++d) {
-              const float e = p[q][d] - fc[t * D + d];
-              s = d == 0 ? e * e : __fmaf_rn(e, e, s);
+              for (int d = 0; d < D; ++d) {
+                const float e = p[q][d] - fc[t * D + d];
+                s = d == 0 ? e * e : __fmaf_rn(e, e, s);
+              }
+              if (__fmaf_rn(sc, s, -fv[t]) > lim) continue;
             }
-            if (__fmaf_rn(sc, s, -fv[t]) > lim) continue;
+            take(t);
           }
-          double s = 0.0;
-#pragma unroll
-          for (int d = 0; d < D; ++d) {
-            const double e = (double)p[q][d] - tc[t * D + d];
-            s += e * e;
-          }
-          const double val = scale * s - tv[t];
-          best[q] = val < best[q] ? val : best[q];
         }
       }
     }

@@ -6,10 +6,21 @@
 //   g_j = eps (log b_j - LSE_i((f_i - C_ij) / eps))        (columns sum to b)
 // start from (f, g) = (u0, v0); the plan is X_ij = exp((f_i + g_j - C_ij) / eps)
 // and its row and column sums r, c. The solver keeps (u0, v0) as its duals.
-// One warp per row or column; every sum in a fixed order, so the result is
-// deterministic. The balancing rounds take their exponentials in FP32 (the
-// plan is only a starting point); the plan entries and their sums are FP64
-// (narrowed to the plan's storage type before they are summed).
+// Every sum is in a fixed order (lane l of a warp takes entries l, l + 32, ... of
+// a row or column, then a shuffle tree), so the result is deterministic. The
+// balancing rounds take their exponentials in FP32 (the plan is only a starting
+// point); the plan entries and their sums are FP64 (narrowed to the plan's storage
+// type before they are summed).
+//
+// A warp takes up to Q neighbouring rows (columns) at once, with the cost kind and
+// the point dimension compiled in: the other side's potential and coordinates are
+// loaded once for Q entries and Q times four dependency chains overlap. What bounds a
+// round is issue and the latency of those chains: 35 instructions an entry, four of
+// them FP64 and two conversions; no round touches the plan. Measured on B200 per
+// half-round (one row at a time with the kind and dimension read at run time, before;
+// as here): 191 -> 71 us at 8000 x 6000 and 967 -> 369 us at 20000 x 15000 from
+// planar points, 20 -> 12 us at 1024 x 1024, 272 -> 124 us for a stored FP64 cost of
+// 6000 x 6000.
 #include <cmath>
 #include <cstdint>
 
@@ -20,6 +31,17 @@ namespace {
 
 constexpr int kWpThreads = 256;
 constexpr int kWpWarps = kWpThreads / 32;
+// CTAs of two warps: a few thousand row groups then spread evenly over the SMs.
+constexpr int kWpGroupThreads = 64;
+constexpr int kWpGroupWarps = kWpGroupThreads / 32;
+constexpr int kWpUnroll = 4;
+// Rows of a warp's group: two, or four for a stored cost of 4 bytes or fewer an entry,
+// whose 32-byte sectors they share (25 against 30 us at 3000 x 3000 in FP32; from
+// points two beat four by 71 to 90 us at 8000 x 6000, where four leave 13 warps per SM).
+constexpr int group_rows(int ck) { return ck == PDOT_COST_F32 || ck == PDOT_COST_BF16 ? 4 : 2; }
+// Groups only where they still leave some 8 warps per SM; below, a warp takes one
+// row, since then latency counts and not the work per entry.
+constexpr bool grouped(long long total, int Q) { return total >= 148ll * 8 * Q; }
 
 __device__ __forceinline__ int find_instance(const long long* prefix, int count, long long q) {
   int lo = 0, hi = count - 1;
@@ -33,36 +55,80 @@ __device__ __forceinline__ int find_instance(const long long* prefix, int count,
   return lo;
 }
 
-// The solver's cost entry C_ij of instance I (coordinate costs in FP32 as the
-// primal pass computes them, times the instance's cost scale).
-__device__ __forceinline__ double cost_at(const WarmPlanArgs& A, const PlanInstance& I, float scale, int64_t i,
-                                          int64_t j) {
-  const int64_t e = I.x_off + i + j * I.ld;
-  if (A.kind == PDOT_COST_F64) return static_cast<const double*>(A.C)[e];
-  if (A.kind == PDOT_COST_F32) return (double)static_cast<const float*>(A.C)[e];
-  if (A.kind == PDOT_COST_BF16) return (double)__bfloat162float(static_cast<const __nv_bfloat16*>(A.C)[e]);
-  const float* x = A.xs + (I.row_off + i) * A.dim;
-  const float* y = A.ys + (I.col_off + j) * A.dim;
-  const bool l1 = is_l1_cost(A.kind);
-  float acc = 0.0f;
-  for (int d = 0; d < A.dim; ++d) {
-    const float t = __ldg(x + d) - __ldg(y + d);
-    acc = l1 ? acc + fabsf(t) : acc + t * t;
+// The solver's cost entries C_ij of instance I between the Q members of a group (rows
+// if BY_ROWS, else columns) and one member of the other side: coordinate costs in FP32
+// as the solver reads them, times the instance's cost scale, or the stored entry.
+// Members past the group's end repeat its last one.
+template <int CK, int Q, bool BY_ROWS>
+struct GroupCost {
+  static constexpr bool kPoints = is_point_cost(CK);
+  static constexpr bool kL1 = is_l1_cost(CK);
+  static constexpr int DIM = kPoints ? CK - (kL1 ? kCostL1Base : kCostSqBase) : 1;
+  const void* C;
+  const float* other;
+  float scale;
+  float own[Q][DIM];
+  float oth[DIM];
+  int64_t base[Q];
+  int64_t stride;
+  __device__ __forceinline__ GroupCost(const WarmPlanArgs& A, const PlanInstance& I, float scl, int64_t first, int count)
+      : C(A.C), scale(scl) {
+    if constexpr (kPoints) {
+      const float* mine = BY_ROWS ? A.xs + I.row_off * DIM : A.ys + I.col_off * DIM;
+      other = BY_ROWS ? A.ys + I.col_off * DIM : A.xs + I.row_off * DIM;
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) own[q][d] = __ldg(mine + (first + (q < count ? q : count - 1)) * DIM + d);
+    } else {
+      stride = BY_ROWS ? I.ld : 1;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int64_t k = first + (q < count ? q : count - 1);
+        base[q] = I.x_off + (BY_ROWS ? k : k * I.ld);
+      }
+    }
   }
-  return (double)(acc * scale);
-}
+  // the other side's member `o` that get() pairs with the group's
+  __device__ __forceinline__ void load(int64_t o) {
+    if constexpr (kPoints) {
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) oth[d] = __ldg(other + o * DIM + d);
+    }
+  }
+  __device__ __forceinline__ double get(int q, int64_t o) const {
+    if constexpr (CK == PDOT_COST_F64) {
+      return __ldg(static_cast<const double*>(C) + base[q] + o * stride);
+    } else if constexpr (CK == PDOT_COST_F32) {
+      return (double)__ldg(static_cast<const float*>(C) + base[q] + o * stride);
+    } else if constexpr (CK == PDOT_COST_BF16) {
+      return (double)__bfloat162float(static_cast<const __nv_bfloat16*>(C)[base[q] + o * stride]);
+    } else {
+      float acc = 0.0f;
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        const float t = BY_ROWS ? own[q][d] - oth[d] : oth[d] - own[q][d];
+        const float e = kL1 ? fabsf(t) : t * t;
+        acc = d == 0 ? e : acc + e;
+      }
+      return (double)(acc * scale);
+    }
+  }
+};
 
 // log-sum-exp accumulator: value = mx + log(s)
 struct Lse {
   double mx = -INFINITY;
   float s = 0.0f;
+  // A new maximum rescales the sum by exp(mx - x) and adds 1, any other x adds
+  // exp(x - mx): one exponential of -|x - mx| either way (0 from mx = -inf), so a
+  // warp whose lanes disagree does not take it twice.
   __device__ __forceinline__ void add(double x) {
-    if (x > mx) {
-      s = (mx == -INFINITY ? 0.0f : s * expf((float)(mx - x))) + 1.0f;
-      mx = x;
-    } else if (x > -INFINITY) {
-      s += expf((float)(x - mx));
-    }
+    const float e = expf((float)-fabs(x - mx));
+    const bool up = x > mx;
+    const float t = up ? s * e + 1.0f : s + e;
+    s = x > -INFINITY ? t : s;  // -inf and NaN leave the sum alone
+    mx = up ? x : mx;
   }
   __device__ __forceinline__ void merge_warp() {
 #pragma unroll
@@ -77,78 +143,136 @@ struct Lse {
   }
 };
 
-// One balancing half-round: rows (by_rows) update f from g, columns g from f.
-// `first` reads the other side from the warm duals.
-__global__ void __launch_bounds__(kWpThreads) k_wp_balance(WarmPlanArgs A, int by_rows, int first) {
-  const long long total = by_rows ? A.total_rows : A.total_cols;
-  const long long* prefix = by_rows ? A.row_prefix : A.col_prefix;
-  const int lane = threadIdx.x & 31;
-  for (long long q = (long long)blockIdx.x * kWpWarps + (threadIdx.x >> 5); q < total;
-       q += (long long)gridDim.x * kWpWarps) {
-    const int k = find_instance(prefix, A.num, q);
-    const PlanInstance I = A.inst[k];
-    if (!I.active) continue;
-    const float scale = (float)A.st[k].cost_scale;
-    const double inv = 1.0 / A.eps;
-    Lse acc;
-    if (by_rows) {
-      const int64_t i = q - I.row_off;
-      const double* g = first ? A.v0 : A.g;
-      for (int64_t j = lane; j < I.n; j += 32) acc.add((g[I.col_off + j] - cost_at(A, I, scale, i, j)) * inv);
-      acc.merge_warp();
-      if (lane == 0) {
-        const double lse = acc.mx + log((double)acc.s);
-        A.f[q] = acc.mx == -INFINITY ? -INFINITY : A.eps * (log(A.a[q]) - lse);
-      }
-    } else {
-      const int64_t j = q - I.col_off;
-      const double* f = first ? A.u0 : A.f;
-      for (int64_t i = lane; i < I.m; i += 32) acc.add((f[I.row_off + i] - cost_at(A, I, scale, i, j)) * inv);
-      acc.merge_warp();
-      if (lane == 0) {
-        const double lse = acc.mx + log((double)acc.s);
-        A.g[q] = acc.mx == -INFINITY ? -INFINITY : A.eps * (log(A.b[q]) - lse);
-      }
+// Calls f(instance, its index, first local row, rows) for the parts of a warp's group of
+// Q global rows (columns) that lie in one active instance each.
+template <int Q, typename F>
+__device__ __forceinline__ void for_groups(const WarmPlanArgs& A, const long long* prefix, long long total, F&& f) {
+  const long long groups = (total + Q - 1) / Q;
+  for (long long w = (long long)blockIdx.x * kWpGroupWarps + (threadIdx.x >> 5); w < groups;
+       w += (long long)gridDim.x * kWpGroupWarps) {
+    long long q = w * Q;
+    const long long qe = q + Q < total ? q + Q : total;
+    while (q < qe) {
+      const int k = find_instance(prefix, A.num, q);
+      const long long b = __ldg(prefix + k), e = __ldg(prefix + k + 1);
+      const long long to = e < qe ? e : qe;
+      const PlanInstance I = A.inst[k];
+      if (I.active) f(I, k, (int64_t)(q - b), (int)(to - q));
+      q = to;
     }
   }
 }
 
-template <typename TX>
-__device__ __forceinline__ double plan_entry(const WarmPlanArgs& A, const PlanInstance& I, float scale, int64_t i,
-                                             int64_t j) {
-  const double x = exp((A.f[I.row_off + i] + A.g[I.col_off + j] - cost_at(A, I, scale, i, j)) / A.eps);
-  return (double)(TX)x;
+// One balancing half-round: rows (BY_ROWS) update f from g, columns g from f.
+// `first` reads the other side from the warm duals.
+template <int CK, int Q, bool BY_ROWS>
+__global__ void __launch_bounds__(kWpGroupThreads) k_wp_balance(WarmPlanArgs A, int first) {
+  const int lane = threadIdx.x & 31;
+  for_groups<Q>(A, BY_ROWS ? A.row_prefix : A.col_prefix, BY_ROWS ? A.total_rows : A.total_cols,
+                [&](const PlanInstance& I, int k, int64_t q0, int count) {
+    const double inv = 1.0 / A.eps;
+    GroupCost<CK, Q, BY_ROWS> cost(A, I, (float)A.st[k].cost_scale, q0, count);
+    const double* other = BY_ROWS ? (first ? A.v0 : A.g) + I.col_off : (first ? A.u0 : A.f) + I.row_off;
+    const int64_t len = BY_ROWS ? I.n : I.m;
+    Lse acc[Q];
+#pragma unroll kWpUnroll
+    for (int64_t o = lane; o < len; o += 32) {
+      const double h = other[o];
+      cost.load(o);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) acc[q].add((h - cost.get(q, o)) * inv);
+    }
+    const int64_t off = (BY_ROWS ? I.row_off : I.col_off) + q0;
+    const double* mass = (BY_ROWS ? A.a : A.b) + off;
+    double* out = (BY_ROWS ? A.f : A.g) + off;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      acc[q].merge_warp();
+      if (lane == q && q < count) {
+        const double lse = acc[q].mx + log((double)acc[q].s);
+        out[q] = acc[q].mx == -INFINITY ? -INFINITY : A.eps * (log(mass[q]) - lse);
+      }
+    }
+  });
 }
 
-// The plan by columns (stored, with the column sums), then the row sums of
-// the same stored values.
-template <typename TX>
-__global__ void __launch_bounds__(kWpThreads) k_wp_plan(WarmPlanArgs A, int by_rows) {
-  const long long total = by_rows ? A.total_rows : A.total_cols;
-  const long long* prefix = by_rows ? A.row_prefix : A.col_prefix;
+// x / eps rounded to nearest, one divisor for many x: two Markstein corrections of
+// x y with y = 1 / eps rounded to nearest (IBM J. Res. Dev. 34, 1990: a quotient
+// within one ulp is corrected to the nearest; the first correction brings it there).
+// Outside the range that keeps every term normal, the division itself.
+struct OverEps {
+  double eps, y;
+  bool usable;
+  __device__ __forceinline__ explicit OverEps(double e) : eps(e) {
+    y = __drcp_rn(e);
+    usable = e >= 0x1p-400 && e <= 0x1p+400;
+  }
+  __device__ __forceinline__ double operator()(double x) const {
+    const double ax = fabs(x);
+    if (usable && ax >= 0x1p-500 && ax <= 0x1p+500) {
+      double q = __dmul_rn(x, y);
+      q = __fma_rn(__fma_rn(-q, eps, x), y, q);
+      return __fma_rn(__fma_rn(-q, eps, x), y, q);
+    }
+    return x / eps;
+  }
+};
+
+// The plan by columns, stored in its type, with the column sums of what is stored.
+template <typename TX, int CK, int Q>
+__global__ void __launch_bounds__(kWpGroupThreads) k_wp_plan(WarmPlanArgs A) {
   const int lane = threadIdx.x & 31;
   TX* X = static_cast<TX*>(A.X);
-  for (long long q = (long long)blockIdx.x * kWpWarps + (threadIdx.x >> 5); q < total;
-       q += (long long)gridDim.x * kWpWarps) {
-    const int k = find_instance(prefix, A.num, q);
-    const PlanInstance I = A.inst[k];
-    if (!I.active) continue;
-    const float scale = (float)A.st[k].cost_scale;
-    double s = 0.0;
-    if (by_rows) {
-      const int64_t i = q - I.row_off;
-      for (int64_t j = lane; j < I.n; j += 32) s += plan_entry<TX>(A, I, scale, i, j);
-    } else {
-      const int64_t j = q - I.col_off;
-      for (int64_t i = lane; i < I.m; i += 32) {
-        const double x = plan_entry<TX>(A, I, scale, i, j);
-        X[I.x_off + i + j * I.ld] = (TX)x;
-        s += x;
-      }
+  const OverEps over(A.eps);
+  for_groups<Q>(A, A.col_prefix, A.total_cols, [&](const PlanInstance& I, int k, int64_t q0, int count) {
+    GroupCost<CK, Q, false> cost(A, I, (float)A.st[k].cost_scale, q0, count);
+    const double* f = A.f + I.row_off;
+    double g[Q], s[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      g[q] = A.g[I.col_off + q0 + (q < count ? q : count - 1)];
+      s[q] = 0.0;
     }
-    s = warp_sum(s);
-    if (lane == 0) (by_rows ? A.r : A.c)[q] = s;
-  }
+    for (int64_t i = lane; i < I.m; i += 32) {
+      const double fi = f[i];
+      cost.load(i);
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+        if (q < count) {
+          const TX x = (TX)exp(over(fi + g[q] - cost.get(q, i)));
+          X[I.x_off + i + (q0 + q) * I.ld] = x;
+          s[q] += (double)x;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      s[q] = warp_sum(s[q]);
+      if (lane == q && q < count) A.c[I.col_off + q0 + q] = s[q];
+    }
+  });
+}
+
+// The stored plan's row sums.
+template <typename TX, int Q>
+__global__ void __launch_bounds__(kWpGroupThreads) k_wp_row_sums(WarmPlanArgs A) {
+  const int lane = threadIdx.x & 31;
+  const TX* X = static_cast<const TX*>(A.X);
+  for_groups<Q>(A, A.row_prefix, A.total_rows, [&](const PlanInstance& I, int, int64_t q0, int count) {
+    double s[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) s[q] = 0.0;
+    const TX* row = X + I.x_off + q0;
+#pragma unroll 4
+    for (int64_t j = lane; j < I.n; j += 32)
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+        if (q < count) s[q] += (double)row[j * I.ld + q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      s[q] = warp_sum(s[q]);
+      if (lane == q && q < count) A.r[I.row_off + q0 + q] = s[q];
+    }
+  });
 }
 
 __global__ void k_wp_copy(const double* __restrict__ src, double* __restrict__ dst, long long count) {
@@ -161,6 +285,33 @@ int wp_grid(long long warps) {
   return (int)(g < 1 ? 1 : (g > 148 * 16 ? 148 * 16 : g));
 }
 
+// CTAs of the group kernels: one per two groups, at most 32 per SM.
+int group_grid(long long total, int Q) {
+  const long long g = ((total + Q - 1) / Q + kWpGroupWarps - 1) / kWpGroupWarps;
+  return (int)(g < 1 ? 1 : (g > 148 * 32 ? 148 * 32 : g));
+}
+
+template <int CK, int Q, bool BY_ROWS>
+void balance(const WarmPlanArgs& A, int first, cudaStream_t s) {
+  k_wp_balance<CK, Q, BY_ROWS>
+      <<<group_grid(BY_ROWS ? A.total_rows : A.total_cols, Q), kWpGroupThreads, 0, s>>>(A, first);
+}
+
+template <typename TX, int CK>
+void warm_plan(const WarmPlanArgs& A, int iterations, cudaStream_t s) {
+  constexpr int Q = group_rows(CK);
+  const bool rows = grouped(A.total_rows, Q), cols = grouped(A.total_cols, Q);
+  for (int it = 0; it < iterations; ++it) {
+    rows ? balance<CK, Q, true>(A, it == 0, s) : balance<CK, 1, true>(A, it == 0, s);
+    cols ? balance<CK, Q, false>(A, 0, s) : balance<CK, 1, false>(A, 0, s);
+  }
+  if (cols)
+    k_wp_plan<TX, CK, Q><<<group_grid(A.total_cols, Q), kWpGroupThreads, 0, s>>>(A);
+  else
+    k_wp_plan<TX, CK, 1><<<group_grid(A.total_cols, 1), kWpGroupThreads, 0, s>>>(A);
+  k_wp_row_sums<TX, Q><<<group_grid(A.total_rows, Q), kWpGroupThreads, 0, s>>>(A);
+}
+
 }  // namespace
 
 cudaError_t launch_warm_plan(const WarmPlanArgs& A, int iterations, cudaStream_t s) {
@@ -169,22 +320,26 @@ cudaError_t launch_warm_plan(const WarmPlanArgs& A, int iterations, cudaStream_t
   if (!A.inst || A.num < 1 || !A.row_prefix || !A.col_prefix || !A.st || !A.a || !A.b || !A.u0 || !A.v0 || !A.f ||
       !A.g || !A.X || !A.r || !A.c || !(A.eps > 0.0) || (stored ? !A.C : (!A.xs || !A.ys || A.dim < 1)))
     return cudaErrorInvalidValue;
-  const int rg = wp_grid(A.total_rows), cg = wp_grid(A.total_cols);
   if (iterations <= 0) {
     // the plan from the warm duals themselves
-    k_wp_copy<<<rg, kWpThreads, 0, s>>>(A.u0, A.f, A.total_rows);
-    k_wp_copy<<<cg, kWpThreads, 0, s>>>(A.v0, A.g, A.total_cols);
+    k_wp_copy<<<wp_grid(A.total_rows), kWpThreads, 0, s>>>(A.u0, A.f, A.total_rows);
+    k_wp_copy<<<wp_grid(A.total_cols), kWpThreads, 0, s>>>(A.v0, A.g, A.total_cols);
   }
-  for (int it = 0; it < iterations; ++it) {
-    k_wp_balance<<<rg, kWpThreads, 0, s>>>(A, 1, it == 0);
-    k_wp_balance<<<cg, kWpThreads, 0, s>>>(A, 0, 0);
-  }
-  if (A.plan_f32) {
-    k_wp_plan<float><<<cg, kWpThreads, 0, s>>>(A, 0);
-    k_wp_plan<float><<<rg, kWpThreads, 0, s>>>(A, 1);
-  } else {
-    k_wp_plan<double><<<cg, kWpThreads, 0, s>>>(A, 0);
-    k_wp_plan<double><<<rg, kWpThreads, 0, s>>>(A, 1);
+  // the FP64 plan goes with the FP64 cost, an FP32 plan with every other kind
+  if (A.plan_f32 == (A.kind == PDOT_COST_F64)) return cudaErrorInvalidValue;
+  switch (A.kind) {
+    case PDOT_COST_F64: warm_plan<double, PDOT_COST_F64>(A, iterations, s); break;
+    case PDOT_COST_F32: warm_plan<float, PDOT_COST_F32>(A, iterations, s); break;
+    case PDOT_COST_BF16: warm_plan<float, PDOT_COST_BF16>(A, iterations, s); break;
+    case kCostSqBase + 1: warm_plan<float, kCostSqBase + 1>(A, iterations, s); break;
+    case kCostSqBase + 2: warm_plan<float, kCostSqBase + 2>(A, iterations, s); break;
+    case kCostSqBase + 3: warm_plan<float, kCostSqBase + 3>(A, iterations, s); break;
+    case kCostSqBase + 4: warm_plan<float, kCostSqBase + 4>(A, iterations, s); break;
+    case kCostL1Base + 1: warm_plan<float, kCostL1Base + 1>(A, iterations, s); break;
+    case kCostL1Base + 2: warm_plan<float, kCostL1Base + 2>(A, iterations, s); break;
+    case kCostL1Base + 3: warm_plan<float, kCostL1Base + 3>(A, iterations, s); break;
+    case kCostL1Base + 4: warm_plan<float, kCostL1Base + 4>(A, iterations, s); break;
+    default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
 }

@@ -122,3 +122,45 @@ def test_pair_passes_ignore_what_is_not_a_number(cuda):
         near = np.fmin.reduce(0.7 * _sq(x.astype(np.float64), centres) - dual[None, :], axis=1, initial=np.inf)
     assert multiscale.max_sq_distance(x, y) == far
     np.testing.assert_array_equal(multiscale.c_transform(x, centres, dual, 0.7), near)
+
+
+@pytest.mark.parametrize("precision,cost", [("f64", None), ("f32", "f32"), ("f32", "bf16"), ("f32", "sqeuclid"), ("f32", "l1")])
+@pytest.mark.parametrize("m,n", [(4739, 33), (35, 4737), (4735, 31), (2367, 29), (2369, 30)])
+def test_recovered_plan_of_grouped_rows(cuda, m, n, precision, cost):
+    """From 2368 rows (columns) on, 4736 for a stored FP32 or BF16 cost, a warp balances two (four) of
+    them; below, one. The balancing's FP32
+    exponentials and sums err by some 1e-6 a round and the costs by 2^-9 max C (BF16) or 1e-7, over eps."""
+    import pdot
+
+    rng = np.random.default_rng(m)
+    xs, ys = rng.uniform(0, 1, (m, 2)).astype(np.float32), rng.uniform(0, 1, (n, 2)).astype(np.float32)
+    l1 = cost == "l1"
+    C = instances.l1_cost(xs.astype(np.float64), ys.astype(np.float64)) if l1 else instances.sqeuclid_cost(xs, ys)
+    if cost == "bf16":  # entries that BF16 holds
+        C = np.asfortranarray(np.round(C * 128) / 128)
+    a, b = rng.dirichlet(np.ones(m)), rng.dirichlet(np.ones(n))
+    u0, v0, eps, rounds = 0.1 * rng.random(m), 0.1 * rng.random(n), 2e-2, 3
+    want, _, _ = oracle.warm_plan(C, a, b, u0, v0, eps, rounds)
+    kw = {"points": (xs, ys)} if cost in ("sqeuclid", "l1") else {}
+    out = pdot.optimize(pdot.default_parameters(1e-4, iteration_limit=0), pdot.OptimalTransportProblem(C, a, b),
+                        precision=precision, cost=cost, warm_start=(u0, v0), recover_plan=(eps, rounds), **kw)
+    np.testing.assert_allclose(out.primal_solution, want, rtol=1e-3, atol=1e-12)
+
+
+def test_recovered_plans_of_a_batch_whose_groups_cross_instances(cuda):
+    import pdot
+
+    probs, pts = instances.batched_l1(80, 41, 95, seed=3)
+    rng = np.random.default_rng(1)
+    warm = [(0.1 * rng.random(p.source_distribution.size), 0.1 * rng.random(p.target_distribution.size)) for p in probs]
+    warm[1] = warm[40] = None  # cold instances in between
+    eps, rounds = 2e-2, 3
+    outs, _ = pdot.optimize_batched(pdot.default_parameters(1e-4, iteration_limit=0), probs, cost="l1", points=pts,
+                                    warm_starts=warm, recover_plan=(eps, rounds))
+    for p, (x, y), w, o in zip(probs, pts, warm, outs):
+        if w is None:
+            assert not o.primal_solution.any()
+            continue
+        C = instances.l1_cost(x.astype(np.float32).astype(np.float64), y.astype(np.float32).astype(np.float64))
+        want, _, _ = oracle.warm_plan(C, p.source_distribution, p.target_distribution, w[0], w[1], eps, rounds)
+        np.testing.assert_allclose(o.primal_solution, want, rtol=1e-3, atol=1e-12)
