@@ -1315,6 +1315,13 @@ void bck(cudaError_t e, const char* what, int line) {
 class BatchSolver {
  public:
   BatchSolver(const pdot_batch_problem& P, const pdot_pdhg_parameters& prm, const pdot_solver_options* opt) {
+    // what a failing constructor holds goes back, the kept slots and pool blocks among it
+    struct Undo {
+      BatchSolver* s;
+      ~Undo() {
+        if (s) s->release();
+      }
+    } undo{this};
     device_ = opt ? opt->device : 0;
     const int pub_kind = opt ? opt->cost_storage : PDOT_COST_F32;
     dim_ = (pub_kind == PDOT_COST_SQEUCLID_POINTS || pub_kind == PDOT_COST_L1_POINTS) ? opt->point_dim : 0;
@@ -1410,44 +1417,43 @@ class BatchSolver {
     D_.dim = dim_;
     if (dim_ == 0) {
       float* C = alloc<float>(total_x_);
-      double* tmp = nullptr;
-      size_t tmp_cap = 0;
+      size_t cap = 0;
+      for (int k = 0; k < B; ++k) cap = std::max(cap, (size_t)inst_[k].m * inst_[k].n);
+      double* tmp = alloc<double>(cap);
       for (int k = 0; k < B; ++k) {
         const size_t mn = (size_t)inst_[k].m * inst_[k].n;
-        if (mn > tmp_cap) {
-          if (tmp) BCK(cudaFree(tmp));
-          BCK(cudaMalloc(&tmp, mn * sizeof(double)));
-          tmp_cap = mn;
-        }
         BCK(cudaMemcpyAsync(tmp, P.cost_matrices[k], mn * sizeof(double), cudaMemcpyHostToDevice, stream_));
         pdot::kb_convert_cost<<<256, 256, 0, stream_>>>(tmp, inst_[k].m, inst_[k].n, inst_[k].ld, C + inst_[k].x_off);
         BCK(cudaGetLastError());
         BCK(cudaStreamSynchronize(stream_));
       }
-      if (tmp) BCK(cudaFree(tmp));
+      drop(tmp);
       D_.C = C;
       D_.xs = D_.ys = nullptr;
     } else {
       float* xs = alloc<float>((size_t)po * dim_);
       float* ys = alloc<float>((size_t)to * dim_);
+      // one copy for all instances, as for the marginals: a small copy costs 5 us and more
+      std::vector<float> hx((size_t)po * dim_), hy((size_t)to * dim_);
       for (int k = 0; k < B; ++k) {
-        BCK(cudaMemcpyAsync(xs + inst_[k].pts_off * dim_, P.source_points[k], (size_t)inst_[k].m * dim_ * sizeof(float),
-                            cudaMemcpyHostToDevice, stream_));
-        BCK(cudaMemcpyAsync(ys + inst_[k].tpts_off * dim_, P.target_points[k], (size_t)inst_[k].n * dim_ * sizeof(float),
-                            cudaMemcpyHostToDevice, stream_));
+        memcpy(hx.data() + inst_[k].pts_off * dim_, P.source_points[k], (size_t)inst_[k].m * dim_ * sizeof(float));
+        memcpy(hy.data() + inst_[k].tpts_off * dim_, P.target_points[k], (size_t)inst_[k].n * dim_ * sizeof(float));
       }
+      put(xs, hx.data(), hx.size());
+      put(ys, hy.data(), hy.size());
       D_.C = nullptr;
       D_.xs = xs;
       D_.ys = ys;
     }
     double* a = alloc<double>(ro);
     double* b = alloc<double>(co);
+    std::vector<double> ha(ro), hb(co);
     for (int k = 0; k < B; ++k) {
-      BCK(cudaMemcpyAsync(a + inst_[k].row_off, P.source_distributions[k], inst_[k].m * sizeof(double),
-                          cudaMemcpyHostToDevice, stream_));
-      BCK(cudaMemcpyAsync(b + inst_[k].col_off, P.target_distributions[k], inst_[k].n * sizeof(double),
-                          cudaMemcpyHostToDevice, stream_));
+      memcpy(ha.data() + inst_[k].row_off, P.source_distributions[k], inst_[k].m * sizeof(double));
+      memcpy(hb.data() + inst_[k].col_off, P.target_distributions[k], inst_[k].n * sizeof(double));
     }
+    put(a, ha.data(), ha.size());
+    put(b, hb.data(), hb.size());
     D_.a = a;
     D_.b = b;
     for (int h = 0; h < 2; ++h) {
@@ -1501,16 +1507,16 @@ class BatchSolver {
           }
           hc[I.col_off + j] = cs;
         }
-        BCK(cudaMemcpy(warm_x_ + I.x_off, hx.data(), hx.size() * sizeof(float), cudaMemcpyHostToDevice));
+        put(warm_x_ + I.x_off, hx.data(), hx.size());
       }
       warm_u_ = alloc<double>(ro);
       warm_v_ = alloc<double>(co);
       warm_r_ = alloc<double>(ro);
       warm_c_ = alloc<double>(co);
-      BCK(cudaMemcpy(warm_u_, hu.data(), ro * sizeof(double), cudaMemcpyHostToDevice));
-      BCK(cudaMemcpy(warm_v_, hv.data(), co * sizeof(double), cudaMemcpyHostToDevice));
-      BCK(cudaMemcpy(warm_r_, hr.data(), ro * sizeof(double), cudaMemcpyHostToDevice));
-      BCK(cudaMemcpy(warm_c_, hc.data(), co * sizeof(double), cudaMemcpyHostToDevice));
+      put(warm_u_, hu.data(), (size_t)ro);
+      put(warm_v_, hv.data(), (size_t)co);
+      put(warm_r_, hr.data(), (size_t)ro);
+      put(warm_c_, hc.data(), (size_t)co);
     }
     // race groups: an instance stops (reason OTHER) once another member of
     // its group has ended optimal
@@ -1573,7 +1579,7 @@ class BatchSolver {
     D_.st = alloc<pdot::DevState>(B);
     D_.rec = alloc<pdot_iteration_stats>(B);
     D_.act = alloc<pdot::BatchActive>(1);
-    BCK(cudaMemset(D_.act, 0, sizeof(pdot::BatchActive)));
+    BCK(cudaMemsetAsync(D_.act, 0, sizeof(pdot::BatchActive), stream_));
     D_.ids = alloc<int>(B);
     D_.unit_prefix = alloc<long long>(B + 1);
     D_.panel_prefix = alloc<long long>(B + 1);
@@ -1584,19 +1590,22 @@ class BatchSolver {
     fill_config(prm);
     freq_ = prm.termination_evaluation_frequency;
     limit_ = prm.termination_criteria.iteration_limit;
-    void* hp = nullptr;
-    BCK(cudaMallocHost(&hp, sizeof(pdot::BatchActive) * 2));
+    void* hp = pdot::pinned_slot_take();
+    if (!hp) BCK(cudaMallocHost(&hp, sizeof(pdot::BatchActive) * 2));
     host_act_ = static_cast<pdot::BatchActive*>(hp);
     for (int k = 0; k < 2; ++k) BCK(cudaEventCreateWithFlags(&ev_[k], cudaEventDisableTiming));
-    if (use_graph_ && !persistent_) capture();
+    use_graph_ = use_graph_ && !persistent_;
+    undo.s = nullptr;
   }
 
-  ~BatchSolver() {
+  ~BatchSolver() { release(); }
+
+  void release() {
     if (stream_) cudaStreamSynchronize(stream_);
     if (graph_) cudaGraphExecDestroy(graph_);
     for (int k = 0; k < 2; ++k)
       if (ev_[k]) cudaEventDestroy(ev_[k]);
-    if (host_act_) cudaFreeHost(host_act_);
+    if (host_act_ && !pdot::pinned_slot_return(host_act_)) cudaFreeHost(host_act_);
     for (void* p : allocs_) cudaFree(p);
     if (stream_) cudaStreamDestroy(stream_);
   }
@@ -1610,7 +1619,7 @@ class BatchSolver {
     long long it = 1;
     int issued = 0, completed = 0;
     for (;;) {
-      while (issued - completed < 2) {
+      while (issued - completed < 2 && (issued == completed || it <= (long long)limit_ + 1)) {
         enqueue_chunk(it);
         BCK(cudaMemcpyAsync(&host_act_[issued % 2], D_.act, sizeof(pdot::BatchActive), cudaMemcpyDeviceToHost, stream_));
         BCK(cudaEventRecord(ev_[issued % 2], stream_));
@@ -1641,14 +1650,25 @@ class BatchSolver {
   template <typename T>
   T* alloc(size_t count) {
     void* p = nullptr;
-    BCK(cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)));
+    BCK(pdot::device_alloc(&p, std::max<size_t>(count * sizeof(T), 16), stream_));
     allocs_.push_back(p);
     return static_cast<T*>(p);
+  }
+  // a temporary, after the stream has been waited for
+  void drop(void* p) {
+    if (!p) return;
+    allocs_.erase(std::find(allocs_.begin(), allocs_.end(), p));
+    BCK(cudaFree(p));
+  }
+  template <typename T>
+  void put(T* d, const T* src, size_t count) {
+    BCK(cudaMemcpyAsync(d, src, count * sizeof(T), cudaMemcpyHostToDevice, stream_));
+    BCK(cudaStreamSynchronize(stream_));
   }
   template <typename T>
   const T* upload(const T* src, size_t count) {
     T* d = alloc<T>(count);
-    BCK(cudaMemcpy(d, src, count * sizeof(T), cudaMemcpyHostToDevice));
+    put(d, src, count);
     return d;
   }
 
@@ -1757,7 +1777,7 @@ class BatchSolver {
   }
 
   bool regular_start(long long it) const {
-    if (!(graph_ || persistent_) || it <= 10 || (it - 1) % freq_ != 0) return false;
+    if (!(use_graph_ || persistent_) || it <= 10 || (it - 1) % freq_ != 0) return false;
     for (long long k = it + 1; k < it + freq_; ++k)
       if (is_eval(k)) return false;
     return true;
@@ -1765,10 +1785,12 @@ class BatchSolver {
 
   void enqueue_chunk(long long& it) {
     if (regular_start(it)) {
-      if (persistent_)
+      if (persistent_) {
         launch_persistent_chunk();
-      else
+      } else {
+        if (!graph_) capture();  // while the GPU runs the chunk before it
         BCK(cudaGraphLaunch(graph_, stream_));
+      }
       it += freq_;
       return;
     }
@@ -1778,7 +1800,8 @@ class BatchSolver {
       launch_step();
       ++it;
       ++k;
-    } while (k < freq_ && !regular_start(it));
+      // the evaluation at iteration_limit + 1 ends every instance: nothing after it runs
+    } while (k < freq_ && it <= limit_ + 1 && !regular_start(it));
   }
 
   // the regular chunk as one cooperative launch of kb_chunk (bit-identical to the graph)
@@ -1809,8 +1832,26 @@ class BatchSolver {
     for (int k = 0; k < num_; ++k)
       if (st[k].kernel_error)
         bfail(PDOT_ERR_CUDA, "instance %d: the staged primal pass gave up waiting for its copies", k);
-    double* tmp = nullptr;
+    // the duals of all instances in four copies (current and average points)
+    std::vector<double> hu[2], hv[2];
+    bool want_u = false, want_v = false;
     size_t cap = 0;
+    for (int k = 0; k < num_; ++k) {
+      want_u = want_u || outs[k].dual_source_solution;
+      want_v = want_v || outs[k].dual_target_solution;
+      if (outs[k].primal_solution) cap = std::max(cap, (size_t)inst_[k].m * inst_[k].n);
+    }
+    for (int h = 0; h < 2; ++h) {
+      if (want_u) {
+        hu[h].resize(rows_);
+        BCK(cudaMemcpy(hu[h].data(), D_.u[h], rows_ * sizeof(double), cudaMemcpyDeviceToHost));
+      }
+      if (want_v) {
+        hv[h].resize(cols_);
+        BCK(cudaMemcpy(hv[h].data(), D_.v[h], cols_ * sizeof(double), cudaMemcpyDeviceToHost));
+      }
+    }
+    double* tmp = cap ? alloc<double>(cap) : nullptr;
     for (int k = 0; k < num_; ++k) {
       const pdot::BatchInstance& I = inst_[k];
       pdot_batch_output& o = outs[k];
@@ -1820,22 +1861,15 @@ class BatchSolver {
       const int xb = st[k].out_current ? st[k].buf : (st[k].buf ^ 1);
       const size_t mn = (size_t)I.m * I.n;
       if (o.primal_solution) {
-        if (mn > cap) {
-          if (tmp) BCK(cudaFree(tmp));
-          BCK(cudaMalloc(&tmp, mn * sizeof(double)));
-          cap = mn;
-        }
         pdot::kb_widen<<<256, 256, 0, stream_>>>(D_.X[xb] + I.x_off, I.m, I.n, I.ld, tmp);
         BCK(cudaGetLastError());
         BCK(cudaMemcpyAsync(o.primal_solution, tmp, mn * sizeof(double), cudaMemcpyDeviceToHost, stream_));
         BCK(cudaStreamSynchronize(stream_));
       }
-      if (o.dual_source_solution)
-        BCK(cudaMemcpy(o.dual_source_solution, D_.u[xb] + I.row_off, I.m * sizeof(double), cudaMemcpyDeviceToHost));
-      if (o.dual_target_solution)
-        BCK(cudaMemcpy(o.dual_target_solution, D_.v[xb] + I.col_off, I.n * sizeof(double), cudaMemcpyDeviceToHost));
+      if (o.dual_source_solution) memcpy(o.dual_source_solution, hu[xb].data() + I.row_off, I.m * sizeof(double));
+      if (o.dual_target_solution) memcpy(o.dual_target_solution, hv[xb].data() + I.col_off, I.n * sizeof(double));
     }
-    if (tmp) BCK(cudaFree(tmp));
+    drop(tmp);
   }
 
   int device_ = 0, num_ = 0, dim_ = 0, kind_ = 0, grid_ = 1, pr_ = 256, chunk_ctas_ = 0;

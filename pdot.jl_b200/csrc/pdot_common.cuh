@@ -277,6 +277,20 @@ cudaError_t copy_to_device(void* dst, const void* src, size_t bytes, cudaStream_
 using ChunkSource = std::function<const double*(size_t off, size_t count, int slot, cudaStream_t s)>;
 cudaError_t copy_to_host(double* dst, size_t count, const ChunkSource& source, cudaStream_t s);
 
+// Device memory of a solve or a device-level call, for use on `s` (pdot_host.cu):
+// up to kPoolBlock bytes from a pool of this library, larger blocks from
+// cudaMalloc. `pooled` (may be null) says which. cudaFree gives either back,
+// after the work that uses it has ended; cudaFreeAsync a pooled one in stream order.
+constexpr size_t kPoolBlock = size_t(512) << 20;
+cudaError_t device_alloc(void** p, size_t bytes, cudaStream_t s, bool* pooled = nullptr);
+// kPinnedSlot bytes of page-locked host memory for a solve's status reads, from a
+// block that is kept; null when all slots are taken (or page-locking failed), the
+// caller then locks its own.
+constexpr size_t kPinnedSlot = 4096;
+void* pinned_slot_take();
+// Returns a slot; false when `p` is none (the caller's own memory).
+bool pinned_slot_return(void* p);
+
 // Sets the thread-local text pdot_last_error() returns (pdot_host.cu).
 void set_last_error(const char* msg);
 

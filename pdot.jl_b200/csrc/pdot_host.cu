@@ -56,6 +56,110 @@ void check_cuda(cudaError_t e, const char* what, int line) {
 
 namespace pdot {
 void set_last_error(const char* msg) { g_last_error = msg ? msg : ""; }
+
+// Memory kept between calls. A solve allocates some twenty device buffers and a
+// page-locked status block; on B200 the latter cost 1.3-2.5 ms to lock and 0.4 ms to
+// unlock, a 192 MB buffer 0.4 ms each way, now and then 100 ms and more when another
+// process kept the driver, where a 127 x 93 solve of 256 iterations runs for 2 ms.
+//
+// Device blocks come from a pool of this library per device, which the driver trims to
+// kPoolKeep bytes at a synchronisation; a block is ordered on its stream like any
+// cudaMallocAsync block, so calls of several threads and streams never share one in
+// use. (The device's default pool keeps nothing unless the program says so: a small
+// rounding after a synchronisation took 0.5 ms for its scratch.) While a stream is
+// captured the block belongs to the graph. When the pool cannot serve a block it is
+// trimmed and the block taken from cudaMalloc.
+constexpr int kPoolDevices = 64;
+constexpr uint64_t kPoolKeep = uint64_t(1) << 30;
+constexpr int kPinnedSlots = 16;
+
+namespace {
+// never destroyed: the driver may be gone by the time static objects are
+struct Kept {
+  std::mutex mu;
+  cudaMemPool_t pool[kPoolDevices] = {};
+  unsigned char* pinned = nullptr;
+  bool pinned_tried = false;
+  unsigned taken = 0;  // bit k: slot k of `pinned`
+};
+Kept& kept() {
+  static Kept* k = new Kept;
+  return *k;
+}
+
+cudaError_t pool_of(int device, cudaMemPool_t* pool) {
+  Kept& k = kept();
+  std::lock_guard<std::mutex> lock(k.mu);
+  if (!k.pool[device]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t made = nullptr;
+    cudaError_t e = cudaMemPoolCreate(&made, &props);
+    if (e != cudaSuccess) return e;
+    uint64_t keep = kPoolKeep;
+    if ((e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+      cudaMemPoolDestroy(made);
+      return e;
+    }
+    k.pool[device] = made;
+  }
+  *pool = k.pool[device];
+  return cudaSuccess;
+}
+}  // namespace
+
+cudaError_t device_alloc(void** p, size_t bytes, cudaStream_t s, bool* pooled) {
+  if (pooled) *pooled = true;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(s, &capture);
+  if (e != cudaSuccess) return e;
+  if (capture != cudaStreamCaptureStatusNone) return cudaMallocAsync(p, bytes, s);
+  int device = 0;
+  if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;
+  if (bytes <= kPoolBlock && device < kPoolDevices) {
+    cudaMemPool_t pool = nullptr;
+    if ((e = pool_of(device, &pool)) == cudaSuccess) {
+      if ((e = cudaMallocFromPoolAsync(p, bytes, pool, s)) == cudaSuccess) return e;
+      cudaGetLastError();
+      cudaMemPoolTrimTo(pool, 0);
+    }
+    cudaGetLastError();
+  }
+  if (pooled) *pooled = false;
+  return cudaMalloc(p, bytes);
+}
+
+void* pinned_slot_take() {
+  Kept& k = kept();
+  std::lock_guard<std::mutex> lock(k.mu);
+  if (!k.pinned_tried) {
+    k.pinned_tried = true;
+    void* q = nullptr;
+    if (cudaHostAlloc(&q, kPinnedSlots * kPinnedSlot, cudaHostAllocPortable) == cudaSuccess)
+      k.pinned = static_cast<unsigned char*>(q);
+    else
+      cudaGetLastError();
+  }
+  if (!k.pinned) return nullptr;
+  for (int i = 0; i < kPinnedSlots; ++i)
+    if (!(k.taken >> i & 1u)) {
+      k.taken |= 1u << i;
+      return k.pinned + i * kPinnedSlot;
+    }
+  return nullptr;
+}
+
+bool pinned_slot_return(void* p) {
+  Kept& k = kept();
+  std::lock_guard<std::mutex> lock(k.mu);
+  const unsigned char* q = static_cast<const unsigned char*>(p);
+  if (!k.pinned || q < k.pinned || q >= k.pinned + kPinnedSlots * kPinnedSlot) return false;
+  k.taken &= ~(1u << ((q - k.pinned) / kPinnedSlot));
+  return true;
+}
 }  // namespace pdot
 
 namespace {
@@ -231,67 +335,30 @@ pdot::SolveConfig make_config(const pdot_pdhg_parameters& p) {
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// A temporary device buffer freed when it goes out of scope, also when a CK
-// check throws on the way (cudaFree waits for the work that still uses it).
+// A temporary device buffer for work on one stream, freed when it goes out of scope,
+// also when a CK check throws on the way: a pooled block in stream order, another
+// once its work has ended (cudaFree waits for it).
 struct DeviceTemp {
   void* p = nullptr;
+  cudaStream_t s = nullptr;
+  bool pooled = false;
   DeviceTemp() = default;
   DeviceTemp(const DeviceTemp&) = delete;
   DeviceTemp& operator=(const DeviceTemp&) = delete;
   ~DeviceTemp() {
-    if (p) cudaFree(p);
+    if (p) pooled ? cudaFreeAsync(p, s) : cudaFree(p);
+  }
+  cudaError_t alloc(size_t bytes, cudaStream_t stream) {
+    s = stream;
+    const cudaError_t e = pdot::device_alloc(&p, bytes, stream, &pooled);
+    if (e != cudaSuccess) p = nullptr;
+    return e;
   }
   template <typename T>
   T* get() const {
     return static_cast<T*>(p);
   }
 };
-
-// Stream-ordered scratch of the device-level calls, from a pool of this library on
-// the current device that keeps at most kPoolKeep bytes between calls. The
-// device's default pool gives its memory back at every synchronisation unless
-// the program asked otherwise, so that a call after one paid for mapping its
-// scratch again: 0.5 ms and more, where a small rounding takes 0.03 ms. The
-// allocation is ordered on the stream like any other, so calls of several threads
-// and streams never share a block in use. While a stream is captured the
-// allocation belongs to the graph, as one of cudaMallocAsync does.
-constexpr int kPoolDevices = 64;
-constexpr uint64_t kPoolKeep = uint64_t(32) << 20;
-
-struct ScratchPools {
-  std::mutex mu;
-  cudaMemPool_t pool[kPoolDevices] = {};
-};
-
-cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
-  static ScratchPools* pools = new ScratchPools;  // never destroyed: the driver may be gone by then
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  cudaError_t e = cudaStreamIsCapturing(s, &capture);
-  if (e != cudaSuccess) return e;
-  int device = 0;
-  if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;
-  if (capture != cudaStreamCaptureStatusNone || device >= kPoolDevices) return cudaMallocAsync(p, bytes, s);
-  cudaMemPool_t pool = nullptr;
-  {
-    std::lock_guard<std::mutex> lock(pools->mu);
-    pool = pools->pool[device];
-    if (!pool) {
-      cudaMemPoolProps props = {};
-      props.allocType = cudaMemAllocationTypePinned;
-      props.handleTypes = cudaMemHandleTypeNone;
-      props.location.type = cudaMemLocationTypeDevice;
-      props.location.id = device;
-      if ((e = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return e;
-      uint64_t keep = kPoolKeep;
-      if ((e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
-        cudaMemPoolDestroy(pool);
-        return e;
-      }
-      pools->pool[device] = pool;
-    }
-  }
-  return cudaMallocFromPoolAsync(p, bytes, pool, s);
-}
 
 int64_t pass_workspace_bytes(const pdot::Geometry& g) {
   return (int64_t)(pdot::pass_scratch_doubles(g) * sizeof(double));
@@ -314,6 +381,13 @@ class Solver {
   Solver(const pdot_problem& P, bool device_inputs, const pdot_pdhg_parameters& prm,
          const pdot_solver_options* opt)
       : params_(prm) {
+    // what a failing constructor holds goes back, the kept slots and pool blocks among it
+    struct Undo {
+      Solver* s;
+      ~Undo() {
+        if (s) s->release();
+      }
+    } undo{this};
     const Variant var = read_options(P, opt);
     device_ = var.device;
     use_graph_ = var.use_graph;
@@ -356,12 +430,11 @@ class Solver {
     } else {
       const size_t cbytes = var.cost_kind == PDOT_COST_F32 ? 4 : 2;
       void* Cs = nullptr;
-      CK(cudaMalloc(&Cs, std::max<size_t>(N, 1) * cbytes));
-      allocs_.push_back(Cs);
+      Cs = alloc_bytes(N * cbytes);
       const double* src = P.cost_matrix;
       DeviceTemp tmp;
       if (!device_inputs) {
-        CK(cudaMalloc(&tmp.p, N * sizeof(double)));
+        CK(tmp.alloc(N * sizeof(double), stream_));
         CK(pdot::copy_to_device(tmp.p, P.cost_matrix, N * sizeof(double), stream_));
         src = tmp.get<const double>();
       }
@@ -401,11 +474,10 @@ class Solver {
       pi.ld = m;
       pi.active = 1;
       const long long pre[4] = {0, (long long)m, 0, (long long)n};
-      void* p = nullptr;
-      CK(cudaMalloc(&p, sizeof(pi) + sizeof(pre)));
-      allocs_.push_back(p);
-      CK(cudaMemcpy(p, &pi, sizeof(pi), cudaMemcpyHostToDevice));
-      CK(cudaMemcpy(static_cast<char*>(p) + sizeof(pi), pre, sizeof(pre), cudaMemcpyHostToDevice));
+      void* p = alloc_bytes(sizeof(pi) + sizeof(pre));
+      CK(cudaMemcpyAsync(p, &pi, sizeof(pi), cudaMemcpyHostToDevice, stream_));
+      CK(cudaMemcpyAsync(static_cast<char*>(p) + sizeof(pi), pre, sizeof(pre), cudaMemcpyHostToDevice, stream_));
+      CK(cudaStreamSynchronize(stream_));
       double *f = nullptr, *gg = nullptr;
       alloc(&f, m);
       alloc(&gg, n);
@@ -422,16 +494,14 @@ class Solver {
     }
     if (var.warm_x) {
       // the warm plan in plan precision, and its row and column sums
-      void* wx = nullptr;
-      CK(cudaMalloc(&wx, std::max<size_t>(N, 1) * xbytes));
-      allocs_.push_back(wx);
+      void* wx = alloc_bytes(N * xbytes);
       warm_x_ = wx;
       alloc(&warm_r_, m);
       alloc(&warm_c_, n);
       const double* src = var.warm_x;
       DeviceTemp tmp, work;
       if (!device_inputs) {
-        CK(cudaMalloc(&tmp.p, std::max<size_t>(N, 1) * sizeof(double)));
+        CK(tmp.alloc(N * sizeof(double), stream_));
         CK(pdot::copy_to_device(tmp.p, var.warm_x, N * sizeof(double), stream_));
         src = tmp.get<const double>();
       }
@@ -439,16 +509,11 @@ class Solver {
         CK(pdot::launch_convert_cost(src, wx, PDOT_COST_F32, N, stream_));
       else
         CK(cudaMemcpyAsync(wx, src, N * sizeof(double), cudaMemcpyDeviceToDevice, stream_));
-      CK(cudaMalloc(&work.p, std::max<size_t>(pdot::plan_sums_workspace_doubles(m, n), 1) * sizeof(double)));
+      CK(work.alloc(std::max<size_t>(pdot::plan_sums_workspace_doubles(m, n), 1) * sizeof(double), stream_));
       CK(pdot::launch_plan_sums(m, n, wx, var.plan_f32, warm_r_, warm_c_, work.get<double>(), stream_));
       CK(cudaStreamSynchronize(stream_));
     }
-    void* xp = nullptr;
-    for (int k = 0; k < 2; ++k) {
-      CK(cudaMalloc(&xp, std::max<size_t>(N, 1) * xbytes));
-      allocs_.push_back(xp);
-      X_[k] = xp;
-    }
+    for (int k = 0; k < 2; ++k) X_[k] = alloc_bytes(N * xbytes);
     xbytes_ = xbytes;
     for (int k = 0; k < 2; ++k) {
       alloc(&u_[k], m);
@@ -457,15 +522,12 @@ class Solver {
       alloc(&c_[k], n);
     }
     alloc(&work_, pdot::workspace_doubles(g_));
-    void* p = nullptr;
-    CK(cudaMalloc(&p, sizeof(pdot::DevState)));
-    allocs_.push_back(p);
-    st_ = static_cast<pdot::DevState*>(p);
-    CK(cudaMalloc(&p, sizeof(pdot_iteration_stats) * kRingCap));
-    allocs_.push_back(p);
-    ring_ = static_cast<pdot_iteration_stats*>(p);
-    CK(cudaMallocHost(&p, sizeof(pdot::DevState) * kInFlight));
-    host_status_ = static_cast<pdot::DevState*>(p);
+    st_ = static_cast<pdot::DevState*>(alloc_bytes(sizeof(pdot::DevState)));
+    ring_ = static_cast<pdot_iteration_stats*>(alloc_bytes(sizeof(pdot_iteration_stats) * kRingCap));
+    static_assert(sizeof(pdot::DevState) * kInFlight <= pdot::kPinnedSlot, "the status records fit a slot");
+    void* hp = pdot::pinned_slot_take();
+    if (!hp) CK(cudaMallocHost(&hp, sizeof(pdot::DevState) * kInFlight));
+    host_status_ = static_cast<pdot::DevState*>(hp);
     for (int k = 0; k < kInFlight; ++k) CK(cudaEventCreateWithFlags(&ev_[k], cudaEventDisableTiming));
 
     B_.cost = cost_;
@@ -519,11 +581,14 @@ class Solver {
     // at every size tried (31 against 16 us per iteration at 1000 x 1000, 1071
     // against 718 at 10000 x 10000)
     persistent_ = g_.chunk_ctas > 0 && !time_kernels_ && var.persistent == 1;
-    if (use_graph_ && !time_kernels_ && !persistent_) capture_regular_chunk();
+    use_graph_ = use_graph_ && !time_kernels_ && !persistent_;
     reset();
+    undo.s = nullptr;
   }
 
-  ~Solver() {
+  ~Solver() { release(); }
+
+  void release() {
     if (stream_) cudaStreamSynchronize(stream_);
     if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
     for (int k = 0; k < kInFlight; ++k) {
@@ -537,7 +602,7 @@ class Solver {
       cudaEventDestroy(t.start);
       cudaEventDestroy(t.stop);
     }
-    if (host_status_) cudaFreeHost(host_status_);
+    if (host_status_ && !pdot::pinned_slot_return(host_status_)) cudaFreeHost(host_status_);
     for (void* p : allocs_) cudaFree(p);
     if (stream_) cudaStreamDestroy(stream_);
   }
@@ -595,7 +660,8 @@ class Solver {
     int64_t remaining = max_iterations;
     int issued = 0, completed = 0;
     while (!status_.done && (remaining > 0 || issued > completed)) {
-      while (issued - completed < kInFlight && remaining > 0 && !status_.done) {
+      while (issued - completed < kInFlight && remaining > 0 && !status_.done &&
+             (issued == completed || host_it_ <= limit_ + 1)) {
         const int slot = issued % kInFlight;
         remaining -= enqueue_chunk(remaining, slot);
         CK(cudaMemcpyAsync(&host_status_[slot], st_, sizeof(pdot::DevState), cudaMemcpyDeviceToHost, stream_));
@@ -681,7 +747,7 @@ class Solver {
         // widen the FP32 plan chunk by chunk into two device buffers
         const size_t chunk = std::min<size_t>(N, pdot::kTransferChunk);
         DeviceTemp tmp;
-        CK(cudaMalloc(&tmp.p, 2 * std::max<size_t>(chunk, 1) * sizeof(double)));
+        CK(tmp.alloc(2 * std::max<size_t>(chunk, 1) * sizeof(double), stream_));
         const float* Xf = static_cast<const float*>(X_[xb]);
         double* buf = tmp.get<double>();
         CK(pdot::copy_to_host(out->primal_solution, N,
@@ -734,10 +800,13 @@ class Solver {
  private:
   template <typename T>
   void alloc(T** p, size_t count) {
+    *p = static_cast<T*>(alloc_bytes(count * sizeof(T)));
+  }
+  void* alloc_bytes(size_t bytes) {
     void* q = nullptr;
-    CK(cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T)));
+    CK(pdot::device_alloc(&q, std::max<size_t>(bytes, 16), stream_));
     allocs_.push_back(q);
-    *p = static_cast<T*>(q);
+    return q;
   }
 
   bool is_eval(long long it) const { return (it - 1) % freq_ == 0 || it == limit_ + 1 || it <= 10; }
@@ -746,7 +815,7 @@ class Solver {
   // kernel: evaluation at its first iteration only, and no forced evaluation
   // (iteration_limit + 1) inside.
   bool regular_start(long long it) const {
-    if (!(graph_exec_ || persistent_) || it <= 10 || (it - 1) % freq_ != 0) return false;
+    if (!(use_graph_ || persistent_) || it <= 10 || (it - 1) % freq_ != 0) return false;
     for (long long k = it + 1; k < it + freq_; ++k)
       if (is_eval(k)) return false;
     return true;
@@ -788,10 +857,14 @@ class Solver {
   // Enqueues up to `budget` loop bodies starting at host_it_; returns how many.
   int64_t enqueue_chunk(int64_t budget, int slot) {
     if (regular_start(host_it_) && budget >= freq_) {
-      if (persistent_)
+      if (persistent_) {
         CK(pdot::launch_chunk(B_, g_, cfg_, stream_, (int)freq_));
-      else
+      } else {
+        // captured on first use, while the GPU runs the chunk before it: capture,
+        // instantiation and upload take 0.8 ms of host time
+        if (!graph_exec_) capture_regular_chunk();
         CK(cudaGraphLaunch(graph_exec_, stream_));
+      }
       host_it_ += freq_;
       return freq_;
     }
@@ -800,7 +873,8 @@ class Solver {
       enqueue_iteration(host_it_, slot);
       ++host_it_;
       ++k;
-    } while (k < freq_ && k < budget && !regular_start(host_it_));
+      // the evaluation at iteration_limit + 1 ends the solve: nothing after it runs
+    } while (k < freq_ && k < budget && host_it_ <= limit_ + 1 && !regular_start(host_it_));
     return k;
   }
 
@@ -852,12 +926,13 @@ class Solver {
     const long long total = status_.num_stats;
     if (total <= drained_) return;
     if (total - drained_ > kRingCap) fail(PDOT_ERR_CUDA, "iteration-stats ring overflow");
-    for (long long k = drained_; k < total; ++k) {
-      pdot_iteration_stats rec;
-      CK(cudaMemcpy(&rec, ring_ + (k % kRingCap), sizeof(rec), cudaMemcpyDeviceToHost));
-      records_.push_back(rec);
+    while (drained_ < total) {  // at most two pieces: up to the ring's end, and from its start
+      const long long at = drained_ % kRingCap, count = std::min<long long>(total - drained_, kRingCap - at);
+      records_.resize(records_.size() + count);
+      CK(cudaMemcpy(records_.data() + records_.size() - count, ring_ + at, count * sizeof(pdot_iteration_stats),
+                    cudaMemcpyDeviceToHost));
+      drained_ += count;
     }
-    drained_ = total;
   }
 
   int device_ = 0;
@@ -1052,12 +1127,9 @@ int pdot_rounding_f64(int64_t m, int64_t n, const double* source, const double* 
     if (m < 1 || n < 1) fail(PDOT_ERR_INVALID_ARGUMENT, "empty matrix");
     if (!source || !target || !plan) fail(PDOT_ERR_INVALID_ARGUMENT, "null pointer argument");
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
-    double* work = nullptr;
-    CK(scratch_alloc(reinterpret_cast<void**>(&work), pdot::rounding_workspace_doubles(m, n) * sizeof(double), s));
-    const cudaError_t e = pdot::launch_rounding(m, n, source, target, plan, work, s);
-    const cudaError_t e2 = cudaFreeAsync(work, s);
-    CK(e);
-    CK(e2);
+    DeviceTemp work;
+    CK(work.alloc(pdot::rounding_workspace_doubles(m, n) * sizeof(double), s));
+    CK(pdot::launch_rounding(m, n, source, target, plan, work.get<double>(), s));
   });
 }
 
