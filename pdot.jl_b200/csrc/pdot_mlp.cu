@@ -21,6 +21,14 @@
 //
 // The loss is the mean squared error over the output entries of the real rows
 // of the batch. All reductions (loss, bias gradients) are in a fixed order.
+//
+// A training step of 256 rows (2048 -> 1024 -> 1024 -> 2048) takes 127 us on B200, 305
+// before the transposed copies went through shared memory, the bias gradients, AdamW
+// and the loss took one parallel launch each and the kernels were launched dependent on
+// one another: features 5, split products 4 x 15, the output layer's 11, weight
+// gradients 7 each, loss 6, bias gradients 5, AdamW 32 us. The products are bound by
+// latency (their bytes take 1 to 3 us from L2), AdamW by its bytes.
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -47,7 +55,7 @@ namespace {
 #ifndef PDOT_MLP_SPLIT_K
 #define PDOT_MLP_SPLIT_K 1
 #endif
-constexpr int kGemmThreads = 128;
+constexpr int kGemmThreads = 256;  // two warps per 32 accumulator rows: the epilogues are latency-bound
 constexpr int kBM = 128;  // rows of A per tile (= TMEM lanes)
 constexpr int kBN = 128;  // rows of B per tile (= accumulator columns)
 constexpr int kBK = 64;   // K per stage: one 128-byte swizzle row of BF16
@@ -70,8 +78,6 @@ struct Epi {
   const float* bias;           // N
   const float* z;              // saved pre-activation, row-major (ld_z)
   int64_t ld_f32, ld_bf16, ld_t, ld_z;
-  float* part;                 // split K: slice z of the partial products at part + z * M * N (row-major M x N)
-  int64_t part_m, part_n;      // M and N of the product
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
@@ -140,6 +146,12 @@ __device__ __forceinline__ float gelu_grad(float z) {
   return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
 
+__device__ __forceinline__ void store_f32x8(float* p, const float* v) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+               "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
+
 // The fused epilogue of W (a multiple of 4) accumulator columns [col, col + W)
 // of one row.
 template <int EPI, int W>
@@ -160,31 +172,53 @@ __device__ __forceinline__ void epilogue_cols(const Epi& ep, int64_t row, int64_
     }
   }
   float* fo = ep.f32 + row * ep.ld_f32 + col;
+  if constexpr (W % 8 == 0) {
 #pragma unroll
-  for (int k = 0; k < W; k += 4) *reinterpret_cast<float4*>(fo + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+    for (int k = 0; k < W; k += 8) store_f32x8(fo + k, v + k);  // whole sectors
+  } else {
+#pragma unroll
+    for (int k = 0; k < W; k += 4) *reinterpret_cast<float4*>(fo + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+  }
   if (EPI == EPI_BIAS_GELU || EPI == EPI_GELU_BWD) {
     __align__(16) __nv_bfloat16 h[W];
 #pragma unroll
     for (int k = 0; k < W; ++k) h[k] = __float2bfloat16_rn(EPI == EPI_BIAS_GELU ? gelu(v[k]) : v[k]);
     if (ep.bf16) {
       __nv_bfloat16* bo = ep.bf16 + row * ep.ld_bf16 + col;
+      if constexpr (W % 8 == 0) {
 #pragma unroll
-      for (int k = 0; k < W; k += 4) *reinterpret_cast<uint2*>(bo + k) = *reinterpret_cast<const uint2*>(h + k);
+        for (int k = 0; k < W; k += 8) *reinterpret_cast<uint4*>(bo + k) = *reinterpret_cast<const uint4*>(h + k);
+      } else {
+#pragma unroll
+        for (int k = 0; k < W; k += 4) *reinterpret_cast<uint2*>(bo + k) = *reinterpret_cast<const uint2*>(h + k);
+      }
     }
 #pragma unroll
     for (int k = 0; k < W; ++k) ep.bf16_t[(col + k) * ep.ld_t + row] = h[k];
   }
 }
 
-// One 128 x 128 tile of D = A B^T per CTA; K a multiple of kBK. With
-// gridDim.z = S > 1 (split K), CTA z multiplies the K blocks
-// [z * KB / S, (z + 1) * KB / S) and writes its raw partial tile to slice z of
-// ep.part; k_splitk_finish then adds the slices in order and runs the
-// epilogue. Products with few output tiles (the batch is 256 rows) thus
-// spread over the SMs instead of 16 of them.
+// One 128 x 128 tile of D = A B^T per CTA; K a multiple of kBK. With split > 1 the K
+// blocks are cut into `split` slices, slice z the blocks [z * KB / split, (z + 1) * KB /
+// split), and a cluster of gridDim.z CTAs shares the tile, each with split / gridDim.z
+// neighbouring slices in accumulators of their own: products with few output tiles (the
+// batch is 256 rows) thus spread over the SMs instead of 16 of them. The CTAs leave
+// their partial tiles in shared memory; each then adds its share of the rows over the
+// cluster, slice by slice in order, and runs their epilogue. (With the partial tiles in
+// global memory and a second kernel for the ordered sum, 256 x 1024 x 2048 took 8.9 +
+// 6.3 us.)
+constexpr int kMaxSplit = 16;
+constexpr int kTileF4 = kBN / 4;  // float4 columns of a tile
+static_assert(2 * kBM * kBN * 4 <= kStages * kStageBytes, "two partial tiles fit the ring");
+// Float4 slot of (row, column group) of a partial tile: lanes of a warp hold the same
+// group of 32 rows when they write and neighbouring rows when they read; the exclusive
+// or spreads both over the banks.
+__device__ __forceinline__ int tile_slot(int row, int c4) { return row * kTileF4 + (c4 ^ (row & (kTileF4 - 1))); }
+
 template <int EPI>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-    k_gemm(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, int K, Epi ep, int* err) {
+    k_gemm(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, int K, int split, Epi ep,
+           int* err) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_addr(smem_raw);
   const uint32_t tiles = (raw + 1023u) & ~1023u;  // the swizzle atoms need 1024-byte alignment
@@ -198,9 +232,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * kBN;
   const int kb_all = K / kBK;
-  const int kb0 = (int)((long long)blockIdx.z * kb_all / gridDim.z);
-  const int kblocks = (int)((long long)(blockIdx.z + 1) * kb_all / gridDim.z) - kb0;
+  const int per = split / (int)gridDim.z;  // slices of this CTA, 1 or 2
+  auto slice_begin = [&](int z) { return (int)((long long)z * kb_all / split); };
+  const int z0 = (int)blockIdx.z * per;
+  const int kb0 = slice_begin(z0), kblocks = slice_begin(z0 + per) - kb0;
+  const int cut = slice_begin(z0 + 1) - kb0;  // first K block of the second slice
+  const uint32_t tmem_cols = (uint32_t)(per * kBN);
   if (threadIdx.x == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&ta)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tb)) : "memory");
     s_err = 0;
     for (int s = 0; s < kStages; ++s) {
       mbar_init(full(s), 1);
@@ -211,7 +251,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   }
   if (warp == 2) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)),
-                 "r"(kBN)
+                 "r"(tmem_cols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -219,6 +259,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  pdl_enter();  // barriers and accumulators are set up while the kernel before this one ends
 
   if (warp == 0 && lane == 0) {
     // producer: TMA loads of the A and B tiles of each K block
@@ -251,7 +292,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const uint64_t db = sw128_kmajor_desc(tiles + s * kStageBytes + kTileABytes);
 #pragma unroll
       for (int kk = 0; kk < kBK / kUmmaK; ++kk)  // +32 bytes along the swizzled row per K step
-        umma_bf16(tmem, da + (uint64_t)(2 * kk), db + (uint64_t)(2 * kk), (kb | kk) != 0 ? 1u : 0u);
+        umma_bf16(tmem + (kb >= cut ? (uint32_t)kBN : 0u), da + (uint64_t)(2 * kk), db + (uint64_t)(2 * kk),
+                  (kb != 0 && kb != cut) || kk != 0 ? 1u : 0u);
       umma_commit(empty(s));
     }
     umma_commit(done);
@@ -261,165 +303,325 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   __syncwarp();
   tc_fence_after();
 
-  // epilogue: thread (warp w, lane l) owns accumulator row 32 w + l
-  const int64_t row = m0 + warp * 32 + lane;
-  const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-  const bool split = gridDim.z > 1;
-#pragma unroll 1
-  for (int c0 = 0; c0 < kBN; c0 += 16) {
-    float v[16];
-    tmem_ld16(lane_base + (uint32_t)c0, v);
-    const int64_t col = n0 + c0;
-    if (split) {
-      float* po = ep.part + ((int64_t)blockIdx.z * ep.part_m + row) * ep.part_n + col;
-#pragma unroll
-      for (int k = 0; k < 16; k += 4) *reinterpret_cast<float4*>(po + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
-    } else {
-      epilogue_cols<EPI, 16>(ep, row, col, v);
+  // thread (warp w, lane l) owns half a row of the accumulator: row 32 (w mod 4) + l,
+  // columns from (w / 4) kBN / 2
+  const int trow = (warp & 3) * 32 + lane, tcol = (warp >> 2) * (kBN / 2);
+  const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  if (split == 1) {
+#pragma unroll 2
+    for (int c0 = tcol; c0 < tcol + kBN / 2; c0 += 16) {
+      float v[16];
+      tmem_ld16(lane_base + (uint32_t)c0, v);
+      epilogue_cols<EPI, 16>(ep, m0 + trow, n0 + c0, v);
     }
+  } else {
+    // the ring is free: every copy has landed and every product has read it
+    float4* tile = reinterpret_cast<float4*>(smem_raw + (tiles - raw));
+    for (int t = 0; t < per; ++t) {
+#pragma unroll 2
+      for (int c0 = tcol; c0 < tcol + kBN / 2; c0 += 16) {
+        float v[16];
+        tmem_ld16(lane_base + (uint32_t)(t * kBN + c0), v);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          tile[t * kBM * kTileF4 + tile_slot(trow, c0 / 4 + k)] =
+              make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+      }
+    }
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+    // lanes on neighbouring rows (the transposed BF16 copy's stores coalesce), two
+    // column groups per warp (the row-major ones fill their sectors)
+    const int rows = kBM / (int)gridDim.z;  // 16 and more
+    const int two = per - 1;                // log2 of the slices per CTA
+#pragma unroll 2
+    for (int item = threadIdx.x; item < rows * kTileF4; item += kGemmThreads) {
+      const int c4 = (item >> 4) & (kTileF4 - 1);
+      const int r = (int)blockIdx.z * rows + (item / (16 * kTileF4)) * 16 + (item & 15);
+      const int slot = tile_slot(r, c4);
+      float4 q[kMaxSplit];
+#pragma unroll
+      for (int z = 0; z < kMaxSplit; ++z)
+        if (z < split) q[z] = cluster.map_shared_rank(tile, z >> two)[(z & two) * kBM * kTileF4 + slot];
+      float v[4] = {q[0].x, q[0].y, q[0].z, q[0].w};
+#pragma unroll
+      for (int z = 1; z < kMaxSplit; ++z)
+        if (z < split) v[0] += q[z].x, v[1] += q[z].y, v[2] += q[z].z, v[3] += q[z].w;
+      epilogue_cols<EPI, 4>(ep, m0 + r, n0 + 4 * c4, v);
+    }
+    cluster.sync();  // no CTA leaves while its tile is read
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 2) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kBN) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols) : "memory");
   }
   if (threadIdx.x == 0 && s_err != 0) atomicCAS(err, 0, s_err);
 }
 
-// Split K: D = the sum of the S partial slices in order z = 0, 1, ..., then the
-// epilogue; a thread per (row, 4 columns), consecutive threads on consecutive
-// rows (the transposed BF16 copy's stores coalesce). The slices' loads are
-// issued together (S <= kMaxSplit), the additions keep their order.
-constexpr int kMaxSplit = 16;
-template <int EPI>
-__global__ void __launch_bounds__(256) k_splitk_finish(Epi ep, int S) {
-  const int64_t M = ep.part_m, N = ep.part_n, total = M * (N / 4);
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = t % M, col = (t / M) * 4;
-    float4 q[kMaxSplit];
-#pragma unroll
-    for (int z = 0; z < kMaxSplit; ++z)
-      if (z < S) q[z] = __ldcs(reinterpret_cast<const float4*>(ep.part + ((int64_t)z * M + row) * N + col));
-    float v[4] = {q[0].x, q[0].y, q[0].z, q[0].w};
-#pragma unroll
-    for (int z = 1; z < kMaxSplit; ++z)
-      if (z < S) v[0] += q[z].x, v[1] += q[z].y, v[2] += q[z].z, v[3] += q[z].w;
-    epilogue_cols<EPI, 4>(ep, row, col, v);
-  }
-}
-
 constexpr int kEw = 256;  // threads of the elementwise kernels
 
+// Tiles of kTr x kTr entries of a row-major matrix whose BF16 form is also stored
+// transposed: the tile goes through shared memory, so that both copies are written in
+// whole sectors. (Written entry by entry, the transposed copy took a 32-byte sector
+// for 2 bytes and most of these kernels' time.) Rows and columns are multiples of kTr.
+constexpr int kTr = 64;
+struct TransposeTile {
+  __nv_bfloat16 h[kTr][kTr + 2];
+};
+// the 4 x 4 entries of a thread: rows (t >> 4) + 16 k, columns 4 (t & 15) ...
+__device__ __forceinline__ void tile_put(TransposeTile& T, int r, int c, const __nv_bfloat16 (&b)[4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) T.h[r][c + e] = b[e];
+}
+// dst[(c0 + c) * ld + r0 + r] for the whole tile; 16 rows of a column per thread
+__device__ __forceinline__ void tile_write_transposed(const TransposeTile& T, __nv_bfloat16* dst, int64_t ld,
+                                                      int64_t r0, int64_t c0) {
+  const int c = threadIdx.x >> 2, r = (threadIdx.x & 3) * 16;
+  __align__(16) __nv_bfloat16 o[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) o[e] = T.h[r + e][c];
+  uint4* p = reinterpret_cast<uint4*>(dst + (c0 + c) * ld + r0 + r);
+  p[0] = reinterpret_cast<const uint4*>(o)[0];
+  p[1] = reinterpret_cast<const uint4*>(o)[1];
+}
+__device__ __forceinline__ void store_bf16x4(__nv_bfloat16* p, const __nv_bfloat16 (&b)[4]) {
+  uint2 w;
+  memcpy(&w, b, 8);
+  *reinterpret_cast<uint2*>(p) = w;
+}
+
 // x[r, k] = bf16((log(max(h, 1e-30)) + shift) * scale) for real rows, 0 for the
-// padding rows up to bp; also the transposed copy xt (leading dimension ld_t).
-__global__ void k_features(const double* __restrict__ hist, int64_t batch, int64_t bp, int64_t dim, double shift,
-                           double scale, __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ xt,
-                           int64_t ld_t) {
-  const int64_t N = bp * dim;
-  for (int64_t e = (int64_t)blockIdx.x * kEw + threadIdx.x; e < N; e += (int64_t)gridDim.x * kEw) {
-    const int64_t r = e / dim, k = e - r * dim;
+// padding rows up to bp; also the transposed copy xt (leading dimension ld_t). A CTA
+// takes kTr rows of kFeatCols columns, four FP64 logarithms a thread: their latency,
+// not the bytes, is what counts, so the tiles are narrow and many.
+constexpr int kFeatCols = 16;
+__global__ void __launch_bounds__(kEw) k_features(const double* __restrict__ hist, int64_t batch, int64_t dim,
+                                                  double shift, double scale, __nv_bfloat16* __restrict__ x,
+                                                  __nv_bfloat16* __restrict__ xt, int64_t ld_t) {
+  __shared__ __nv_bfloat16 T[kTr][kFeatCols + 2];
+  pdl_enter();
+  const int64_t r0 = (int64_t)blockIdx.y * kTr, c0 = (int64_t)blockIdx.x * kFeatCols;
+  const int r = threadIdx.x >> 2, c = 4 * (threadIdx.x & 3);
+  __align__(8) __nv_bfloat16 b[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
     double f = 0.0;
-    if (r < batch) {
-      const double h = hist[e];
+    if (r0 + r < batch) {
+      const double h = hist[(r0 + r) * dim + c0 + c + e];
       f = (log(h > 1e-30 ? h : 1e-30) + shift) * scale;
     }
-    const __nv_bfloat16 b = __double2bfloat16(f);
-    x[e] = b;
-    xt[k * ld_t + r] = b;
+    b[e] = __double2bfloat16(f);
+    T[r][c + e] = b[e];
   }
+  store_bf16x4(x + (r0 + r) * dim + c0 + c, b);
+  __syncthreads();
+  const int tc = threadIdx.x >> 4, tr = 4 * (threadIdx.x & 15);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) b[e] = T[tr + e][tc];
+  store_bf16x4(xt + (c0 + tc) * ld_t + r0 + tr, b);
 }
 
 // dY = 2 (Y - T) / (batch * O) on real rows (0 on padding), its BF16 copy and
 // transpose, and per-CTA partial sums of (Y - T)^2.
-__global__ void k_loss(const float* __restrict__ y, const float* __restrict__ t, int64_t batch, int64_t bp,
-                       int64_t dim, float* __restrict__ dy, __nv_bfloat16* __restrict__ dyb,
-                       __nv_bfloat16* __restrict__ dyt, int64_t ld_t, double* __restrict__ part) {
-  const int64_t N = bp * dim;
+__global__ void __launch_bounds__(kEw) k_loss(const float* __restrict__ y, const float* __restrict__ t, int64_t batch,
+                                              int64_t dim, float* __restrict__ dy, __nv_bfloat16* __restrict__ dyb,
+                                              __nv_bfloat16* __restrict__ dyt, int64_t ld_t,
+                                              double* __restrict__ part) {
+  __shared__ TransposeTile T;
+  __shared__ double sh[kEw / 32];
+  pdl_enter();
+  const int64_t r0 = (int64_t)blockIdx.y * kTr, c0 = (int64_t)blockIdx.x * kTr;
+  const int c = 4 * (threadIdx.x & 15);
   const float g = 2.0f / (float)(batch * dim);
   double acc = 0.0;
-  for (int64_t e = (int64_t)blockIdx.x * kEw + threadIdx.x; e < N; e += (int64_t)gridDim.x * kEw) {
-    const int64_t r = e / dim, k = e - r * dim;
-    float d = 0.0f;
-    if (r < batch) {
-      const float diff = y[e] - t[e];
-      acc += (double)diff * (double)diff;
-      d = g * diff;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int r = (threadIdx.x >> 4) + 16 * k;
+    const int64_t at = (r0 + r) * dim + c0 + c;
+    float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (r0 + r < batch) {
+      const float4 yv = *reinterpret_cast<const float4*>(y + at);
+      float tv[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) tv[e] = t[at + e];  // the caller's array: any alignment
+      const float diff[4] = {yv.x - tv[0], yv.y - tv[1], yv.z - tv[2], yv.w - tv[3]};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        acc += (double)diff[e] * (double)diff[e];
+        d[e] = g * diff[e];
+      }
     }
-    dy[e] = d;
-    const __nv_bfloat16 b = __float2bfloat16_rn(d);
-    dyb[e] = b;
-    dyt[k * ld_t + r] = b;
+    *reinterpret_cast<float4*>(dy + at) = make_float4(d[0], d[1], d[2], d[3]);
+    __align__(8) __nv_bfloat16 b[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) b[e] = __float2bfloat16_rn(d[e]);
+    store_bf16x4(dyb + at, b);
+    tile_put(T, r, c, b);
   }
-  __shared__ double sh[kEw];
-  sh[threadIdx.x] = acc;
+  acc = warp_sum(acc);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
   __syncthreads();
-  for (int w = kEw / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-    __syncthreads();
+  tile_write_transposed(T, dyt, ld_t, r0, c0);
+  if (threadIdx.x == 0) {
+    double s = sh[0];
+#pragma unroll
+    for (int w = 1; w < kEw / 32; ++w) s += sh[w];
+    part[blockIdx.y * gridDim.x + blockIdx.x] = s;
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-__global__ void k_loss_total(const double* __restrict__ part, int parts, int64_t count, double* __restrict__ loss) {
-  if (threadIdx.x != 0) return;
+// One CTA: thread t adds partials t, t + kEw, ..., then a tree (50 us by one thread).
+__global__ void __launch_bounds__(kEw) k_loss_total(const double* __restrict__ part, int parts, int64_t count,
+                                                    double* __restrict__ loss) {
+  __shared__ double sh[kEw / 32];
+  pdl_enter();
   double s = 0.0;
-  for (int k = 0; k < parts; ++k) s += part[k];
-  *loss = s / (double)count;
+  for (int k = threadIdx.x; k < parts; k += kEw) s += part[k];
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < kEw / 32; ++w) s += sh[w];
+    *loss = s / (double)count;
+  }
 }
 
-// out[c] = sum over the first `rows` rows of in[r, c] (bias gradients)
-__global__ void k_colsum(const float* __restrict__ in, int64_t rows, int64_t cols, float* __restrict__ out) {
-  const int64_t c = (int64_t)blockIdx.x * kEw + threadIdx.x;
-  if (c >= cols) return;
+// The bias gradients of all layers: out[c] = sum over the first `rows` rows of in[r, c].
+// A CTA takes 32 columns of one layer with 16 row groups side by side, added in order
+// (one thread per column, a launch per layer: 25 us each at 256 rows).
+constexpr int kColGroups = 16;
+struct ColSums {
+  const float* in[3];
+  float* out[3];
+  int blocks[3];  // CTAs of each layer: columns / 32
+  int64_t cols[3];
+};
+__global__ void __launch_bounds__(32 * kColGroups) k_colsum(ColSums S, int64_t rows) {
+  __shared__ double sh[kColGroups][32];
+  pdl_enter();
+  int l = 0, b = blockIdx.x;
+  while (b >= S.blocks[l]) b -= S.blocks[l++];
+  const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
+  const int64_t cols = S.cols[l], c = (int64_t)b * 32 + lane;
+  const float* in = S.in[l] + c;
   double s = 0.0;
-  for (int64_t r = 0; r < rows; ++r) s += (double)in[r * cols + c];
-  out[c] = (float)s;
+#pragma unroll 8
+  for (int64_t r = grp; r < rows; r += kColGroups) s += (double)in[r * cols];
+  sh[grp][lane] = s;
+  __syncthreads();
+  if (grp == 0) {
+#pragma unroll
+    for (int g = 1; g < kColGroups; ++g) s += sh[g][lane];
+    S.out[l][c] = (float)s;
+  }
 }
 
-// AdamW on one tensor (rows x cols; a bias has rows = 1 and no BF16 copies):
+// AdamW on every tensor in one launch: CTAs of kTr x kTr tiles of the three weight
+// matrices, then CTAs of kEw entries of the three biases (no decay, no BF16 copies).
 // m = b1 m + (1 - b1) g, v = b2 v + (1 - b2) g^2,
 // p -= lr (m / (1 - b1^t) / (sqrt(v / (1 - b2^t)) + eps) + wd p);
-// then the BF16 copy and its transpose.
-__global__ void k_adamw(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                        float* __restrict__ v, int64_t rows, int64_t cols, float lr, float b1, float b2, float eps,
-                        float wd, float c1, float c2, __nv_bfloat16* __restrict__ pb,
-                        __nv_bfloat16* __restrict__ pt) {
-  const int64_t N = rows * cols;
-  for (int64_t e = (int64_t)blockIdx.x * kEw + threadIdx.x; e < N; e += (int64_t)gridDim.x * kEw) {
-    const float gr = g[e];
-    const float mm = b1 * m[e] + (1.0f - b1) * gr;
-    const float vv = b2 * v[e] + (1.0f - b2) * gr * gr;
-    m[e] = mm;
-    v[e] = vv;
-    const float upd = (mm / c1) / (sqrtf(vv / c2) + eps) + wd * p[e];
-    const float np = p[e] - lr * upd;
-    p[e] = np;
-    if (pb) {
-      const __nv_bfloat16 b = __float2bfloat16_rn(np);
-      pb[e] = b;
-      const int64_t r = e / cols, c = e - r * cols;
-      pt[c * rows + r] = b;
+// then the BF16 copy and its transpose. Bound by the 32 B per parameter it streams: 32 us for
+// 5.2 M parameters on B200, 82 us with a launch per tensor and the transposes entry by entry.
+struct AdamTensors {
+  float* p[3];         // weights
+  const float* g[3];
+  float* m[3];
+  float* v[3];
+  __nv_bfloat16* pb[3];
+  __nv_bfloat16* pt[3];
+  int64_t rows[3], cols[3];
+  int tiles[3];
+  float* bp[3];        // biases, rows[l] entries
+  const float* bg[3];
+  float* bm[3];
+  float* bv[3];
+  int bias_blocks[3];
+};
+struct AdamStep {
+  float lr, b1, b2, eps, wd, c1, c2;
+};
+__device__ __forceinline__ float adamw_entry(const AdamStep& A, float wd, float p, float gr, float& m, float& v) {
+  const float mm = A.b1 * m + (1.0f - A.b1) * gr;
+  const float vv = A.b2 * v + (1.0f - A.b2) * gr * gr;
+  m = mm;
+  v = vv;
+  const float upd = (mm / A.c1) / (sqrtf(vv / A.c2) + A.eps) + wd * p;
+  return p - A.lr * upd;
+}
+__global__ void __launch_bounds__(kEw) k_adamw(AdamTensors T, AdamStep A) {
+  __shared__ TransposeTile tile;
+  pdl_enter();
+  int l = 0, b = blockIdx.x;
+  while (l < 3 && b >= T.tiles[l]) b -= T.tiles[l++];
+  if (l == 3) {  // a bias
+    l = 0;
+    while (b >= T.bias_blocks[l]) b -= T.bias_blocks[l++];
+    const int64_t e = (int64_t)b * kEw + threadIdx.x;
+    if (e < T.rows[l]) {
+      float m = T.bm[l][e], v = T.bv[l][e];
+      T.bp[l][e] = adamw_entry(A, 0.0f, T.bp[l][e], T.bg[l][e], m, v);
+      T.bm[l][e] = m;
+      T.bv[l][e] = v;
     }
+    return;
   }
+  const int64_t rows = T.rows[l], cols = T.cols[l], across = cols / kTr;
+  const int64_t r0 = b / across * kTr, c0 = b % across * kTr;
+  const int c = 4 * (threadIdx.x & 15);
+  float4 p[4], g[4], m[4], v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int64_t at = (r0 + (threadIdx.x >> 4) + 16 * k) * cols + c0 + c;
+    p[k] = *reinterpret_cast<const float4*>(T.p[l] + at);
+    g[k] = *reinterpret_cast<const float4*>(T.g[l] + at);
+    m[k] = *reinterpret_cast<const float4*>(T.m[l] + at);
+    v[k] = *reinterpret_cast<const float4*>(T.v[l] + at);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int r = (threadIdx.x >> 4) + 16 * k;
+    const int64_t at = (r0 + r) * cols + c0 + c;
+    p[k].x = adamw_entry(A, A.wd, p[k].x, g[k].x, m[k].x, v[k].x);
+    p[k].y = adamw_entry(A, A.wd, p[k].y, g[k].y, m[k].y, v[k].y);
+    p[k].z = adamw_entry(A, A.wd, p[k].z, g[k].z, m[k].z, v[k].z);
+    p[k].w = adamw_entry(A, A.wd, p[k].w, g[k].w, m[k].w, v[k].w);
+    *reinterpret_cast<float4*>(T.p[l] + at) = p[k];
+    *reinterpret_cast<float4*>(T.m[l] + at) = m[k];
+    *reinterpret_cast<float4*>(T.v[l] + at) = v[k];
+    const __nv_bfloat16 h[4] = {__float2bfloat16_rn(p[k].x), __float2bfloat16_rn(p[k].y), __float2bfloat16_rn(p[k].z),
+                                __float2bfloat16_rn(p[k].w)};
+    store_bf16x4(T.pb[l] + at, h);
+    tile_put(tile, r, c, h);
+  }
+  __syncthreads();
+  tile_write_transposed(tile, T.pt[l], rows, r0, c0);
 }
 
 // BF16 copies (and transposes) of the weight matrices from the FP32 masters.
-__global__ void k_to_bf16(const float* __restrict__ p, int64_t rows, int64_t cols, __nv_bfloat16* __restrict__ pb,
-                          __nv_bfloat16* __restrict__ pt) {
-  const int64_t N = rows * cols;
-  for (int64_t e = (int64_t)blockIdx.x * kEw + threadIdx.x; e < N; e += (int64_t)gridDim.x * kEw) {
-    const __nv_bfloat16 b = __float2bfloat16_rn(p[e]);
-    pb[e] = b;
-    const int64_t r = e / cols, c = e - r * cols;
-    pt[c * rows + r] = b;
+__global__ void __launch_bounds__(kEw) k_to_bf16(const float* __restrict__ p, int64_t rows, int64_t cols,
+                                                 __nv_bfloat16* __restrict__ pb, __nv_bfloat16* __restrict__ pt) {
+  __shared__ TransposeTile T;
+  pdl_enter();
+  const int64_t r0 = (int64_t)blockIdx.y * kTr, c0 = (int64_t)blockIdx.x * kTr;
+  const int c = 4 * (threadIdx.x & 15);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int r = (threadIdx.x >> 4) + 16 * k;
+    const int64_t at = (r0 + r) * cols + c0 + c;
+    const float4 w = *reinterpret_cast<const float4*>(p + at);
+    const __nv_bfloat16 h[4] = {__float2bfloat16_rn(w.x), __float2bfloat16_rn(w.y), __float2bfloat16_rn(w.z),
+                                __float2bfloat16_rn(w.w)};
+    store_bf16x4(pb + at, h);
+    tile_put(T, r, c, h);
   }
+  __syncthreads();
+  tile_write_transposed(T, pt, rows, r0, c0);
 }
 
-int ew_grid(int64_t n) {
-  int64_t g = (n + kEw - 1) / kEw;
-  return (int)(g < 1 ? 1 : (g > 148 * 8 ? 148 * 8 : g));
-}
+dim3 tile_grid(int64_t rows, int64_t cols) { return dim3((unsigned)(cols / kTr), (unsigned)(rows / kTr)); }
 
 }  // namespace
 }  // namespace pdot
@@ -511,7 +713,6 @@ struct pdot_mlp {
   bf16 *dyb = nullptr, *dyt = nullptr, *dz2b = nullptr, *dz2t = nullptr, *dz1t = nullptr;
   double *loss_part = nullptr, *loss = nullptr;
   int* err = nullptr;
-  float* part = nullptr;  // split-K partial products: at most one 128 x 128 tile per SM
   int sms = 148;
   int loss_parts = 0;
   int64_t batch = 0;  // rows of the current input
@@ -533,11 +734,16 @@ struct pdot_mlp {
     if (stream) cudaStreamDestroy(stream);
   }
 
+  // the network's kernels are launched with programmatic dependent launch (pdot::pdl_launch)
+  template <typename... P, typename... A>
+  void launch(void (*kfn)(P...), dim3 grid, A... args) {
+    MCK(pdot::pdl_launch(kfn, grid, dim3(pdot::kEw), 0, stream, P(args)...));
+  }
+
   void sync_bf16() {
     const int64_t rows[3] = {H, H, O}, cols[3] = {I, H, H};
     for (int l = 0; l < 3; ++l)
-      pdot::k_to_bf16<<<pdot::ew_grid(rows[l] * cols[l]), pdot::kEw, 0, stream>>>(W[l], rows[l], cols[l], Wb[l], Wt[l]);
-    MCK(cudaGetLastError());
+      launch(pdot::k_to_bf16, pdot::tile_grid(rows[l], cols[l]), W[l], rows[l], cols[l], Wb[l], Wt[l]);
   }
 
   void check_err() {
@@ -558,28 +764,30 @@ struct pdot_mlp {
     MCK(cudaFuncSetAttribute(pdot::k_gemm<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, pdot::kGemmSmem));
     // split K where the tiles cover at most an eighth of the SMs (the batch's
     // 256-row products with a 1024-wide output), while the slices fill at
-    // most every SM and each keeps at least two K blocks. Measured per launch
-    // (ncu, cold cache) for 256 x 1024 x 2048: 8.9 us + 6.3 us for the
-    // ordered sum and epilogue, against 22.5 us in one K loop; 256 x 2048 x
-    // 1024 (32 tiles) split in four measured 16.6 us against 14.4 us, so it
-    // stays whole, as do the weight gradients (64 and more tiles).
+    // most every SM and each keeps at least two K blocks. 256 x 2048 x 1024 (32
+    // tiles) split in four measured 16.6 us against 14.4 us whole, so it and the
+    // weight gradients (64 and more tiles) are not split.
     const int64_t tiles = (N / pdot::kBN) * (M / pdot::kBM), kb = K / pdot::kBK;
     int S = 1;
     if (PDOT_MLP_SPLIT_K && tiles * 8 <= sms)
       while (tiles * S * 2 <= sms && kb / (S * 2) >= 2 && S * 2 <= pdot::kMaxSplit) S *= 2;
-    const dim3 grid((unsigned)(N / pdot::kBN), (unsigned)(M / pdot::kBM), (unsigned)S);
-    pdot::Epi e = ep;
-    e.part = part;
-    e.part_m = M;
-    e.part_n = N;
-    pdot::k_gemm<EPI><<<grid, pdot::kGemmThreads, pdot::kGemmSmem, stream>>>(a, bm, (int)K, e, err);
-    MCK(cudaGetLastError());
-    if (S > 1) {
-      const int64_t threads = M * (N / 4);
-      const int blocks = (int)std::min<int64_t>((threads + 255) / 256, (int64_t)sms * 8);
-      pdot::k_splitk_finish<EPI><<<blocks, 256, 0, stream>>>(e, S);
-      MCK(cudaGetLastError());
-    }
+    // eight slices to four CTAs, two each: 16 clusters of eight wait for room on the
+    // GPCs (20 us a product against 14)
+    const int ctas = S >= 8 ? S / 2 : S;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)(N / pdot::kBN), (unsigned)(M / pdot::kBM), (unsigned)ctas);
+    c.blockDim = dim3(pdot::kGemmThreads);
+    c.dynamicSmemBytes = pdot::kGemmSmem;
+    c.stream = stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = PDOT_PDL;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = at[1].val.clusterDim.y = 1;
+    at[1].val.clusterDim.z = c.gridDim.z;
+    c.attrs = at;
+    c.numAttrs = 2;
+    MCK(cudaLaunchKernelEx(&c, pdot::k_gemm<EPI>, a, bm, (int)K, S, ep, err));
   }
 
   int64_t padded(int64_t rows) const { return (rows + pdot::kBM - 1) / pdot::kBM * pdot::kBM; }
@@ -597,11 +805,12 @@ struct pdot_mlp {
     gemm<pdot::EPI_BIAS>(mh2, mW[2], bp, O, H, e);
   }
 
-  void backward(const float* target) {
+  // want_loss: the caller reads `loss` afterwards
+  void backward(const float* target, bool want_loss) {
     const int64_t bp = padded(batch);
-    pdot::k_loss<<<loss_parts, pdot::kEw, 0, stream>>>(y, target, batch, bp, O, dy, dyb, dyt, Bp, loss_part);
-    pdot::k_loss_total<<<1, 32, 0, stream>>>(loss_part, loss_parts, batch * O, loss);
-    MCK(cudaGetLastError());
+    const dim3 lg = pdot::tile_grid(bp, O);
+    launch(pdot::k_loss, lg, y, target, batch, O, dy, dyb, dyt, Bp, loss_part);
+    if (want_loss) launch(pdot::k_loss_total, dim3(1), loss_part, (int)(lg.x * lg.y), batch * O, loss);
     // the transposed operands were written with leading dimension Bp; the
     // products over the batch read the first bp columns of them
     pdot::Epi e{};
@@ -619,25 +828,27 @@ struct pdot_mlp {
     e = pdot::Epi{};
     e.f32 = gW[0]; e.ld_f32 = I;
     gemm<pdot::EPI_F32>(mdz1t, mxt, H, I, bp, e);
-    pdot::k_colsum<<<(unsigned)((O + pdot::kEw - 1) / pdot::kEw), pdot::kEw, 0, stream>>>(dy, bp, O, gb[2]);
-    pdot::k_colsum<<<(unsigned)((H + pdot::kEw - 1) / pdot::kEw), pdot::kEw, 0, stream>>>(dz2, bp, H, gb[1]);
-    pdot::k_colsum<<<(unsigned)((H + pdot::kEw - 1) / pdot::kEw), pdot::kEw, 0, stream>>>(dz1, bp, H, gb[0]);
-    MCK(cudaGetLastError());
+    pdot::ColSums cs{{dy, dz2, dz1}, {gb[2], gb[1], gb[0]}, {(int)(O / 32), (int)(H / 32), (int)(H / 32)}, {O, H, H}};
+    MCK(pdot::pdl_launch(pdot::k_colsum, dim3((unsigned)((O + 2 * H) / 32)), dim3(32 * pdot::kColGroups), 0, stream, cs,
+                         bp));
   }
 
   void adamw(float lr, float b1_, float b2_, float eps, float wd) {
     ++step;
     const float c1 = 1.0f - powf(b1_, (float)step), c2 = 1.0f - powf(b2_, (float)step);
     const int64_t rows[3] = {H, H, O}, cols[3] = {I, H, H};
+    pdot::AdamTensors t{};
+    unsigned blocks = 0;
     for (int l = 0; l < 3; ++l) {
       const int64_t off_w = W[l] - theta, off_b = b[l] - theta;
-      pdot::k_adamw<<<pdot::ew_grid(rows[l] * cols[l]), pdot::kEw, 0, stream>>>(
-          W[l], grad + off_w, m1 + off_w, m2 + off_w, rows[l], cols[l], lr, b1_, b2_, eps, wd, c1, c2, Wb[l], Wt[l]);
-      pdot::k_adamw<<<pdot::ew_grid(rows[l]), pdot::kEw, 0, stream>>>(b[l], grad + off_b, m1 + off_b, m2 + off_b, 1,
-                                                                      rows[l], lr, b1_, b2_, eps, 0.0f, c1, c2,
-                                                                      nullptr, nullptr);
+      t.p[l] = W[l], t.g[l] = grad + off_w, t.m[l] = m1 + off_w, t.v[l] = m2 + off_w;
+      t.pb[l] = Wb[l], t.pt[l] = Wt[l], t.rows[l] = rows[l], t.cols[l] = cols[l];
+      t.tiles[l] = (int)(rows[l] / pdot::kTr * (cols[l] / pdot::kTr));
+      t.bp[l] = b[l], t.bg[l] = grad + off_b, t.bm[l] = m1 + off_b, t.bv[l] = m2 + off_b;
+      t.bias_blocks[l] = (int)((rows[l] + pdot::kEw - 1) / pdot::kEw);
+      blocks += (unsigned)(t.tiles[l] + t.bias_blocks[l]);
     }
-    MCK(cudaGetLastError());
+    launch(pdot::k_adamw, dim3(blocks), t, pdot::AdamStep{lr, b1_, b2_, eps, wd, c1, c2});
   }
 };
 
@@ -732,11 +943,10 @@ extern "C" int pdot_mlp_create(int32_t device, int64_t input_dim, int64_t hidden
     m->dz2t = m->alloc<bf16>(H * Bp);
     m->dz1 = m->alloc<float>(Bp * H);
     m->dz1t = m->alloc<bf16>(H * Bp);
-    m->loss_parts = pdot::ew_grid(Bp * O);
+    m->loss_parts = (int)(Bp / pdot::kTr * (O / pdot::kTr));
     m->loss_part = m->alloc<double>(m->loss_parts);
     m->loss = m->alloc<double>(1);
     m->err = m->alloc<int>(1);
-    m->part = m->alloc<float>((size_t)m->sms * pdot::kBM * pdot::kBN);
     // initial weights and biases uniform in +-1/sqrt(fan_in)
     std::vector<float> h(P);
     uint64_t s = seed;
@@ -822,9 +1032,7 @@ extern "C" int pdot_mlp_set_input(pdot_mlp* m, int64_t batch, const double* hist
     m->batch = batch;
     const int64_t bp = m->padded(batch);
     // rows past bp stay as they are: no product reads them
-    pdot::k_features<<<pdot::ew_grid(bp * m->I), pdot::kEw, 0, m->stream>>>(histograms, batch, bp, m->I, shift, scale,
-                                                                           m->x, m->xt, m->Bp);
-    MCK(cudaGetLastError());
+    m->launch(pdot::k_features, dim3((unsigned)(m->I / pdot::kFeatCols), (unsigned)(bp / pdot::kTr)), histograms, batch, m->I, shift, scale, m->x, m->xt, m->Bp);
   });
 }
 
@@ -843,7 +1051,7 @@ extern "C" int pdot_mlp_backward(pdot_mlp* m, const float* target, double* loss)
   return mguarded([&] {
     if (!m || !target || m->batch < 1) mfail(PDOT_ERR_INVALID_ARGUMENT, "bad arguments");
     MCK(cudaSetDevice(m->device));
-    m->backward(target);
+    m->backward(target, loss != nullptr);
     if (loss) MCK(cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->stream));
     m->check_err();
   });
@@ -862,7 +1070,7 @@ extern "C" int pdot_mlp_train_step(pdot_mlp* m, const float* target, float lr, f
     if (!m || !target || m->batch < 1) mfail(PDOT_ERR_INVALID_ARGUMENT, "bad arguments");
     MCK(cudaSetDevice(m->device));
     m->forward();
-    m->backward(target);
+    m->backward(target, loss != nullptr);
     m->adamw(lr, 0.9f, 0.999f, 1e-8f, weight_decay);
     if (loss) {
       MCK(cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->stream));

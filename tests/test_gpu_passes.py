@@ -164,3 +164,38 @@ def test_recovered_plans_of_a_batch_whose_groups_cross_instances(cuda):
         C = instances.l1_cost(x.astype(np.float32).astype(np.float64), y.astype(np.float32).astype(np.float64))
         want, _, _ = oracle.warm_plan(C, p.source_distribution, p.target_distribution, w[0], w[1], eps, rounds)
         np.testing.assert_allclose(o.primal_solution, want, rtol=1e-3, atol=1e-12)
+
+
+@pytest.mark.parametrize("dims,batch", [((128, 128, 128), 1), ((2048, 128, 128), 130), ((1024, 256, 384), 257),
+                                        ((4096, 128, 256), 128), ((256, 1024, 512), 513)])
+def test_network_step_at_odd_shapes(cuda, dims, batch):
+    """A training step against the network's oracle for products split 1 to 16 ways over a cluster and for
+    batches that end inside a tile: outputs to 1e-3 and gradients to 1e-2 in the 2-norm, as at full size,
+    and the loss, summed in FP64 over FP32 differences, to 1e-4."""
+    import mlp_oracle as mo
+    import torch
+
+    from pdot import learned
+
+    I, H, O = dims
+    rng = np.random.default_rng(I + batch)
+    net = learned.MLP(I, H, O, max_batch=batch, seed=3)
+    hist = np.exp(rng.normal(size=(batch, I)))
+    hist /= hist.sum(1, keepdims=True)
+    target = rng.normal(size=(batch, O)).astype(np.float32)
+    h, t = torch.from_numpy(hist).to(cuda), torch.from_numpy(target).to(cuda)
+    y = torch.zeros((batch, O), dtype=torch.float32, device=cuda)
+    theta = net.get_parameters()
+    torch.cuda.synchronize()
+    net.set_input(h.data_ptr(), batch)
+    net.forward(y.data_ptr())
+    loss = net.backward(t.data_ptr())
+    x = mo.features(hist, learned.FEATURE_SHIFT, learned.FEATURE_SCALE)
+    want_y, _ = mo.forward(theta, x, I, H, O)
+    want_loss, want_g = mo.loss_and_gradients(theta, x, target, I, H, O)
+    assert np.linalg.norm(y.cpu().numpy() - want_y) <= 1e-3 * np.linalg.norm(want_y)
+    assert loss == pytest.approx(want_loss, rel=1e-4)
+    g = net.gradients()
+    sizes = [H * I, H, H * H, H, O * H, O]
+    for name, lo, k in zip(["W1", "b1", "W2", "b2", "W3", "b3"], np.cumsum([0] + sizes), sizes):
+        assert np.linalg.norm(g[lo : lo + k] - want_g[lo : lo + k]) <= 1e-2 * np.linalg.norm(want_g[lo : lo + k]), name
