@@ -183,8 +183,10 @@ typedef struct pdot_solver_options {
   /* Regular chunks of loop bodies (the evaluation and the steps up to the next
    * one) as one persistent cooperative launch with grid barriers between the
    * phases, instead of a CUDA graph of separate launches; the results are
-   * bit-identical. 0: automatic (the CUDA graph, which measured faster on
-   * B200), 1: whenever the direct 16-byte pass runs, -1: never. The batched
+   * bit-identical. 0: automatic (for problems whose plan, average and cost fit
+   * the SMs' shared memory, the steps between two evaluations as one such launch
+   * with them resident there; else, or with use_cuda_graph 0, as for -1), 1:
+   * whenever the direct 16-byte pass runs, -1: never. The batched
    * solver takes it too: 1 runs its regular chunks (evaluation, compaction,
    * steps) as one persistent launch with the direct pass throughout (the
    * staged pass is then refused). */

@@ -210,6 +210,14 @@ cudaError_t launch_step(const Buffers& B, const Geometry& g, const SolveConfig& 
 // one persistent cooperative launch (needs g.chunk_ctas > 0); bit-identical to
 // launch_eval followed by the steps.
 cudaError_t launch_chunk(const Buffers& B, const Geometry& g, const SolveConfig& cfg, cudaStream_t s, int steps);
+// `steps` steps of a small problem as one cooperative launch of `ctas` CTAs with the
+// plan and cost in shared memory (pdot_resident.cu), bit-identical to launch_step so
+// often; `scratch` is device memory of the caller's. resident_ctas: the CTAs, 0 where
+// the problem does not fit.
+int resident_ctas(const Geometry& g, int device);
+size_t resident_scratch_bytes();
+cudaError_t launch_resident(const Buffers& B, const Geometry& g, const SolveConfig& cfg, cudaStream_t s, int ctas,
+                            int steps, void* scratch);
 // start_only = 1: a warm start's initial point becomes the last restart
 // point; nothing else of the evaluation block runs.
 cudaError_t launch_eval(const Buffers& B, const Geometry& g, const SolveConfig& cfg, cudaStream_t s,

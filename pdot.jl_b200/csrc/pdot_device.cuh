@@ -31,9 +31,9 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 }
 
 // Base.max(x, 0.0): NaN propagates, -0.0 becomes 0.0.
-__device__ __forceinline__ double jl_max0(double x) { return x > 0.0 ? x : (x != x ? x : 0.0); }
+__device__ __forceinline__ double jl_max0(double x) { return !(x <= 0.0) ? x : 0.0; }
 // |min(x, 0.0)| with NaN propagating.
-__device__ __forceinline__ double neg_part(double x) { return x < 0.0 ? -x : (x != x ? x : 0.0); }
+__device__ __forceinline__ double neg_part(double x) { return !(x >= 0.0) ? -x : 0.0; }
 // Base.min(x, y) for Float64.
 __device__ __forceinline__ double jl_min(double x, double y) {
   if (x != x) return x;
@@ -378,7 +378,7 @@ struct CostReader<PDOT_COST_BF16, R, RPL> : StoredCost<__nv_bfloat16, R, RPL> {
 // multiply-adds where the drop-in rounds twice. The step d between the two
 // stored values is formed exactly in FP64, so the FP64 row, column and
 // squared-norm sums the caller accumulates add exactly what was stored.
-__device__ __forceinline__ float jl_max0f(float x) { return x > 0.0f ? x : (x != x ? x : 0.0f); }
+__device__ __forceinline__ float jl_max0f(float x) { return !(x <= 0.0f) ? x : 0.0f; }
 
 // The sum of squared steps: the FP64 plan rounds the product and the sum as
 // the reference does; an FP32 plan's sum takes one fused multiply-add.
@@ -567,53 +567,57 @@ struct UnitCursor {
 // (the kernels use solver_state.step_size, not the shrunk local step), so the
 // candidate computed once is the accepted one; a rejection only adds an
 // attempt to the counters and one more application of the shrink rule.
-// First-attempt powers of the step-size rule, computed by a spare warp while
-// the finishing CTA's other warps reduce the partial sums: (k + 1)^e for the
-// iteration count k that the first attempt sees.
+// The first attempt's factors of the step-size rule, 1 - (k + 1)^-e and 1 + (k + 1)^-e
+// for the iteration count k that it sees, and 0.5 / omega: taken by a spare warp
+// while the finishing CTA's other warps reduce the partial sums.
 struct StepPowers {
-  double k1 = -1.0, reduction = 0.0, growth = 0.0;
+  double k1 = -1.0, shrink = 0.0, grow = 0.0, half_over_omega = 0.0;
 };
+__device__ __forceinline__ double step_shrink(const SolveConfig& cfg, double k1) {
+  return __dsub_rn(1.0, __ddiv_rn(1.0, powd(k1, cfg.reduction_exponent)));
+}
+__device__ __forceinline__ double step_grow(const SolveConfig& cfg, double k1) {
+  return __dadd_rn(1.0, __ddiv_rn(1.0, powd(k1, cfg.growth_exponent)));
+}
 __device__ __forceinline__ StepPowers step_powers(const DevState* st, const SolveConfig& cfg) {
   StepPowers p;
   p.k1 = (double)(st->total_iters + 2);
-  p.reduction = powd(p.k1, cfg.reduction_exponent);
-  p.growth = powd(p.k1, cfg.growth_exponent);
+  p.shrink = step_shrink(cfg, p.k1);
+  p.grow = step_grow(cfg, p.k1);
+  p.half_over_omega = __ddiv_rn(0.5, st->primal_weight);
   return p;
 }
 
-__device__ void step_control(DevState* st, const SolveConfig& cfg, double dot_r, double dot_c, double dx2,
-                             double dy2, const StepPowers& pre = StepPowers()) {
-  const double omega = st->primal_weight;
+// The movement of a step, from the norms of its two parts.
+__device__ __forceinline__ double step_movement(double omega, double half_over_omega, double ndp, double ndd) {
+  return __dadd_rn(__dmul_rn(__dmul_rn(0.5, omega), __dmul_rn(ndp, ndp)), __dmul_rn(half_over_omega, __dmul_rn(ndd, ndd)));
+}
+__device__ __forceinline__ double step_limit(double movement, double interaction) {
+  return interaction > 0.0 ? __ddiv_rn(movement, interaction) : INFINITY;
+}
+
+// The attempts of the adaptive rule (or the constant step's counters) and the update of
+// the state.
+__device__ __forceinline__ void step_attempts(DevState* st, const SolveConfig& cfg, double interaction,
+                                              double movement, double limit, const StepPowers& pre) {
   const double weight = st->step_size;
   const bool fresh = !(st->sum_weights > 0.0);
   bool accepted = true;
   if (cfg.adaptive) {
-    const double interaction = fabs(dot_r + dot_c);
-    const double ndp = sqrt(dx2), ndd = sqrt(dy2);
-    const double movement = __dadd_rn(__dmul_rn(__dmul_rn(0.5, omega), __dmul_rn(ndp, ndp)),
-                                      __dmul_rn(__ddiv_rn(0.5, omega), __dmul_rn(ndd, ndd)));
     double tau = st->step_size;
     accepted = false;
     for (int attempt = 0; attempt < 64; ++attempt) {
       st->total_iters += 1;
       st->kkt_passes += 1.0;
-      double limit;
-      if (interaction > 0.0) {
-        limit = __ddiv_rn(movement, interaction);
-        if (movement == 0.0) {
-          st->numerical_error = 1;
-          break;
-        }
-      } else {
-        limit = INFINITY;
+      if (interaction > 0.0 && movement == 0.0) {
+        st->numerical_error = 1;
+        break;
       }
       if (tau <= limit) accepted = true;
       const double k1 = (double)(st->total_iters + 1);
       const bool have = k1 == pre.k1;
-      const double pr = have ? pre.reduction : powd(k1, cfg.reduction_exponent);
-      const double pg = have ? pre.growth : powd(k1, cfg.growth_exponent);
-      const double first_term = __dmul_rn(__dsub_rn(1.0, __ddiv_rn(1.0, pr)), limit);
-      const double second_term = __dmul_rn(__dadd_rn(1.0, __ddiv_rn(1.0, pg)), tau);
+      const double first_term = __dmul_rn(have ? pre.shrink : step_shrink(cfg, k1), limit);
+      const double second_term = __dmul_rn(have ? pre.grow : step_grow(cfg, k1), tau);
       tau = jl_min(first_term, second_term);
       if (accepted) break;
       // the reference loops forever on a NaN limit; stop with a numerical error
@@ -635,6 +639,13 @@ __device__ void step_control(DevState* st, const SolveConfig& cfg, double dot_r,
   st->primal_passes += 1;
   st->fresh_passes += fresh ? 1 : 0;
   st->iteration += 1;
+}
+
+__device__ void step_control(DevState* st, const SolveConfig& cfg, double dot_r, double dot_c, double dx2,
+                             double dy2, const StepPowers& pre) {
+  const double interaction = fabs(dot_r + dot_c);
+  const double movement = step_movement(st->primal_weight, pre.half_over_omega, sqrt(dx2), sqrt(dy2));
+  step_attempts(st, cfg, interaction, movement, step_limit(movement, interaction), pre);
 }
 
 struct DualArgs {

@@ -366,6 +366,7 @@ int64_t pass_workspace_bytes(const pdot::Geometry& g) {
 
 constexpr int kRingCap = 4096;
 constexpr int kInFlight = 2;
+constexpr int kResidentSteps = 4;  // fewest steps of a resident launch
 
 
 enum TimedKind { kTimedPrimal = 0, kTimedDual = 1, kTimedEval = 2 };
@@ -582,6 +583,11 @@ class Solver {
     // against 718 at 10000 x 10000)
     persistent_ = g_.chunk_ctas > 0 && !time_kernels_ && var.persistent == 1;
     use_graph_ = use_graph_ && !time_kernels_ && !persistent_;
+    // small problems: the steps between two evaluations as one launch with the plan in
+    // shared memory, bit-identical to the graph's
+    if (use_graph_ && var.persistent == 0 && !g_.fail_waits && freq_ >= kResidentSteps)
+      resident_ = pdot::resident_ctas(g_, device_);
+    if (resident_) resident_scratch_ = alloc_bytes(pdot::resident_scratch_bytes());
     reset();
     undo.s = nullptr;
   }
@@ -856,6 +862,18 @@ class Solver {
 
   // Enqueues up to `budget` loop bodies starting at host_it_; returns how many.
   int64_t enqueue_chunk(int64_t budget, int slot) {
+    if (resident_ && host_it_ >= 10) {
+      // the evaluation due now, then every step up to the next one in one launch (a
+      // launch of a few steps would spend more on filling shared memory)
+      int64_t k = 1;
+      while (k < budget && !is_eval(host_it_ + k)) ++k;
+      if (k >= kResidentSteps || host_it_ > limit_) {
+        if (is_eval(host_it_)) CK(pdot::launch_eval(B_, g_, cfg_, stream_));
+        if (host_it_ <= limit_) CK(pdot::launch_resident(B_, g_, cfg_, stream_, resident_, (int)k, resident_scratch_));
+        host_it_ += k;
+        return k;
+      }
+    }
     if (regular_start(host_it_) && budget >= freq_) {
       if (persistent_) {
         CK(pdot::launch_chunk(B_, g_, cfg_, stream_, (int)freq_));
@@ -874,7 +892,8 @@ class Solver {
       ++host_it_;
       ++k;
       // the evaluation at iteration_limit + 1 ends the solve: nothing after it runs
-    } while (k < freq_ && k < budget && host_it_ <= limit_ + 1 && !regular_start(host_it_));
+    } while (k < freq_ && k < budget && host_it_ <= limit_ + 1 && !regular_start(host_it_) &&
+             !(resident_ && host_it_ >= 10));
     return k;
   }
 
@@ -938,6 +957,8 @@ class Solver {
   int device_ = 0;
   bool use_graph_ = true, time_kernels_ = false;
   bool persistent_ = false;  // regular chunks run as one persistent launch
+  int resident_ = 0;         // CTAs of the resident steps, 0: the problem does not fit
+  void* resident_scratch_ = nullptr;
   pdot_pdhg_parameters params_;
   pdot::Geometry g_{};
   pdot::SolveConfig cfg_{};
