@@ -34,6 +34,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "pdot_device.cuh"
@@ -382,6 +383,12 @@ __global__ void __launch_bounds__(kThreads, Tile<PR>::kMinBlocks) kb_primal(Batc
 // zero in the plan and in the stored cost. Every wait is bounded: on a timeout
 // the kernel sets kernel_error of the instance at hand, drains (bounded) the
 // copies in flight and leaves its remaining units alone.
+//
+// Full panels of an instance with a gradient and an average run straight-line code,
+// without a test per row: 163 -> 146 us a pass over 48 instances of 1024 x 1024 on B200
+// (150 us at the rate of an in-place update of two matrices), 603 -> 595 us over the 512
+// uneven ones, most of whose panels are ragged. Two columns a stage, which halve the
+// waits and cursors, measured 146 and 637 us: the second column's state spills.
 template <int CK, int PR>
 struct BatchStagedLayout {
   static constexpr bool kPts = is_point_cost(CK);
@@ -568,34 +575,18 @@ __global__ void __launch_bounds__(kThreads, Tile<PR>::kMinBlocks) kb_primal_stag
         if (!zero_g) vnext = __ldg(v + jb + warp);
         cost.prefetch(jb + warp);
       }
-      for (long long j = jb + warp; !failed && j < je; j += kWarps) {
-        const int stage = cstage;
-        const uint32_t parity = cphase;
-        if (!mbar_wait_bounded(bar0 + 8 * stage, parity)) {
-          failed = true;
-          if (lane == 0) {
-            atomicExch(&st->kernel_error, 1);
-            atomicExch(&B.act->error, 1);
-          }
-          break;
-        }
-        const unsigned char* stg = ring + (size_t)stage * L::kStageBytes;
+      // one unit; PLAIN: a full panel, a gradient and an average (straight-line code)
+      double csk[kBRPL];
+      auto unit = [&](auto plain, const unsigned char* stg, float vj, long long col) {
+        constexpr bool PLAIN = decltype(plain)::value;
         const float* sC = reinterpret_cast<const float*>(stg);
         const float* sX = reinterpret_cast<const float*>(stg + L::kCBytes);
         const float* sXa = reinterpret_cast<const float*>(stg + L::kCBytes + L::kXBytes);
-        const float vj = (float)vnext;
-        cost.take();
-        if (j + kWarps < je) {
-          if (!zero_g) vnext = __ldg(v + j + kWarps);
-          cost.prefetch(j + kWarps);
-        }
-        const long long col = j * I.ld + row0 + lane * kBR;
-        double csk[kBRPL];
 #pragma unroll
         for (int kq = 0; kq < kBRPL; ++kq) csk[kq] = 0.0;
 #pragma unroll
         for (int kq = 0; kq < kBRPL; ++kq) {
-          if (ok[kq]) {
+          if (PLAIN || ok[kq]) {
             const int r = kq * 32 * kBR + lane * kBR;
             typename CostReader<CK, kBR, kBRPL>::value_t cv[kBR];
             if constexpr (L::kPts)
@@ -604,12 +595,13 @@ __global__ void __launch_bounds__(kThreads, Tile<PR>::kMinBlocks) kb_primal_stag
               vld<float, kBR>(sC + r, cv);
             float xv[kBR], av[kBR];
             vld<float, kBR>(sX + r, xv);
-            if (!first) vld<float, kBR>(sXa + r, av);
+            if (PLAIN || !first) vld<float, kBR>(sXa + r, av);
 #pragma unroll
             for (int e = 0; e < kBR; ++e) {
-              if (e < nv[kq]) {
+              if (PLAIN || e < nv[kq]) {
                 double d;
-                primal_entry<float>(widen(cv[e]), ur[kq][e], vj, s, nw, aw, zero_g, first, xv[e], av[e], d);
+                primal_entry<float>(widen(cv[e]), ur[kq][e], vj, s, nw, aw, !PLAIN && zero_g, !PLAIN && first, xv[e],
+                                    av[e], d);
                 acc[kq][e] += d;
                 csk[kq] += d;
                 sqk[kq] = __fma_rn(d, d, sqk[kq]);
@@ -622,6 +614,32 @@ __global__ void __launch_bounds__(kThreads, Tile<PR>::kMinBlocks) kb_primal_stag
             vst<float, kBR>(Xa + col + kq * 32 * kBR, av);
           }
         }
+      };
+      // (a 128-row tile has no registers for the second form)
+      const bool whole = PR == 256 && row0 + PR <= I.m && !first && !zero_g;
+      for (long long j = jb + warp; !failed && j < je; j += kWarps) {
+        const int stage = cstage;
+        const uint32_t parity = cphase;
+        if (!mbar_wait_bounded(bar0 + 8 * stage, parity)) {
+          failed = true;
+          if (lane == 0) {
+            atomicExch(&st->kernel_error, 1);
+            atomicExch(&B.act->error, 1);
+          }
+          break;
+        }
+        const unsigned char* stg = ring + (size_t)stage * L::kStageBytes;
+        const float vj = (float)vnext;
+        cost.take();
+        if (j + kWarps < je) {
+          if (!zero_g) vnext = __ldg(v + j + kWarps);
+          cost.prefetch(j + kWarps);
+        }
+        const long long col = j * I.ld + row0 + lane * kBR;
+        if (PR == 256 && whole)
+          unit(std::integral_constant<bool, PR == 256>(), stg, vj, col);
+        else
+          unit(std::false_type(), stg, vj, col);
         const double cs = warp_sum(lane_sum(csk));
         if (lane == 0) B.colpart[base_u + p * I.n + j] = cs;
         __syncwarp();
@@ -764,11 +782,12 @@ __global__ void __launch_bounds__(kVecThreads) kb_dual(BatchBuffers B, SolveConf
 template <int CK, int PR, bool CO>
 __device__ __forceinline__ void kb_eval_body(const BatchBuffers& B, const long long cta, const int grid) {
   constexpr int kBRPL = Tile<PR>::RPL;
+  __shared__ __align__(16) double su[PR], sua[PR];
   const BatchActive act = *B.act;
   if (act.count == 0 || act.error) return;
   const long long q0 = B.cta_begin[cta], q1 = B.cta_begin[cta + 1];
   if (q0 >= q1) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   int kk = find_segment<CO>(B.unit_prefix, act.count, q0);
   long long q = q0;
   while (q < q1) {
@@ -793,68 +812,43 @@ __device__ __forceinline__ void kb_eval_body(const BatchBuffers& B, const long l
     csrc.ys = B.ys ? B.ys + I.tpts_off * B.dim : nullptr;
     csrc.dim = B.dim;
     CostReader<CK, kBR, kBRPL> cost(csrc, (float)st->cost_scale);
-    double accv[kEvalSums];
-#pragma unroll
-    for (int e = 0; e < kEvalSums; ++e) accv[e] = 0.0;
+    EvalSums sum;
     const long long ql0 = q - base_u, ql1 = seg_end - base_u;
     for (long long p = ql0 / I.n; p * I.n < ql1; ++p) {
       const long long jb = (ql0 > p * I.n ? ql0 : p * I.n) - p * I.n;
       const long long je = (ql1 < (p + 1) * I.n ? ql1 : (p + 1) * I.n) - p * I.n;
       const long long row0 = p * PR;
-      double ur[kBRPL][kBR], uar[kBRPL][kBR];
+      __syncthreads();  // the panel before is done with
+      for (int t = threadIdx.x; t < PR; t += kThreads) {
+        su[panel_slot<kBR>(t)] = row0 + t < I.m ? ldro<CO>(u + row0 + t) : 0.0;
+        sua[panel_slot<kBR>(t)] = row0 + t < I.m && have_avg ? ldro<CO>(ua + row0 + t) : 0.0;
+      }
+      __syncthreads();
       bool ok[kBRPL];
+      int nv[kBRPL];
 #pragma unroll
       for (int kq = 0; kq < kBRPL; ++kq) {
         const long long i = row0 + kq * 32 * kBR + lane * kBR;
-        ok[kq] = i < I.m;
-#pragma unroll
-        for (int e = 0; e < kBR; ++e) {
-          const bool in = ok[kq] && i + e < I.m;
-          ur[kq][e] = in ? ldro<CO>(u + i + e) : 0.0;
-          uar[kq][e] = (in && have_avg) ? ldro<CO>(ua + i + e) : 0.0;
-        }
+        nv[kq] = (int)min(max(I.m - i, 0ll), (long long)kBR);
+        ok[kq] = nv[kq] > 0;
       }
       cost.panel(row0, lane, I.m, ok);
-      for (long long j = jb + warp; j < je; j += kWarps) {
-        const double vj = ldro<CO>(v + j);
-        const double vaj = have_avg ? ldro<CO>(va + j) : 0.0;
-        cost.column(j);
-        const long long col = j * I.ld + row0 + lane * kBR;
-#pragma unroll
-        for (int kq = 0; kq < kBRPL; ++kq) {
-          if (!ok[kq]) continue;
-          const long long idx = col + kq * 32 * kBR;
-          const long long i = row0 + kq * 32 * kBR + lane * kBR;
-          typename CostReader<CK, kBR, kBRPL>::value_t cv[kBR];
-          float xv[kBR], av[kBR];
-          cost.get(idx, kq, cv);
-          vldro<CO>(X + idx, xv);
-          if (have_avg) vldro<CO>(Xa + idx, av);
-#pragma unroll
-          for (int e = 0; e < kBR; ++e) {
-            if (i + e >= I.m) continue;
-            const double c = widen(cv[e]), x = widen(xv[e]);
-            const double gg = zero_g ? 0.0 : __dsub_rn(__dsub_rn(c, ur[kq][e]), vj);
-            const double mg = neg_part(gg);
-            accv[E_DOT] += c * x;
-            accv[E_SQX] += x * x;
-            accv[E_MAXX] = nanmax(accv[E_MAXX], fabs(x));
-            accv[E_SQG] += mg * mg;
-            accv[E_MAXG] = nanmax(accv[E_MAXG], mg);
-            if (have_avg) {
-              const double xa = widen(av[e]);
-              const double ga = __dsub_rn(__dsub_rn(c, uar[kq][e]), vaj);
-              const double mga = neg_part(ga);
-              accv[E_AVG + E_DOT] += c * xa;
-              accv[E_AVG + E_SQX] += xa * xa;
-              accv[E_AVG + E_MAXX] = nanmax(accv[E_AVG + E_MAXX], fabs(xa));
-              accv[E_AVG + E_SQG] += mga * mga;
-              accv[E_AVG + E_MAXG] = nanmax(accv[E_AVG + E_MAXG], mga);
-            }
-          }
-        }
-      }
+      auto at = [&](int64_t j) { return j * I.ld + row0 + lane * kBR; };
+      auto load_x = [&](bool avg, int64_t idx, float (&x)[kBR], float (&xa)[kBR]) {
+        vldro<CO>(X + idx, x);
+        if (avg) vldro<CO>(Xa + idx, xa);
+      };
+      auto load_v = [&](bool avg, int64_t j, double& vj, double& vaj) {
+        vj = ldro<CO>(v + j);
+        vaj = avg ? ldro<CO>(va + j) : 0.0;
+      };
+      if (!have_avg || zero_g)
+        eval_columns<false, true, kBR, kBRPL>(cost, nv, su, sua, zero_g, have_avg, jb, je, at, load_x, load_v, sum);
+      else
+        eval_columns<true, true, kBR, kBRPL>(cost, nv, su, sua, zero_g, have_avg, jb, je, at, load_x, load_v, sum);
     }
+    double accv[kEvalSums];
+    sum.store(accv);
     block_reduce<kEvalSums>(accv, kEvalMaxMask, B.evpart + (cta + kk) * kEvalSums);
     q = seg_end;
     ++kk;
@@ -965,15 +959,15 @@ __global__ void __launch_bounds__(kVecThreads) kb_eval_vec(BatchBuffers B, Solve
 // persistent chunk: CTA 0 with its 256).
 template <int PR>
 __device__ __forceinline__ void kb_compact_body(const BatchBuffers& B, const int grid) {
-  __shared__ int flags[1024];
-  __shared__ int base;
-  __shared__ long long total_cost;
+  // prefix sums of the active instances before the one at hand: their number, units,
+  // panels, vector blocks and balancing cost
+  constexpr int kSums = 5;
+  __shared__ long long warp_total[32][kSums];
+  __shared__ long long base[kSums];
   __shared__ int empty_flag;
-  const int T = (int)blockDim.x;
-  if (threadIdx.x == 0) {
-    base = 0;
-    empty_flag = 0;
-  }
+  const int T = (int)blockDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < kSums) base[threadIdx.x] = 0;
+  if (threadIdx.x == 0) empty_flag = 0;
   if (B.race) {
     // racing instances: once a member of a group is optimal, the others stop
     for (int k = threadIdx.x; k < B.num; k += blockDim.x) {
@@ -993,45 +987,72 @@ __device__ __forceinline__ void kb_compact_body(const BatchBuffers& B, const int
     }
   }
   __syncthreads();
-  long long units = 0, panels = 0, vblocks = 0, cost = 0;
   const long long wu = (long long)B.unit_cost * kUnitCostRows;
+  // a block scan per T instances (by one thread in turn: 235 us for 512 instances on B200)
   for (int off = 0; off < B.num; off += T) {
     const int k = off + threadIdx.x;
-    flags[threadIdx.x] = (k < B.num && !B.st[k].done) ? 1 : 0;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int c = base;
-      for (int t = 0; t < T && off + t < B.num; ++t) {
-        if (!flags[t]) continue;
-        const int kk = off + t;
-        const BatchInstance& I = B.inst[kk];
-        B.ids[c] = kk;
-        B.unit_prefix[c] = units;
-        B.panel_prefix[c] = panels;
-        B.vblock_prefix[c] = vblocks;
-        B.cost_prefix[c] = cost;
-        units += I.panels * I.n;
-        panels += I.panels;
-        vblocks += I.rblocks + I.cblocks;
-        cost += I.n * (8 * I.m + wu * I.panels);
-        ++c;
+    const bool active = k < B.num && !B.st[k].done;
+    long long own[kSums] = {0, 0, 0, 0, 0}, x[kSums];
+    if (active) {
+      const BatchInstance& I = B.inst[k];
+      own[0] = 1;
+      own[1] = I.panels * I.n;
+      own[2] = I.panels;
+      own[3] = I.rblocks + I.cblocks;
+      own[4] = I.n * (8 * I.m + wu * I.panels);
+    }
+#pragma unroll
+    for (int e = 0; e < kSums; ++e) {
+      x[e] = own[e];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const long long y = __shfl_up_sync(0xffffffffu, x[e], o);
+        if (lane >= o) x[e] += y;
       }
-      base = c;
-      B.unit_prefix[c] = units;
-      B.panel_prefix[c] = panels;
-      B.vblock_prefix[c] = vblocks;
-      B.cost_prefix[c] = cost;
+      if (lane == 31) warp_total[warp][e] = x[e];
+    }
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+      for (int e = 0; e < kSums; ++e) {
+        const long long t = lane < T / 32 ? warp_total[lane][e] : 0;
+        long long y = t;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const long long z = __shfl_up_sync(0xffffffffu, y, o);
+          if (lane >= o) y += z;
+        }
+        const long long b0 = base[e];
+        __syncwarp();
+        if (lane < T / 32) warp_total[lane][e] = b0 + y - t;  // what comes before the warp
+        if (lane == 31) base[e] = b0 + y;
+      }
+    }
+    __syncthreads();
+    if (active) {
+      long long at[kSums];
+#pragma unroll
+      for (int e = 0; e < kSums; ++e) at[e] = warp_total[warp][e] + x[e] - own[e];
+      const int c = (int)at[0];
+      B.ids[c] = k;
+      B.unit_prefix[c] = at[1];
+      B.panel_prefix[c] = at[2];
+      B.vblock_prefix[c] = at[3];
+      B.cost_prefix[c] = at[4];
     }
     __syncthreads();
   }
+  const int count = (int)base[0];
   if (threadIdx.x == 0) {
-    B.act->count = base;
-    B.act->total_units = units;
-    total_cost = cost;
+    B.unit_prefix[count] = base[1];
+    B.panel_prefix[count] = base[2];
+    B.vblock_prefix[count] = base[3];
+    B.cost_prefix[count] = base[4];
+    B.act->count = count;
+    B.act->total_units = base[1];
   }
   __syncthreads();
-  const int count = base;
-  const long long W = total_cost;
+  const long long W = base[4];
   for (int c = threadIdx.x; c <= grid; c += blockDim.x) {
     long long q;
     if (count == 0 || c == 0) {

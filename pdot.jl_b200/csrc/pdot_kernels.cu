@@ -575,68 +575,108 @@ __device__ __forceinline__ void k3_eval_body(const Buffers& B, const Geometry& g
   double acc[kEvalSums];
 #pragma unroll
   for (int k = 0; k < kEvalSums; ++k) acc[k] = 0.0;
-  for (int64_t p = q0 / n; p * n < q1; ++p) {
-    const int64_t jb = (q0 > p * n ? q0 : p * n) - p * n;
-    const int64_t je = (q1 < (p + 1) * n ? q1 : (p + 1) * n) - p * n;
-    const int64_t row0 = p * kPanelRows;
-    double ur[RPL][R], uar[RPL][R];
-    bool ok[RPL];
-#pragma unroll
-    for (int k = 0; k < RPL; ++k) {
-      const int64_t i = row0 + k * 32 * R + lane * R;
-      ok[k] = i < m;
-#pragma unroll
-      for (int e = 0; e < R; ++e) {
-        ur[k][e] = ok[k] ? __ldcg(u + i + e) : 0.0;
-        uar[k][e] = (ok[k] && have_avg) ? __ldcg(ua + i + e) : 0.0;
+  if constexpr (sizeof(TX) == 4) {
+    __shared__ __align__(16) double su[kPanelRows], sua[kPanelRows];
+    EvalSums sum;
+    for (int64_t p = q0 / n; p * n < q1; ++p) {
+      const int64_t jb = (q0 > p * n ? q0 : p * n) - p * n;
+      const int64_t je = (q1 < (p + 1) * n ? q1 : (p + 1) * n) - p * n;
+      const int64_t row0 = p * kPanelRows;
+      __syncthreads();  // the panel before is done with
+      for (int t = threadIdx.x; t < kPanelRows; t += kThreads) {
+        su[panel_slot<R>(t)] = row0 + t < m ? __ldcg(u + row0 + t) : 0.0;
+        sua[panel_slot<R>(t)] = row0 + t < m && have_avg ? __ldcg(ua + row0 + t) : 0.0;
       }
-    }
-    cost.panel(row0, lane, m, ok);
-    for (int64_t j = jb + warp; j < je; j += kWarps) {
-      const double vj = __ldcg(v + j);
-      const double vaj = have_avg ? __ldcg(va + j) : 0.0;
-      cost.column(j);
-      const int64_t base = j * m + row0 + lane * R;
-      typename CostReader<CK, R, RPL>::value_t cv[RPL][R];
-      TX xv[RPL][R], av[RPL][R];
+      __syncthreads();
+      bool ok[RPL];
+      int nv[RPL];
 #pragma unroll
       for (int k = 0; k < RPL; ++k) {
-        if (ok[k]) {
-          const int64_t idx = base + k * 32 * R;
-          cost.get(idx, k, cv[k]);
-          if (need_x) {
-            vldcg<TX, R>(X + idx, xv[k]);
-            if (have_avg) vldcg<TX, R>(Xa + idx, av[k]);
-          }
+        ok[k] = row0 + k * 32 * R + lane * R < m;
+        nv[k] = ok[k] ? R : 0;
+      }
+      cost.panel(row0, lane, m, ok);
+      auto at = [&](int64_t j) { return j * m + row0 + lane * R; };
+      auto load_x = [&](bool avg, int64_t idx, TX (&x)[R], TX (&xa)[R]) {
+        vldcg<TX, R>(X + idx, x);
+        if (avg) vldcg<TX, R>(Xa + idx, xa);
+      };
+      auto load_v = [&](bool avg, int64_t j, double& vj, double& vaj) {
+        vj = __ldcg(v + j);
+        vaj = avg ? __ldcg(va + j) : 0.0;
+      };
+      if (!have_avg || zero_g)
+        eval_columns<false, true, R, RPL>(cost, nv, su, sua, zero_g, have_avg, jb, je, at, load_x, load_v, sum);
+      else if (need_x)
+        eval_columns<true, true, R, RPL>(cost, nv, su, sua, zero_g, have_avg, jb, je, at, load_x, load_v, sum);
+      else
+        eval_columns<true, false, R, RPL>(cost, nv, su, sua, zero_g, have_avg, jb, je, at, load_x, load_v, sum);
+    }
+    sum.store(acc);
+  } else {
+    for (int64_t p = q0 / n; p * n < q1; ++p) {
+      const int64_t jb = (q0 > p * n ? q0 : p * n) - p * n;
+      const int64_t je = (q1 < (p + 1) * n ? q1 : (p + 1) * n) - p * n;
+      const int64_t row0 = p * kPanelRows;
+      double ur[RPL][R], uar[RPL][R];
+      bool ok[RPL];
+#pragma unroll
+      for (int k = 0; k < RPL; ++k) {
+        const int64_t i = row0 + k * 32 * R + lane * R;
+        ok[k] = i < m;
+#pragma unroll
+        for (int e = 0; e < R; ++e) {
+          ur[k][e] = ok[k] ? __ldcg(u + i + e) : 0.0;
+          uar[k][e] = (ok[k] && have_avg) ? __ldcg(ua + i + e) : 0.0;
         }
       }
+      cost.panel(row0, lane, m, ok);
+      for (int64_t j = jb + warp; j < je; j += kWarps) {
+        const double vj = __ldcg(v + j);
+        const double vaj = have_avg ? __ldcg(va + j) : 0.0;
+        cost.column(j);
+        const int64_t base = j * m + row0 + lane * R;
+        typename CostReader<CK, R, RPL>::value_t cv[RPL][R];
+        TX xv[RPL][R], av[RPL][R];
 #pragma unroll
-      for (int k = 0; k < RPL; ++k) {
-        if (ok[k]) {
-#pragma unroll
-          for (int e = 0; e < R; ++e) {
-            const double c = widen(cv[k][e]);
-            const double gg = zero_g ? 0.0 : __dsub_rn(__dsub_rn(c, ur[k][e]), vj);
-            const double mg = neg_part(gg);
+        for (int k = 0; k < RPL; ++k) {
+          if (ok[k]) {
+            const int64_t idx = base + k * 32 * R;
+            cost.get(idx, k, cv[k]);
             if (need_x) {
-              const double x = widen(xv[k][e]);
-              acc[E_DOT] += c * x;
-              acc[E_SQX] += x * x;
-              acc[E_MAXX] = nanmax(acc[E_MAXX], fabs(x));
+              vldcg<TX, R>(X + idx, xv[k]);
+              if (have_avg) vldcg<TX, R>(Xa + idx, av[k]);
             }
-            acc[E_SQG] += mg * mg;
-            acc[E_MAXG] = nanmax(acc[E_MAXG], mg);
-            if (have_avg) {
-              const double ga = __dsub_rn(__dsub_rn(c, uar[k][e]), vaj);
-              const double mga = neg_part(ga);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < RPL; ++k) {
+          if (ok[k]) {
+#pragma unroll
+            for (int e = 0; e < R; ++e) {
+              const double c = widen(cv[k][e]);
+              const double gg = zero_g ? 0.0 : __dsub_rn(__dsub_rn(c, ur[k][e]), vj);
+              const double mg = neg_part(gg);
               if (need_x) {
-                const double xa = widen(av[k][e]);
-                acc[E_AVG + E_DOT] += c * xa;
-                acc[E_AVG + E_SQX] += xa * xa;
-                acc[E_AVG + E_MAXX] = nanmax(acc[E_AVG + E_MAXX], fabs(xa));
+                const double x = widen(xv[k][e]);
+                acc[E_DOT] += c * x;
+                acc[E_SQX] += x * x;
+                acc[E_MAXX] = nanmax(acc[E_MAXX], fabs(x));
               }
-              acc[E_AVG + E_SQG] += mga * mga;
-              acc[E_AVG + E_MAXG] = nanmax(acc[E_AVG + E_MAXG], mga);
+              acc[E_SQG] += mg * mg;
+              acc[E_MAXG] = nanmax(acc[E_MAXG], mg);
+              if (have_avg) {
+                const double ga = __dsub_rn(__dsub_rn(c, uar[k][e]), vaj);
+                const double mga = neg_part(ga);
+                if (need_x) {
+                  const double xa = widen(av[k][e]);
+                  acc[E_AVG + E_DOT] += c * xa;
+                  acc[E_AVG + E_SQX] += xa * xa;
+                  acc[E_AVG + E_MAXX] = nanmax(acc[E_AVG + E_MAXX], fabs(xa));
+                }
+                acc[E_AVG + E_SQG] += mga * mga;
+                acc[E_AVG + E_MAXG] = nanmax(acc[E_AVG + E_MAXG], mga);
+              }
             }
           }
         }
