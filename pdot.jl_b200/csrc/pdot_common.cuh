@@ -192,6 +192,14 @@ struct Buffers {
 Geometry make_geometry(int64_t m, int64_t n, int vec_ok, int device, int plan_f32 = 0,
                        int cost_kind = PDOT_COST_F64, int staged_ok = 0);
 size_t workspace_doubles(const Geometry& g);
+// The geometry of the stand-alone primal pass: up to kPassGrid times the resident CTAs,
+// each with kPassUnits units and more. CTAs that follow the first ones start at
+// different times, which evens the load on the memory: 20000 x 15000 takes 1900 us on
+// B200 (1979 with one CTA range per resident CTA, 1967 with two, 1913 with four); at
+// 4000 x 3000, 162 units a resident CTA, six ranges took 104 us against 95. (A solve keeps
+// one: its ranges fix the order of its row sums.)
+constexpr int kPassGrid = 6, kPassUnits = 160;
+Geometry pass_geometry(int64_t m, int64_t n, int vec_ok, int device);
 // Scratch of the stand-alone primal pass (launch_primal_pass): its row
 // partials, column partials and per-CTA sums of squares, in that order.
 inline size_t pass_scratch_doubles(const Geometry& g) {

@@ -1112,8 +1112,8 @@ int64_t pdot_primal_pass_workspace_bytes(int64_t m, int64_t n) {
     return 0;
   }
   // the grid depends on the load width the buffers allow: cover both
-  const int64_t a = pass_workspace_bytes(pdot::make_geometry(m, n, 1, device));
-  const int64_t b = pass_workspace_bytes(pdot::make_geometry(m, n, 0, device));
+  const int64_t a = pass_workspace_bytes(pdot::pass_geometry(m, n, 1, device));
+  const int64_t b = pass_workspace_bytes(pdot::pass_geometry(m, n, 0, device));
   return a > b ? a : b;
 }
 
@@ -1131,7 +1131,7 @@ int pdot_primal_pass_f64(int64_t m, int64_t n, const double* cost, double* prima
     int device = 0;
     CK(cudaGetDevice(&device));
     const int vec_ok = aligned16(cost) && aligned16(primal) && aligned16(primal_avg);
-    const pdot::Geometry g = pdot::make_geometry(m, n, vec_ok, device);
+    const pdot::Geometry g = pdot::pass_geometry(m, n, vec_ok, device);
     const int64_t need = pass_workspace_bytes(g);
     if (workspace_bytes < need)
       fail(PDOT_ERR_INVALID_ARGUMENT, "workspace of %lld bytes, %lld needed", (long long)workspace_bytes,

@@ -1152,6 +1152,16 @@ Geometry make_geometry(int64_t m, int64_t n, int vec_ok, int device, int plan_f3
   return g;
 }
 
+Geometry pass_geometry(int64_t m, int64_t n, int vec_ok, int device) {
+  Geometry g = make_geometry(m, n, vec_ok, device);
+  const int64_t times = g.units / ((int64_t)g.grid * kPassUnits);
+  Geometry wide = g;
+  wide.grid *= (int32_t)(times < 1 ? 1 : times > kPassGrid ? kPassGrid : times);
+  // what the fixed scratch of the no-alloc entry holds stays so, and both entries agree
+  const size_t fixed = PDOT_NOALLOC_SCRATCH_BYTES / sizeof(double);
+  return pass_scratch_doubles(g) <= fixed && pass_scratch_doubles(wide) > fixed ? g : wide;
+}
+
 size_t workspace_doubles(const Geometry& g) {
   const size_t vb = (size_t)g.row_blocks + g.col_blocks;
   const size_t db = (size_t)g.dual_row_blocks + g.col_blocks;

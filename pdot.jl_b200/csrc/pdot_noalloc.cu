@@ -74,7 +74,7 @@ extern "C" int pdot_primal_pass_f64_noalloc(int64_t m, int64_t n, const double* 
   cudaError_t e = cudaGetDevice(&device);
   if (e != cudaSuccess) return report(PDOT_ERR_CUDA, "cudaGetDevice failed: %s", cudaGetErrorString(e));
   const int vec_ok = aligned16(cost) && aligned16(primal) && aligned16(primal_avg);
-  const pdot::Geometry g = pdot::make_geometry(m, n, vec_ok, device);
+  const pdot::Geometry g = pdot::pass_geometry(m, n, vec_ok, device);
   const size_t need = pdot::pass_scratch_doubles(g);
   if (need > kScratchDoubles)
     return report(PDOT_ERR_TOO_LARGE,

@@ -199,3 +199,31 @@ def test_network_step_at_odd_shapes(cuda, dims, batch):
     sizes = [H * I, H, H * H, H, O * H, O]
     for name, lo, k in zip(["W1", "b1", "W2", "b2", "W3", "b3"], np.cumsum([0] + sizes), sizes):
         assert np.linalg.norm(g[lo : lo + k] - want_g[lo : lo + k]) <= 1e-2 * np.linalg.norm(want_g[lo : lo + k]), name
+
+
+@pytest.mark.parametrize("m,n", [(256, 47359), (256, 47360), (256, 94720), (257, 47360), (255, 94721), (2048, 36000)])
+def test_primal_pass_where_its_grid_grows(cuda, m, n):
+    """The stand-alone pass around the sizes at which its grid becomes a multiple of the resident CTAs (160
+    units a CTA range, two ranges per SM): entries bit for bit, sums to 1e-12 of their terms' magnitude."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    rand = lambda *s: torch.rand(*s, generator=g, device="cuda", dtype=torch.float64)  # noqa: E731
+    C, X, Xa, u, v = rand(n, m), rand(n, m), rand(n, m), rand(m), rand(n)
+    dr, dc, dq = torch.empty(m, dtype=torch.float64, device=cuda), torch.empty(n, dtype=torch.float64, device=cuda), torch.empty(1, dtype=torch.float64, device=cuda)
+    s, nw, aw = 0.3, 0.25, 0.8
+    D = (X - s * ((C - u[None, :]) - v[:, None])).clamp(min=0.0) - X
+    want_x = X + D
+    want_a = (Xa + want_x * nw) * aw
+    lib = _abi.load()
+    need = lib.pdot_primal_pass_workspace_bytes(m, n)
+    work = torch.empty(need, dtype=torch.uint8, device=cuda)
+    torch.cuda.synchronize()
+    _abi.check(lib, lib.pdot_primal_pass_f64(m, n, C.data_ptr(), X.data_ptr(), Xa.data_ptr(), u.data_ptr(), v.data_ptr(), s, nw,
+                                             aw, 0, dr.data_ptr(), dc.data_ptr(), dq.data_ptr(), work.data_ptr(), need, None),
+               "pdot_primal_pass_f64")
+    torch.cuda.synchronize()
+    assert torch.equal(X, want_x) and torch.equal(Xa, want_a)
+    assert (dr - D.sum(0)).abs().max() <= 1e-12 * D.abs().sum(0).max()
+    assert (dc - D.sum(1)).abs().max() <= 1e-12 * D.abs().sum(1).max()
+    assert abs(float(dq - D.square().sum())) <= 1e-12 * float(D.square().sum())
