@@ -10,6 +10,7 @@
 #include <cstdint>
 
 #include "pdot_common.cuh"
+#include "pdot_pairs.cuh"
 
 namespace pdot {
 namespace {
@@ -217,9 +218,9 @@ __global__ void __launch_bounds__(kAuxThreads)
 // C_ij = ||x_i - y_j||^2 in FP64, divided by its maximum when `normalise`. The
 // maximum is taken from the points, nothing stored, and the cost is then written
 // once (8 B per entry); stored first, scanned and divided in place it took 32 B per
-// entry: 0.93 ms at 10000 x 10000 in three dimensions on B200, now 0.25: 88 us for the
-// maximum, 165 for the write, both bound by FP64 issue (10 and 14 operations an entry;
-// the bytes alone would take 122).
+// entry: 0.93 ms at 10000 x 10000 in three dimensions on B200, now 0.20: 39 us for the
+// maximum, 159 for the write, which is bound by FP64 issue (14 operations an entry; the
+// bytes alone would take 122).
 //
 // DIM 1..4 are compiled in, 0 is any dimension (coordinates from global memory).
 constexpr int kCostRows = 2;  // rows per thread of the write
@@ -269,11 +270,133 @@ struct DivideBy {
 
 // The largest entry (NaNs ignored), at least 0, by an atomicMax on its bits
 // (non-negative doubles order as their bits do).
+//
+// DIM 1..4, large problems: a tile of columns is first passed over in FP32, with the
+// coordinates taken relative to the first point. An FP32 distance is within
+// E = 32 * 2^-24 * D A^2 of the FP64 one, A = |x|_max + |y|_max of those coordinates:
+// narrowing moves a difference by 2^-24 A and its rounding by as much, a square then
+// errs by 5 * 2^-24 A^2, and sum and test add less than that once more. Threads whose
+// largest value cannot reach the CTA's largest lower bound, or the result so far, are
+// done with the tile; the others take the FP64 distances of the columns, by fours, that
+// can. Where E is not finite no pair is left out. 88 us in FP64 throughout at
+// 10000 x 10000 in three dimensions, 39 this way; its FP32 operations alone take 17.
+constexpr int kMaxTile = 128;  // columns of a tile
+constexpr int kMaxRows = 2;    // rows per thread: a column's coordinates serve both
+template <int D>
+__global__ void __launch_bounds__(kAuxThreads)
+    k_sqeuclid_max(int64_t m, int64_t n, int64_t share, const double* __restrict__ xs, const double* __restrict__ ys,
+                   unsigned long long* __restrict__ out) {
+  __shared__ double ty[kMaxTile * D];
+  __shared__ __align__(16) float fy[D][kMaxTile];
+  __shared__ double red[kAuxWarps];
+  __shared__ float sbest;  // a lower bound of the result
+  __shared__ int bound;    // bits of the tile's |y|_max
+  double origin[D], x[kMaxRows][D];
+  unsigned long long minus[kMaxRows][D];
+  float reach[kMaxRows];
+  bool ok[kMaxRows];
+#pragma unroll
+  for (int d = 0; d < D; ++d) origin[d] = fabs(xs[d]) < INFINITY ? xs[d] : 0.0;
+#pragma unroll
+  for (int q = 0; q < kMaxRows; ++q) {
+    const int64_t i = ((int64_t)blockIdx.x * kMaxRows + q) * kAuxThreads + threadIdx.x;
+    ok[q] = i < m;
+    reach[q] = 0.0f;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      x[q][d] = ok[q] ? xs[i * D + d] : origin[d];
+      const float f = (float)(x[q][d] - origin[d]);
+      reach[q] = fmaxf(reach[q], fabsf(f));
+      minus[q][d] = pack2(-f, -f);
+    }
+  }
+  if (threadIdx.x == 0)
+    sbest = __double2float_rd(__longlong_as_double((long long)*reinterpret_cast<volatile unsigned long long*>(out)));
+  double best = 0.0;
+  const int64_t jb = (int64_t)blockIdx.y * share, je = (jb + share < n) ? jb + share : n;
+  for (int64_t j0 = jb; j0 < je; j0 += kMaxTile) {
+    const int cnt = (int)((je - j0) < kMaxTile ? (je - j0) : kMaxTile);
+    __syncthreads();
+    if (threadIdx.x == 0) bound = 0;
+    __syncthreads();
+    float my = 0.0f;
+    // the FP32 entries past the last column repeat it
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      const int t = threadIdx.x, c = t < cnt ? t : cnt - 1;
+      if (t >= kMaxTile) break;
+      const double y = ys[(j0 + c) * D + d];
+      const float f = (float)(y - origin[d]);
+      ty[t * D + d] = y;
+      fy[d][t] = f;
+      my = fmaxf(my, fabsf(f));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) my = fmaxf(my, __shfl_xor_sync(0xffffffffu, my, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(&bound, __float_as_int(my));
+    __syncthreads();
+    float top[kMaxRows], err[kMaxRows];
+#pragma unroll
+    for (int q = 0; q < kMaxRows; ++q) {
+      const float A = reach[q] + __int_as_float(bound);
+      err[q] = 32.0f * kUnit * (float)D * A * A + 1e-30f;
+      top[q] = -1.0f;
+    }
+#pragma unroll 2
+    for (int t = 0; t < cnt; t += 4) {
+      ulonglong2 c[D];
+#pragma unroll
+      for (int d = 0; d < D; ++d) c[d] = *reinterpret_cast<const ulonglong2*>(&fy[d][t]);
+#pragma unroll
+      for (int q = 0; q < kMaxRows; ++q) top[q] = max_sqdist4<D>(minus[q], c, top[q]);
+    }
+    // the bits of non-negative floats order as the floats do
+    float lower = 0.0f;
+#pragma unroll
+    for (int q = 0; q < kMaxRows; ++q)
+      if (ok[q] && err[q] < INFINITY && top[q] < INFINITY) lower = fmaxf(lower, top[q] - err[q]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) lower = fmaxf(lower, __shfl_xor_sync(0xffffffffu, lower, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int*>(&sbest), __float_as_int(lower));
+    __syncthreads();
+    const float lim = sbest;
+#pragma unroll
+    for (int q = 0; q < kMaxRows; ++q) {
+      // with a finite bound a tile of NaNs alone leaves top at -1 and has nothing to offer
+      const bool finite = err[q] < INFINITY;
+      if (!ok[q] || (finite && (top[q] < 0.0f || top[q] + err[q] < lim))) continue;
+      for (int t = 0; t < cnt; t += 4) {
+        ulonglong2 c[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) c[d] = *reinterpret_cast<const ulonglong2*>(&fy[d][t]);
+        if (finite && max_sqdist4<D>(minus[q], c, -1.0f) + err[q] < lim) continue;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (t + k < cnt) best = fmax(best, sq_distance<D>(x[q], ty + (t + k) * D, D));
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) best = fmax(best, __shfl_xor_sync(0xffffffffu, best, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < kAuxWarps; ++w) best = fmax(best, red[w]);
+    atomicMax(out, (unsigned long long)__double_as_longlong(best));
+  }
+}
+
+// The same in FP64 throughout: any dimension, and small problems, where the tiles' barriers
+// and second passes cost more than the arithmetic (500 x 500 in one dimension, whole cost:
+// 14.3 us against 17; 3000 x 2500 in two: 30.6 either way).
+constexpr int kSmallRows = 4;  // rows per thread: a column's coordinates serve four distances
+constexpr int64_t kSmallPairs = int64_t(1) << 22;
 template <int DIM>
 __global__ void __launch_bounds__(kAuxThreads)
-    k_sqeuclid_max(int64_t m, int64_t n, int dim, int64_t chunk, const double* __restrict__ xs,
+    k_sqeuclid_max_small(int64_t m, int64_t n, int dim, int64_t chunk, const double* __restrict__ xs,
                    const double* __restrict__ ys, unsigned long long* __restrict__ out) {
-  constexpr int Q = 4;  // rows per thread: a column's coordinates serve four distances
+  constexpr int Q = kSmallRows;
   constexpr int D = DIM > 0 ? DIM : 1;
   const int64_t i0 = (int64_t)blockIdx.x * kAuxThreads * Q + threadIdx.x;
   double x[Q][D], mx[Q];
@@ -466,10 +589,19 @@ cudaError_t sqeuclid_passes(int64_t m, int64_t n, int dim, const double* xs, con
     top = C;
     cudaError_t e = cudaMemsetAsync(top, 0, sizeof(double), s);
     if (e != cudaSuccess) return e;
-    const int64_t strips = (m + kAuxThreads * 4 - 1) / (kAuxThreads * 4);
-    const int64_t chunk = column_chunk(n, strips, 148 * 16, 16);
-    k_sqeuclid_max<DIM><<<dim3((unsigned)strips, (unsigned)((n + chunk - 1) / chunk)), kAuxThreads, 0, s>>>(
-        m, n, dim, chunk, xs, ys, reinterpret_cast<unsigned long long*>(top));
+    auto* bits = reinterpret_cast<unsigned long long*>(top);
+    if (DIM == 0 || m * n <= kSmallPairs) {
+      const int64_t strips = (m + kAuxThreads * kSmallRows - 1) / (kAuxThreads * kSmallRows);
+      const int64_t chunk = column_chunk(n, strips, 148 * 16, 16);
+      k_sqeuclid_max_small<DIM>
+          <<<dim3((unsigned)strips, (unsigned)((n + chunk - 1) / chunk)), kAuxThreads, 0, s>>>(m, n, dim, chunk, xs, ys, bits);
+    } else if constexpr (DIM > 0) {
+      const int64_t strips = (m + kAuxThreads * kMaxRows - 1) / (kAuxThreads * kMaxRows);
+      // some 16 CTAs per SM, none with less than a tile
+      const int64_t share = column_chunk(n, strips, 148 * 16, kMaxTile);
+      k_sqeuclid_max<DIM><<<dim3((unsigned)strips, (unsigned)((n + share - 1) / share)), kAuxThreads, 0, s>>>(
+          m, n, share, xs, ys, bits);
+    }
   }
   const bool wide = m % kCostRows == 0 && (reinterpret_cast<uintptr_t>(C) & 15u) == 0;
   const int R = wide ? kCostRows : 1;

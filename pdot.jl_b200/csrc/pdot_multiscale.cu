@@ -11,24 +11,35 @@
 // are taken. The results are those of FP64 throughout, bit for bit (a maximum and a
 // minimum do not depend on the pairs that are left out). FP64 arithmetic was what
 // bounded them: B200 does two FP32 operations for one in FP64, and none of the FP32
-// ones needs the conversions.
+// ones needs the conversions. The FP32 pass is bound by issue, so it does two pairs in
+// an instruction and one comparison for two distances; the c-transform keeps the
+// minima of groups of eight centres, and which groups hold the smallest ones, in place
+// of every centre's. 20000 x 15000 points in the plane: the maximum 80 us a pair at a
+// time, 60 this way (the FP32 operations alone take 33); 20000 points against 6000
+// centres: 96 and 53 (17).
 //
 // The second set is split over CTAs too, so that 20000 points, 79 CTAs of 256, fill
-// the 148 SMs: the maximum by atomicMax, the minimum by a cluster's shared memory.
+// the 148 SMs: the maximum by atomicMax, the minimum by a cluster's shared memory. Tiles
+// of 128 points for the maximum, which took 74 us with 512, and of 256 centres, which
+// took 58 with 128.
 #include <cooperative_groups.h>
 
 #include <cfloat>
 #include <cmath>
 
 #include "pdot_common.cuh"
+#include "pdot_pairs.cuh"
 
 namespace pdot {
 namespace {
 
-constexpr int kTile = 256;      // points of the second set per shared-memory tile (= threads per CTA)
+constexpr int kFarTile = 128;   // points of the second set per shared-memory tile of the maximum
+constexpr int kTile = 256;      // and of the c-transform
+constexpr int kMaxThreads = 256;  // threads of a CTA of the maximum
+constexpr int kMinThreads = 128;  // and of the c-transform
+constexpr int kGroup = 8;       // centres whose minimum the c-transform takes as one
 constexpr int kPointsPer = 2;   // points of the first set per thread: a tile entry read once serves both
 constexpr int kSplit = 8;       // CTAs of a cluster, each with a share of the centres
-constexpr float kUnit = 5.9604645e-8f;  // 2^-24, the relative error of one FP32 rounding
 
 // Threads keep max_j ||x_i - y_j||^2 of their points (FP64 from FP32 coordinates) over a
 // share of the y_j; a CTA reduces its threads and one atomicMax on the bit pattern
@@ -41,45 +52,48 @@ constexpr float kUnit = 5.9604645e-8f;  // 2^-24, the relative error of one FP32
 // the tile; the others take its FP64 distances. Which threads those are can differ
 // from run to run, the maximum cannot.
 template <int D>
-__global__ void __launch_bounds__(kTile) k_max_sqdist(int64_t m, int64_t n, int64_t share, const float* __restrict__ xs,
+__global__ void __launch_bounds__(kMaxThreads) k_max_sqdist(int64_t m, int64_t n, int64_t share, const float* __restrict__ xs,
                                                       const float* __restrict__ ys,
                                                       unsigned long long* __restrict__ out_bits) {
-  __shared__ float ty[kTile * D];
-  __shared__ double red[kTile / 32];
+  __shared__ __align__(16) float ty[D][kFarTile];
+  __shared__ double red[kMaxThreads / 32];
   __shared__ float sbest;  // a lower bound of the result
   float xi[kPointsPer][D];
+  unsigned long long minus[kPointsPer][D];
   bool ok[kPointsPer];
 #pragma unroll
   for (int q = 0; q < kPointsPer; ++q) {
-    const int64_t i = ((int64_t)blockIdx.x * kPointsPer + q) * kTile + threadIdx.x;
+    const int64_t i = ((int64_t)blockIdx.x * kPointsPer + q) * kMaxThreads + threadIdx.x;
     ok[q] = i < m;
 #pragma unroll
-    for (int d = 0; d < D; ++d) xi[q][d] = ok[q] ? xs[i * D + d] : 0.0f;
+    for (int d = 0; d < D; ++d) {
+      xi[q][d] = ok[q] ? xs[i * D + d] : 0.0f;
+      minus[q][d] = pack2(-xi[q][d], -xi[q][d]);
+    }
   }
   double best = 0.0;
   if (threadIdx.x == 0)
     sbest = __double2float_rd(__longlong_as_double((long long)*reinterpret_cast<volatile unsigned long long*>(out_bits)));
   const int64_t jb = (int64_t)blockIdx.y * share, je = (jb + share < n) ? jb + share : n;
-  for (int64_t j0 = jb; j0 < je; j0 += kTile) {
-    const int cnt = (int)((je - j0) < kTile ? (je - j0) : kTile);
+  for (int64_t j0 = jb; j0 < je; j0 += kFarTile) {
+    const int cnt = (int)((je - j0) < kFarTile ? (je - j0) : kFarTile);
     __syncthreads();
-    for (int t = threadIdx.x; t < cnt * D; t += kTile) ty[t] = ys[j0 * D + t];
+    // the entries past the last point repeat it
+    for (int t = threadIdx.x; t < kFarTile * D; t += kMaxThreads) {
+      const int j = t / D < cnt ? t / D : cnt - 1;
+      ty[t % D][t / D] = ys[(j0 + j) * D + t % D];
+    }
     __syncthreads();
     float top[kPointsPer];
 #pragma unroll
     for (int q = 0; q < kPointsPer; ++q) top[q] = -1.0f;
-#pragma unroll 4
-    for (int t = 0; t < cnt; ++t) {
+#pragma unroll 2
+    for (int t = 0; t < cnt; t += 4) {
+      ulonglong2 c[D];
 #pragma unroll
-      for (int q = 0; q < kPointsPer; ++q) {
-        float s = 0.0f;
+      for (int d = 0; d < D; ++d) c[d] = *reinterpret_cast<const ulonglong2*>(&ty[d][t]);
 #pragma unroll
-        for (int d = 0; d < D; ++d) {
-          const float e = xi[q][d] - ty[t * D + d];
-          s = d == 0 ? e * e : __fmaf_rn(e, e, s);
-        }
-        top[q] = fmaxf(top[q], s);
-      }
+      for (int q = 0; q < kPointsPer; ++q) top[q] = max_sqdist4<D>(minus[q], c, top[q]);
     }
     // the bits of non-negative floats order as the floats do
     float lower = 0.0f;
@@ -94,12 +108,18 @@ __global__ void __launch_bounds__(kTile) k_max_sqdist(int64_t m, int64_t n, int6
 #pragma unroll
     for (int q = 0; q < kPointsPer; ++q) {
       // a tile of NaNs leaves top at -1 and has nothing to offer
-      if (ok[q] && top[q] >= 0.0f && !(top[q] * 1.000002f + 1e-30f < lim)) {
-        for (int t = 0; t < cnt; ++t) {
+      if (!ok[q] || top[q] < 0.0f || top[q] * 1.000002f + 1e-30f < lim) continue;
+      for (int t = 0; t < cnt; t += 4) {
+        ulonglong2 c[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) c[d] = *reinterpret_cast<const ulonglong2*>(&ty[d][t]);
+        if (max_sqdist4<D>(minus[q], c, -1.0f) * 1.000002f + 1e-30f < lim) continue;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
           double s = 0.0;
 #pragma unroll
           for (int d = 0; d < D; ++d) {
-            const double e = (double)xi[q][d] - (double)ty[t * D + d];
+            const double e = (double)xi[q][d] - (double)ty[d][t + k];
             s += e * e;
           }
           best = s > best ? s : best;
@@ -116,7 +136,7 @@ __global__ void __launch_bounds__(kTile) k_max_sqdist(int64_t m, int64_t n, int6
   __syncthreads();
   if (threadIdx.x == 0) {
     double b = red[0];
-    for (int w = 1; w < kTile / 32; ++w) b = red[w] > b ? red[w] : b;
+    for (int w = 1; w < kMaxThreads / 32; ++w) b = red[w] > b ? red[w] : b;
     atomicMax(out_bits, (unsigned long long)__double_as_longlong(b));
   }
 }
@@ -131,24 +151,26 @@ __global__ void __launch_bounds__(kTile) k_max_sqdist(int64_t m, int64_t n, int6
 // of the FP64 one over a tile (each coordinate difference is at most A and errs by at
 // most 2 * 2^-24 A, a square by 5 * 2^-24 A^2, their sum, the product and the
 // difference by a rounding each; 16 covers D <= 3). A pair whose FP32 value exceeds
-// min(best so far, tile's FP32 minimum + E) + E cannot be the minimum. Where a bound
-// is not finite no pair is left out.
+// min(best so far, tile's FP32 minimum + E) + E cannot be the minimum: only the groups
+// whose minima are within that are taken up again, at most two, or the whole tile where
+// a third one is. Where a bound is not finite no pair is left out.
 template <int D>
-__global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kTile)
+__global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kMinThreads)
     k_c_transform(int64_t np, int64_t nc, const float* __restrict__ pts, const double* __restrict__ centres,
                   const double* __restrict__ duals, double scale, double* __restrict__ out) {
   __shared__ double tc[kTile * D];
   __shared__ double tv[kTile];
-  __shared__ float fc[kTile * D];
-  __shared__ float fv[kTile];
+  __shared__ __align__(16) float fc[D][kTile];
+  __shared__ __align__(16) float fv[kTile];  // minus the duals
   __shared__ int bound_c, bound_v;  // bits of the tile's |c|_max and |dual|_max
-  __shared__ double part[kTile * kPointsPer];
+  __shared__ double part[kMinThreads * kPointsPer];
   float p[kPointsPer][D], reach[kPointsPer];
+  unsigned long long minus[kPointsPer][D];
   double best[kPointsPer];
   bool ok[kPointsPer];
 #pragma unroll
   for (int q = 0; q < kPointsPer; ++q) {
-    const int64_t i = ((int64_t)blockIdx.x * kPointsPer + q) * kTile + threadIdx.x;
+    const int64_t i = ((int64_t)blockIdx.x * kPointsPer + q) * kMinThreads + threadIdx.x;
     ok[q] = i < np;
     best[q] = INFINITY;
     reach[q] = 0.0f;
@@ -156,9 +178,11 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kTile)
     for (int d = 0; d < D; ++d) {
       p[q][d] = ok[q] ? pts[i * D + d] : 0.0f;
       reach[q] = fmaxf(reach[q], fabsf(p[q][d]));
+      minus[q][d] = pack2(-p[q][d], -p[q][d]);
     }
   }
   const float sc = (float)scale;
+  const unsigned long long sc2 = pack2(sc, sc);
   const int64_t share = (nc + kSplit - 1) / kSplit;
   const int64_t jb = (int64_t)blockIdx.y * share, je = (jb + share < nc) ? jb + share : nc;
   for (int64_t j0 = jb; j0 < je; j0 += kTile) {
@@ -168,19 +192,27 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kTile)
     __syncthreads();
     float mc = 0.0f, mv = 0.0f;
     bool odd = false;  // a value that FP32 cannot hold or that is not a number
-    for (int t = threadIdx.x; t < cnt * D; t += kTile) {
+    for (int t = threadIdx.x; t < cnt * D; t += kMinThreads) {
       const double c = centres[j0 * D + t];
+      const float f = (float)c;
       tc[t] = c;
-      fc[t] = (float)c;
-      mc = fmaxf(mc, fabsf(fc[t]));
-      odd |= !(fabsf(fc[t]) < INFINITY);
+      fc[t % D][t / D] = f;
+      mc = fmaxf(mc, fabsf(f));
+      odd |= !(fabsf(f) < INFINITY);
     }
-    for (int t = threadIdx.x; t < cnt; t += kTile) {
+    for (int t = threadIdx.x; t < cnt; t += kMinThreads) {
       const double v = duals[j0 + t];
+      const float f = (float)v;
       tv[t] = v;
-      fv[t] = (float)v;
-      mv = fmaxf(mv, fabsf(fv[t]));
-      odd |= !(fabsf(fv[t]) < INFINITY);
+      fv[t] = -f;
+      mv = fmaxf(mv, fabsf(f));
+      odd |= !(fabsf(f) < INFINITY);
+    }
+    // a last group is filled up with centres that are never the smallest
+    if (const int t = cnt + (int)threadIdx.x; t < ((cnt + kGroup - 1) / kGroup) * kGroup) {
+      fv[t] = INFINITY;
+#pragma unroll
+      for (int d = 0; d < D; ++d) fc[d][t] = 0.0f;
     }
     if (odd) mc = INFINITY;
 #pragma unroll
@@ -193,28 +225,40 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kTile)
       atomicMax(&bound_v, __float_as_int(mv));
     }
     __syncthreads();
-    // the tile's smallest and second smallest FP32 value and where the smallest is
-    float low[kPointsPer], next[kPointsPer];
-    int at[kPointsPer];
+    // the three smallest minima of a group and where the first two are
+    float low[kPointsPer], next[kPointsPer], third[kPointsPer];
+    int at[kPointsPer], at2[kPointsPer];
 #pragma unroll
     for (int q = 0; q < kPointsPer; ++q) {
-      low[q] = next[q] = INFINITY;
-      at[q] = 0;
+      low[q] = next[q] = third[q] = INFINITY;
+      at[q] = at2[q] = 0;
     }
-#pragma unroll 4
-    for (int t = 0; t < cnt; ++t) {
+    for (int t = 0; t < cnt; t += kGroup) {
+      float least[kPointsPer];
+#pragma unroll
+      for (int h = 0; h < kGroup; h += 4) {
+        ulonglong2 c[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) c[d] = *reinterpret_cast<const ulonglong2*>(&fc[d][t + h]);
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(&fv[t + h]);
+#pragma unroll
+        for (int q = 0; q < kPointsPer; ++q) {
+          unsigned long long s[2];
+          sqdist4<D>(minus[q], c, s);
+          float v0, v1, v2, v3;
+          unpack2(fma2(sc2, s[0], w.x), v0, v1);
+          unpack2(fma2(sc2, s[1], w.y), v2, v3);
+          least[q] = h == 0 ? fminf(min3(v0, v1, v2), v3) : min3(min3(least[q], v0, v1), v2, v3);
+        }
+      }
 #pragma unroll
       for (int q = 0; q < kPointsPer; ++q) {
-        float s = 0.0f;
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          const float e = p[q][d] - fc[t * D + d];
-          s = d == 0 ? e * e : __fmaf_rn(e, e, s);
-        }
-        const float v = __fmaf_rn(sc, s, -fv[t]);
-        next[q] = fminf(next[q], fmaxf(v, low[q]));
-        at[q] = v < low[q] ? t : at[q];
-        low[q] = fminf(low[q], v);
+        const bool first = least[q] < low[q];
+        third[q] = fminf(third[q], fmaxf(least[q], next[q]));
+        at2[q] = first ? at[q] : least[q] < next[q] ? t : at2[q];
+        next[q] = fminf(next[q], fmaxf(least[q], low[q]));
+        at[q] = first ? t : at[q];
+        low[q] = fminf(low[q], least[q]);
       }
     }
 #pragma unroll
@@ -236,27 +280,33 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kTile)
         best[q] = val < best[q] ? val : best[q];
       };
       if (ok[q] && (all || !(low[q] > lim))) {
-        if (!all && next[q] > lim) {
-          take(at[q]);  // the only pair within the error
-        } else {
-          for (int t = 0; t < cnt; ++t) {
+        auto scan = [&](int t0, int t1) {
+          for (int t = t0; t < t1; ++t) {
             if (!all) {
               float s = 0.0f;
 #pragma unroll
               for (int d = 0; d < D; ++d) {
-                const float e = p[q][d] - fc[t * D + d];
+                const float e = p[q][d] - fc[d][t];
                 s = d == 0 ? e * e : __fmaf_rn(e, e, s);
               }
-              if (__fmaf_rn(sc, s, -fv[t]) > lim) continue;
+              if (__fmaf_rn(sc, s, fv[t]) > lim) continue;
             }
             take(t);
           }
+        };
+        auto group = [&](int t) { scan(t, t + kGroup < cnt ? t + kGroup : cnt); };
+        // the pairs within the error are in the groups whose minima are
+        if (all || !(third[q] > lim)) {
+          scan(0, cnt);
+        } else {
+          group(at[q]);
+          if (!(next[q] > lim)) group(at2[q]);
         }
       }
     }
   }
 #pragma unroll
-  for (int q = 0; q < kPointsPer; ++q) part[q * kTile + threadIdx.x] = best[q];
+  for (int q = 0; q < kPointsPer; ++q) part[q * kMinThreads + threadIdx.x] = best[q];
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   cluster.sync();
   if (cluster.block_rank() == 0) {
@@ -264,10 +314,10 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kTile)
     for (int q = 0; q < kPointsPer; ++q) {
       double b = best[q];
       for (int r = 1; r < kSplit; ++r) {
-        const double o = *cluster.map_shared_rank(part + q * kTile + threadIdx.x, r);
+        const double o = *cluster.map_shared_rank(part + q * kMinThreads + threadIdx.x, r);
         b = o < b ? o : b;
       }
-      const int64_t i = ((int64_t)blockIdx.x * kPointsPer + q) * kTile + threadIdx.x;
+      const int64_t i = ((int64_t)blockIdx.x * kPointsPer + q) * kMinThreads + threadIdx.x;
       if (ok[q]) out[i] = b;
     }
   }
@@ -292,19 +342,20 @@ extern "C" int pdot_points_max_sqdist(int64_t m, int64_t n, int32_t dim, const f
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaMemsetAsync(out, 0, sizeof(double), s);
   if (e != cudaSuccess) return report(PDOT_ERR_CUDA, cudaGetErrorString(e));
-  const int64_t blocks = (m + kTile * kPointsPer - 1) / (kTile * kPointsPer);
-  // the second set in shares so that some 8 CTAs per SM run, none below a tile
-  int64_t shares = (148 * 8 + blocks - 1) / blocks;
-  shares = shares < (n + kTile - 1) / kTile ? shares : (n + kTile - 1) / kTile;
-  const int64_t share = (n + shares - 1) / shares;
+  const int64_t blocks = (m + kMaxThreads * kPointsPer - 1) / (kMaxThreads * kPointsPer);
+  // the second set in shares of whole tiles, some 16 CTAs per SM
+  const int64_t tiles = (n + kFarTile - 1) / kFarTile;
+  int64_t shares = (148 * 16 + blocks - 1) / blocks;
+  shares = shares < tiles ? shares : tiles;
+  const int64_t share = (tiles + shares - 1) / shares * kFarTile;
   const dim3 grid((unsigned)blocks, (unsigned)((n + share - 1) / share));
   auto* bits = reinterpret_cast<unsigned long long*>(out);
   if (dim == 1)
-    k_max_sqdist<1><<<grid, kTile, 0, s>>>(m, n, share, source_points, target_points, bits);
+    k_max_sqdist<1><<<grid, kMaxThreads, 0, s>>>(m, n, share, source_points, target_points, bits);
   else if (dim == 2)
-    k_max_sqdist<2><<<grid, kTile, 0, s>>>(m, n, share, source_points, target_points, bits);
+    k_max_sqdist<2><<<grid, kMaxThreads, 0, s>>>(m, n, share, source_points, target_points, bits);
   else
-    k_max_sqdist<3><<<grid, kTile, 0, s>>>(m, n, share, source_points, target_points, bits);
+    k_max_sqdist<3><<<grid, kMaxThreads, 0, s>>>(m, n, share, source_points, target_points, bits);
   e = cudaGetLastError();
   if (e != cudaSuccess) return report(PDOT_ERR_CUDA, cudaGetErrorString(e));
   return PDOT_OK;
@@ -320,13 +371,13 @@ extern "C" int pdot_points_c_transform(int64_t num_points, int64_t num_centres, 
   if (!points || !centres || !duals || !out) return report(PDOT_ERR_INVALID_ARGUMENT, "null pointer argument");
   if (!std::isfinite(scale)) return report(PDOT_ERR_INVALID_ARGUMENT, "scale must be finite");
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const dim3 blocks((unsigned)((num_points + kTile * kPointsPer - 1) / (kTile * kPointsPer)), kSplit);
+  const dim3 blocks((unsigned)((num_points + kMinThreads * kPointsPer - 1) / (kMinThreads * kPointsPer)), kSplit);
   if (dim == 1)
-    k_c_transform<1><<<blocks, kTile, 0, s>>>(num_points, num_centres, points, centres, duals, scale, out);
+    k_c_transform<1><<<blocks, kMinThreads, 0, s>>>(num_points, num_centres, points, centres, duals, scale, out);
   else if (dim == 2)
-    k_c_transform<2><<<blocks, kTile, 0, s>>>(num_points, num_centres, points, centres, duals, scale, out);
+    k_c_transform<2><<<blocks, kMinThreads, 0, s>>>(num_points, num_centres, points, centres, duals, scale, out);
   else
-    k_c_transform<3><<<blocks, kTile, 0, s>>>(num_points, num_centres, points, centres, duals, scale, out);
+    k_c_transform<3><<<blocks, kMinThreads, 0, s>>>(num_points, num_centres, points, centres, duals, scale, out);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return report(PDOT_ERR_CUDA, cudaGetErrorString(e));
   return PDOT_OK;

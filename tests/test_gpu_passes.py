@@ -60,6 +60,21 @@ def test_cost_builder_is_exact_at_the_ends_of_the_range(cuda, scale):
     np.testing.assert_array_equal(_device_cost(cuda, x, y, 1), want)
 
 
+@pytest.mark.parametrize("offset,spread", [(0.0, 1.0), (1e4, 1e-3), (0.0, 1e-25), (0.0, 1e25), (-1e30, 1e16), (0.0, 1e45)])
+@pytest.mark.parametrize("m,n,d", [(700, 1030, 3), (1, 4200001, 1), (513, 8300, 2), (2300, 1930, 3), (2047, 2051, 4)])
+def test_cost_maximum_is_exact(cuda, m, n, d, offset, spread):
+    """Bit for bit on both sides of 2^22 pairs, where FP32 tells the pairs apart and where it does not, and
+    with a first point that is not a number or infinite."""
+    rng = np.random.default_rng(m + n + d)
+    x, y = offset + spread * rng.normal(size=(m, d)), offset + spread * rng.normal(size=(n, d))
+    assert np.array_equal(_device_cost(cuda, x, y, 1), _cost(x, y, 1))
+    for odd in (np.nan, np.inf):
+        x[0, 0], y[n // 2, d - 1] = odd, np.nan
+        with np.errstate(invalid="ignore"):
+            want = _cost(x, y, 1)
+        np.testing.assert_array_equal(_device_cost(cuda, x, y, 1), want)
+
+
 def test_cost_quotients_are_correctly_rounded(cuda):
     """Many quotients by one divisor, of all magnitudes below it: one-dimensional points against the origin."""
     rng = np.random.default_rng(6)
@@ -97,7 +112,7 @@ def _sq(p, q):
 
 
 @pytest.mark.parametrize("offset,spread", [(0.0, 1.0), (1e4, 1e-3), (0.0, 1e-25), (0.0, 1e25)])
-@pytest.mark.parametrize("m,n,d", [(1, 1, 1), (513, 1, 2), (700, 257, 3), (1, 4100, 2), (1025, 2049, 1)])
+@pytest.mark.parametrize("m,n,d", [(1, 1, 1), (513, 1, 2), (700, 257, 3), (1, 4100, 2), (1025, 2049, 1), (256, 64, 2), (129, 2063, 3)])
 def test_pair_passes_are_exact(cuda, m, n, d, offset, spread):
     """Bit for bit, also where FP32 tells no pairs apart (an offset, far above the spread) and where its
     squares underflow or overflow."""
