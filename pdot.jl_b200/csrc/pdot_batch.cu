@@ -173,6 +173,34 @@ __device__ __forceinline__ int find_segment(const long long* prefix, int count, 
   return lo;
 }
 
+// The same for two values at once and a whole warp, each step one load a lane for 32
+// places: two trips to L2 for 512 entries in place of nine, which were a quarter of the
+// time of the vector kernels: their blocks run for a few microseconds and find L1 empty.
+template <bool CO>
+__device__ __forceinline__ void warp_segments(const long long* prefix, int count, long long q0, long long q1, int& k0,
+                                              int& k1) {
+  const int lane = threadIdx.x & 31;
+  int n0 = count, n1 = count;  // the segment is one of [k, k + n)
+  k0 = k1 = 0;
+  while (n0 > 1 || n1 > 1) {
+    const int s0 = (n0 + 31) >> 5, s1 = (n1 + 31) >> 5;
+    const bool in0 = lane * s0 < n0, in1 = lane * s1 < n1;
+    const long long p0 = ldro<CO>(prefix + k0 + (in0 ? lane * s0 : 0)), p1 = ldro<CO>(prefix + k1 + (in1 ? lane * s1 : 0));
+    const int j0 = 31 - __clz(__ballot_sync(0xffffffffu, in0 && p0 <= q0) | 1);
+    const int j1 = 31 - __clz(__ballot_sync(0xffffffffu, in1 && p1 <= q1) | 1);
+    k0 += j0 * s0;
+    k1 += j1 * s1;
+    n0 = n0 - j0 * s0 < s0 ? n0 - j0 * s0 : s0;
+    n1 = n1 - j1 * s1 < s1 ? n1 - j1 * s1 : s1;
+  }
+}
+template <bool CO>
+__device__ __forceinline__ int warp_segment(const long long* prefix, int count, long long q) {
+  int k0, k1;
+  warp_segments<CO>(prefix, count, q, q, k0, k1);
+  return k0;
+}
+
 
 // A lane's per-load partial sums added in load order.
 template <int N>
@@ -699,8 +727,8 @@ __device__ __forceinline__ void kb_dual_body(const BatchBuffers& B, const SolveC
                                              const long long blk) {
   const BatchActive act = *B.act;
   if (act.count == 0 || act.error) return;
-  if (blk >= B.vblock_prefix[act.count]) return;
-  const int kk = find_segment<CO>(B.vblock_prefix, act.count, blk);
+  const int kk = warp_segment<CO>(B.vblock_prefix, act.count, blk);
+  if (blk >= B.vblock_prefix[kk + 1]) return;
   const int k = B.ids[kk];
   const BatchInstance I = B.inst[k];
   DevState* st = B.st + k;
@@ -716,10 +744,13 @@ __device__ __forceinline__ void kb_dual_body(const BatchBuffers& B, const SolveC
   double vals[kStepSums] = {0.0, 0.0};
   if (lb < I.rblocks) {
     const long long i = lb * kVecThreads + threadIdx.x;
+    const long long p = i / PR, t = i - p * PR;
+    int lo = 0, hi = 0;  // the warp's rows lie in one panel
+    if (i - (threadIdx.x & 31) < I.m)
+      warp_segments<CO>(B.cta_begin, grid, ubase + p * I.n, ubase + (p + 1) * I.n - 1, lo, hi);
     if (i < I.m) {
-      const long long p = i / PR, t = i - p * PR;
-      const long long gp = B.panel_prefix[kk] + p;
-      const long long lo = bcta_of_unit(B.cta_begin, grid, ubase + p * I.n), hi = bcta_of_unit(B.cta_begin, grid, ubase + (p + 1) * I.n - 1);
+      const long long gp = B.panel_prefix[kk] + p, o = I.row_off + i;
+      DualPlace place(B.a + o, B.r[buf] + o, B.u[buf] + o, B.r[buf ^ 1] + o, B.u[buf ^ 1] + o);
       double sd = 0.0;
       if (!act.any_empty) {
         // every CTA owns a unit: the slots c + gp, c = lo..hi, all hold partials
@@ -732,15 +763,14 @@ __device__ __forceinline__ void kb_dual_body(const BatchBuffers& B, const SolveC
           sd += B.rowpart[(c + gp) * PR + t];
         }
       }
-      const long long o = I.row_off + i;
-      dual_entry(sd, B.a[o], B.r[buf] + o, B.u[buf] + o, B.r[buf ^ 1] + o, B.u[buf ^ 1] + o, A, vals[0], vals[1]);
+      place.step(sd, A, vals[0], vals[1]);
     }
   } else {
     const long long j = (lb - I.rblocks) * kVecThreads + threadIdx.x;
     if (j < I.n) {
-      const double sd = sum_strided(B.colpart + ubase + j, I.panels, I.n);
       const long long o = I.col_off + j;
-      dual_entry(sd, B.b[o], B.c[buf] + o, B.v[buf] + o, B.c[buf ^ 1] + o, B.v[buf ^ 1] + o, A, vals[0], vals[1]);
+      DualPlace place(B.b + o, B.c[buf] + o, B.v[buf] + o, B.c[buf ^ 1] + o, B.v[buf ^ 1] + o);
+      place.step(sum_strided(B.colpart + ubase + j, I.panels, I.n), A, vals[0], vals[1]);
     }
   }
   block_reduce<kStepSums>(vals, 0u, B.steppart + blk * kStepSums);
@@ -760,7 +790,8 @@ __device__ __forceinline__ void kb_dual_body(const BatchBuffers& B, const SolveC
     if (lane == 0) fin[2] = cs[0], fin[3] = cs[1];
   } else if (w == 2) {
     double xs[1];
-    const long long lo = bcta_of_unit(B.cta_begin, grid, ubase), hi = bcta_of_unit(B.cta_begin, grid, B.unit_prefix[kk + 1] - 1);
+    int lo, hi;
+    warp_segments<CO>(B.cta_begin, grid, ubase, B.unit_prefix[kk + 1] - 1, lo, hi);
     sum_cta_slots<1>(B.sqpart, B.cta_begin, lo, hi, kk, 0u, xs);
     if (lane == 0) fin[4] = xs[0];
   } else if (w == 3 && lane == 0) {
@@ -772,8 +803,11 @@ __device__ __forceinline__ void kb_dual_body(const BatchBuffers& B, const SolveC
     st->ticket_step = 0;
   }
 }
+// A block is a chain of trips to L2, so what counts is their number and how many blocks
+// are resident: 512 instances 47 us and 48 of 1024 x 1024 19 us with the searches of one
+// thread and the loads in turn, 33 and 13 now (43 and 14 with four CTAs per SM).
 template <int PR>
-__global__ void __launch_bounds__(kVecThreads) kb_dual(BatchBuffers B, SolveConfig cfg, int grid) {
+__global__ void __launch_bounds__(kVecThreads, 5) kb_dual(BatchBuffers B, SolveConfig cfg, int grid) {
   pdl_enter();
   kb_dual_body<PR, false>(B, cfg, grid, blockIdx.x);
 }
@@ -870,8 +904,8 @@ __device__ __forceinline__ void kb_eval_vec_body(const BatchBuffers& B, const So
                                                  const int start_only, const long long blk) {
   const BatchActive act = *B.act;
   if (act.count == 0 || act.error) return;
-  if (blk >= B.vblock_prefix[act.count]) return;
-  const int kk = find_segment<CO>(B.vblock_prefix, act.count, blk);
+  const int kk = warp_segment<CO>(B.vblock_prefix, act.count, blk);
+  if (blk >= B.vblock_prefix[kk + 1]) return;
   const int k = B.ids[kk];
   const BatchInstance I = B.inst[k];
   DevState* st = B.st + k;
@@ -911,8 +945,8 @@ __device__ __forceinline__ void kb_eval_vec_body(const BatchBuffers& B, const So
   __shared__ double fin[kEvalSums + 2 * kVecSums];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (w == 0) {
-    const long long lo = bcta_of_unit(B.cta_begin, grid, B.unit_prefix[kk]);
-    const long long hi = bcta_of_unit(B.cta_begin, grid, B.unit_prefix[kk + 1] - 1);
+    int lo, hi;
+    warp_segments<CO>(B.cta_begin, grid, B.unit_prefix[kk], B.unit_prefix[kk + 1] - 1, lo, hi);
     double E[kEvalSums];
     sum_cta_slots<kEvalSums>(B.evpart, B.cta_begin, lo, hi, kk, kEvalMaxMask, E);
     if (lane == 0)
@@ -942,7 +976,9 @@ __device__ __forceinline__ void kb_eval_vec_body(const BatchBuffers& B, const So
     st->ticket_eval = 0;
   }
 }
-__global__ void __launch_bounds__(kVecThreads) kb_eval_vec(BatchBuffers B, SolveConfig cfg, int grid,
+// four CTAs per SM: the blocks wait most of their time (512 instances: 65 us with the two
+// that 122 registers leave room for, 43 with four, some control spilled)
+__global__ void __launch_bounds__(kVecThreads, 4) kb_eval_vec(BatchBuffers B, SolveConfig cfg, int grid,
                                                             int start_only) {
   pdl_enter();
   kb_eval_vec_body<false>(B, cfg, grid, start_only, blockIdx.x);

@@ -672,6 +672,22 @@ __device__ __forceinline__ void dual_entry(double sum_delta, double dist, double
   *ravg = A.first ? rn : __dmul_rn(__dadd_rn(*ravg, __dmul_rn(rn, A.nw)), A.aw);
   *uavg = A.first ? un : __dmul_rn(__dadd_rn(*uavg, __dmul_rn(un, A.nw)), A.aw);
 }
+// A row's or column's place in the dual step. The values are loaded when it is made,
+// before the sum of the partials is there, so that one trip to memory serves both; in
+// turn they took three (the averages' loads could not pass the new values' stores).
+struct DualPlace {
+  double *r, *u, *ravg, *uavg;
+  double dist, vr, vu, vravg, vuavg;
+  __device__ __forceinline__ DualPlace(const double* d, double* r_, double* u_, double* ravg_, double* uavg_)
+      : r(r_), u(u_), ravg(ravg_), uavg(uavg_), dist(*d), vr(*r_), vu(*u_), vravg(*ravg_), vuavg(*uavg_) {}
+  __device__ __forceinline__ void step(double sum_delta, const DualArgs& A, double& dot, double& dy2) {
+    dual_entry(sum_delta, dist, &vr, &vu, &vravg, &vuavg, A, dot, dy2);
+    *r = vr;
+    *u = vu;
+    *ravg = vravg;
+    *uavg = vuavg;
+  }
+};
 
 
 enum { E_DOT = 0, E_SQX, E_MAXX, E_SQG, E_MAXG, E_AVG = 5 };

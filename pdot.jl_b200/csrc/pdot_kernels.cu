@@ -478,9 +478,10 @@ __device__ __forceinline__ void k2_dual_body(const Buffers& B, const Geometry& g
   const int rb = g.dual_row_blocks;
   if (bid < rb && rb == g.row_blocks) {
     const int64_t i = (int64_t)bid * kVecThreads + threadIdx.x;
-    if (i < g.m)
-      dual_entry(finish_row_sum(g, B.rowpart, i), B.a[i], B.r[buf] + i, B.u[buf] + i, B.r[buf ^ 1] + i,
-                 B.u[buf ^ 1] + i, A, vals[0], vals[1]);
+    if (i < g.m) {
+      DualPlace place(B.a + i, B.r[buf] + i, B.u[buf] + i, B.r[buf ^ 1] + i, B.u[buf ^ 1] + i);
+      place.step(finish_row_sum(g, B.rowpart, i), A, vals[0], vals[1]);
+    }
   } else if (bid < rb) {
     // a warp per row: lane l adds slots l, l + 32, ... in order, then a fixed
     // shuffle tree; the row's many slots are read in parallel, not in a chain
@@ -490,18 +491,18 @@ __device__ __forceinline__ void k2_dual_body(const Buffers& B, const Geometry& g
       const int64_t p = i / kPanelRows, t = i - p * kPanelRows;
       const int64_t lo = cta_of_unit(g, p * g.n), hi = cta_of_unit(g, (p + 1) * g.n - 1);
       const double* q = B.rowpart + row_slot(lo, p) * kPanelRows + t;
+      DualPlace place(B.a + i, B.r[buf] + i, B.u[buf] + i, B.r[buf ^ 1] + i, B.u[buf ^ 1] + i);
       double sd = 0.0;
       for (int64_t c = lane; c <= hi - lo; c += 32) sd += q[c * kPanelRows];
       sd = warp_sum(sd);
-      if (lane == 0)
-        dual_entry(sd, B.a[i], B.r[buf] + i, B.u[buf] + i, B.r[buf ^ 1] + i, B.u[buf ^ 1] + i, A, vals[0],
-                   vals[1]);
+      if (lane == 0) place.step(sd, A, vals[0], vals[1]);
     }
   } else {
     const int64_t j = (int64_t)(bid - rb) * kVecThreads + threadIdx.x;
-    if (j < g.n)
-      dual_entry(finish_col_sum(g, B.colpart, j), B.b[j], B.c[buf] + j, B.v[buf] + j, B.c[buf ^ 1] + j,
-                 B.v[buf ^ 1] + j, A, vals[0], vals[1]);
+    if (j < g.n) {
+      DualPlace place(B.b + j, B.c[buf] + j, B.v[buf] + j, B.c[buf ^ 1] + j, B.v[buf ^ 1] + j);
+      place.step(finish_col_sum(g, B.colpart, j), A, vals[0], vals[1]);
+    }
   }
   block_reduce<kStepSums>(vals, 0u, B.steppart + (int64_t)bid * kStepSums);
   if (!elect_last_of(&st->ticket_step, nblocks)) return;
