@@ -6,10 +6,12 @@
 // an optional evaluation (k3 + k4) and a step (k1 + k2). Iterations are
 // grouped in chunks of termination_evaluation_frequency iterations; the
 // regular chunk [eval, step x freq] is captured once as a CUDA graph and
-// replayed. Two chunks are kept in flight; after each one the host reads the
-// device state record (a 200-byte copy) and the new iteration-stats records,
-// and stops once the device has set `done`. All decisions (step size, restart,
-// primal weight, termination) are taken on the device.
+// replayed, or, where the plan fits in the shared memory of the GPU, is an
+// evaluation and one cooperative launch of all its steps (pdot_resident.cu).
+// Two chunks are kept in flight; after each one the host reads the device state
+// record (a 300-byte copy) and the new iteration-stats records, and stops once
+// the device has set `done`. All decisions (step size, restart, primal weight,
+// termination) are taken on the device.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -578,8 +580,8 @@ class Solver {
     warm_zero_ = var.warm_zero;
     freq_ = prm.termination_evaluation_frequency;
     limit_ = prm.termination_criteria.iteration_limit;
-    // automatic = the CUDA graph: on B200 the persistent chunk measured slower
-    // at every size tried (31 against 16 us per iteration at 1000 x 1000, 1071
+    // only on request: on B200 the persistent chunk measured slower than the CUDA
+    // graph at every size tried (31 against 16 us per iteration at 1000 x 1000, 1071
     // against 718 at 10000 x 10000)
     persistent_ = g_.chunk_ctas > 0 && !time_kernels_ && var.persistent == 1;
     use_graph_ = use_graph_ && !time_kernels_ && !persistent_;
