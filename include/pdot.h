@@ -165,7 +165,10 @@ typedef struct pdot_solver_options {
   /* Test hook, 0 in normal use. 1: each consumer wait of the staged fused pass
    * reports a timeout without polling; the kernel still waits (bounded) for the
    * copies it has in flight, sets its error word and returns, and the call
-   * fails with PDOT_ERR_CUDA. It exercises the timeout path without a fault. */
+   * fails with PDOT_ERR_CUDA. Where small problems run their steps as one
+   * launch, one CTA's wait at a grid barrier reports a timeout in the same way,
+   * and the others leave on its error. It exercises the timeout paths without a
+   * fault. */
   int32_t fail_bounded_waits;
   /* With a warm start: 0 (default) starts the restart information (the last
    * restart point of the adaptive restart test and of the primal-weight

@@ -50,7 +50,9 @@ struct Geometry {
   int32_t cost_kind;   // PDOT_COST_F64 / _F32 / _BF16, or a coordinate kind (internal_cost_kind)
   int32_t tma;         // 1: the fused pass stages its operands with bulk copies
   int32_t tma_smem;    // dynamic shared memory of the staged pass (bytes)
-  int32_t fail_waits;  // test hook: the staged pass's consumer waits report a timeout at once
+  // test hook: the staged pass's consumer waits, and a barrier of the resident steps in one
+  // CTA, report a timeout at once
+  int32_t fail_waits;
   // CTAs of the dual step covering the rows: row_blocks (a thread per row) or,
   // when a panel's row partials lie in many CTA slots (small problems, kDualWarpSlots
   // or more), ceil(m / kWarps) (a warp per row)

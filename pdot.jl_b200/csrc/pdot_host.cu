@@ -239,7 +239,7 @@ struct Variant {
   double plan_eps = 0.0;  // > 0: recover the warm plan from the warm duals
   int plan_iters = 0;
   int staged = 2;  // 0 direct, 1 staged, 2 automatic
-  int fail_waits = 0;  // test hook: the staged pass's waits report timeouts
+  int fail_waits = 0;  // test hook: waits of the staged pass and the resident steps report timeouts
   double warm_omega = 0.0;  // > 0: initial primal weight of a warm start
   bool warm_zero = false;   // a warm start's restart information starts at the zero point
   int persistent = 0;       // persistent chunk kernel: 0 automatic, 1 on, -1 off
@@ -587,7 +587,7 @@ class Solver {
     use_graph_ = use_graph_ && !time_kernels_ && !persistent_;
     // small problems: the steps between two evaluations as one launch with the plan in
     // shared memory, bit-identical to the graph's
-    if (use_graph_ && var.persistent == 0 && !g_.fail_waits && freq_ >= kResidentSteps)
+    if (use_graph_ && var.persistent == 0 && freq_ >= kResidentSteps)
       resident_ = pdot::resident_ctas(g_, device_);
     if (resident_) resident_scratch_ = alloc_bytes(pdot::resident_scratch_bytes());
     reset();
@@ -685,7 +685,8 @@ class Solver {
       if (status_.kernel_error) {
         sync_all(issued, completed);
         fail(PDOT_ERR_CUDA,
-             "a bounded wait timed out (staged primal pass or persistent chunk barrier; kernel_error %d)",
+             "a bounded wait timed out (staged primal pass, or a barrier of the resident steps or the persistent "
+             "chunk; kernel_error %d)",
              status_.kernel_error);
       }
       if (status_.done) break;

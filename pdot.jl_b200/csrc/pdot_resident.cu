@@ -50,15 +50,17 @@ __device__ __forceinline__ void half_sync(int half) { asm volatile("bar.sync %0,
 // Arrives and waits until all CTAs of the grid have arrived `round` times (the counter
 // is zero at the launch). The CTA's writes are released by thread 0 after the CTA's
 // own barrier, and what the others released is visible to the CTA after it. False when
-// the wait ran out or another CTA's did.
-__device__ __forceinline__ bool res_barrier(unsigned* count, unsigned target, const int* abort_flag) {
+// the wait ran out or another CTA's did. A CTA that is to `give_up` (test hook) reports
+// a run-out in place of arriving, so that the others' waits end by its error.
+__device__ __forceinline__ bool res_barrier(unsigned* count, unsigned target, const int* abort_flag,
+                                            bool give_up = false) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
-    int good = 1, it = 0;
+    if (!give_up) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+    int good = give_up ? 0 : 1, it = 0;
     unsigned long long t0 = 0;
-    while (ld_acquire_gpu(count) < target) {
+    while (good && ld_acquire_gpu(count) < target) {
       if ((++it & 255) == 0) {
         const unsigned long long t = globaltimer_ns();
         if (t0 == 0) t0 = t;
@@ -114,7 +116,10 @@ __global__ void __launch_bounds__(kResThreads, 1)
   __shared__ StepPowers pw;
   __shared__ DevState loc;
   DevState* st = B.st;
-  if (st->done | st->numerical_error | st->kernel_error) return;  // nothing of it changes before the first barrier
+  // One answer for the CTA: done and numerical_error stay as they are until every CTA is
+  // here, but a CTA whose wait ran out may set kernel_error while this one starts, and
+  // warps that left on it would be missed for good by the others' named barriers.
+  if (__syncthreads_or(st->done | st->numerical_error | st->kernel_error)) return;
   const int buf = st->buf;
   const int half = threadIdx.x / kHalf, tid = threadIdx.x % kHalf, lane = tid & 31, warp = tid >> 5;
   const int64_t m = g.m, n = g.n, vcta = (int64_t)blockIdx.x * 2 + half;
@@ -375,7 +380,8 @@ __global__ void __launch_bounds__(kResThreads, 1)
       warp_reduce_partials<1>(B.sqpart, 0, g.grid, 0u, xs);
       if (lane == 0) *sqsum = xs[0];
     }
-    if (!(alive = res_barrier(bar, ctas * ++round, &st->kernel_error))) break;
+    const bool give_up = g.fail_waits && blockIdx.x == 0;
+    if (!(alive = res_barrier(bar, ctas * ++round, &st->kernel_error, give_up))) break;
 
     fetch();
     if (threadIdx.x < 32) {

@@ -402,7 +402,8 @@ def _options(device: int, use_cuda_graph: bool, time_kernels: bool = False, *, p
     recover_plan  (eps, rounds): with warm duals and no plan, the plan is
                recovered from the duals by `rounds` of log-domain balancing
                of exp((u_i + v_j - C_ij) / eps)
-    fail_bounded_waits  test hook: the staged pass's waits report a timeout at
+    fail_bounded_waits  test hook: the staged pass's waits, and one CTA's at a
+               grid barrier of a small problem's steps, report a timeout at
                once (the call then fails with PDOT_ERR_CUDA)
     warm_primal_weight  with a warm start: the initial primal weight (None:
                primal_importance, or the scale-invariant choice)

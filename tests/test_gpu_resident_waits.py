@@ -1,0 +1,35 @@
+"""The grid barriers of a small problem's resident steps, when a wait runs out: no fault
+and no hang, every CTA leaves, and the context serves the next solve."""
+import numpy as np
+import pytest
+
+import pdot
+from pdot import _abi, instances
+
+pytestmark = pytest.mark.gpu
+
+
+def _same(a, b):
+    assert a.iteration_count == b.iteration_count
+    assert a.termination_reason == b.termination_reason
+    for f in ("primal_solution", "dual_source_solution", "dual_target_solution"):
+        assert np.array_equal(getattr(a, f), getattr(b, f)), f
+
+
+# one CTA, a few, and one on every SM; FP64, and an FP32 plan with a computed cost
+@pytest.mark.parametrize("m,n,cost", [(20, 1, "f64"), (127, 93, "f64"), (600, 500, "f64"), (700, 600, "sqeuclid")])
+def test_a_run_out_barrier_ends_the_call(cuda, m, n, cost):
+    """One CTA's wait reports a run-out at the second barrier of the launch; the others, which wait for it,
+    leave on its error. Then the same solve, unhooked, is the graph's bit for bit."""
+    rng = np.random.default_rng(2)
+    prob = instances.uniform_sqeuclid(m, n, seed=2)
+    kw = {"primal_pass": "direct"}
+    if cost != "f64":
+        kw.update(precision="f32", cost=cost, points=tuple(rng.uniform(0, 1, (k, 2)).astype(np.float32) for k in (m, n)))
+    params = pdot.default_parameters(1e-9, iteration_limit=150)
+    for _ in range(3):
+        with pytest.raises(_abi.PdotError) as ei:
+            pdot.optimize(params, prob, fail_bounded_waits=True, **kw)
+        assert ei.value.code == _abi.PDOT_ERR_CUDA
+        assert "resident steps" in str(ei.value)
+    _same(pdot.optimize(params, prob, persistent=False, **kw), pdot.optimize(params, prob, **kw))
