@@ -187,8 +187,9 @@ typedef struct pdot_solver_options {
    * one) as one persistent cooperative launch with grid barriers between the
    * phases, instead of a CUDA graph of separate launches; the results are
    * bit-identical. 0: automatic (for problems whose plan, average and cost fit
-   * the SMs' shared memory, the steps between two evaluations as one such launch
-   * with them resident there; else, or with use_cuda_graph 0, as for -1), 1:
+   * the SMs' shared memory, the steps between two evaluations as one launch with
+   * them resident there, while no other work holds the SMs that it needs; else, or
+   * with use_cuda_graph 0, as for -1), 1:
    * whenever the direct 16-byte pass runs, -1: never. The batched
    * solver takes it too: 1 runs its regular chunks (evaluation, compaction,
    * steps) as one persistent launch with the direct pass throughout (the

@@ -137,7 +137,7 @@ struct DevState {
   int buf;                   // which half of each pair is the current iterate
   int out_current;           // at termination: 1 = return current, 0 = average
   int last_restart_choice;
-  int kernel_error;          // non-zero: a bounded wait in a kernel timed out
+  int kernel_error;          // non-zero: a bounded wait in a kernel timed out (kWaitRanOut, kNotStarted)
   unsigned int ticket_step;  // last-CTA tickets
   unsigned int ticket_eval;
   unsigned int ticket_init;
@@ -145,6 +145,10 @@ struct DevState {
   unsigned int bar_gen;      // and generation
   int pad_[1];
 };
+
+// DevState::kernel_error. Either stops every kernel of the solve that follows.
+constexpr int kWaitRanOut = 1;   // a wait inside a kernel or between its CTAs: an error
+constexpr int kNotStarted = 2;   // the CTAs of resident steps were not all on the GPU: nothing ran
 
 // Parameters of one solve, passed by value to the control kernels.
 struct SolveConfig {
@@ -220,10 +224,11 @@ cudaError_t launch_step(const Buffers& B, const Geometry& g, const SolveConfig& 
 // one persistent cooperative launch (needs g.chunk_ctas > 0); bit-identical to
 // launch_eval followed by the steps.
 cudaError_t launch_chunk(const Buffers& B, const Geometry& g, const SolveConfig& cfg, cudaStream_t s, int steps);
-// `steps` steps of a small problem as one cooperative launch of `ctas` CTAs with the
-// plan and cost in shared memory (pdot_resident.cu), bit-identical to launch_step so
-// often; `scratch` is device memory of the caller's. resident_ctas: the CTAs, 0 where
-// the problem does not fit.
+// `steps` steps of a small problem as one launch of `ctas` CTAs with the plan and cost
+// in shared memory (pdot_resident.cu), bit-identical to launch_step so often; `scratch`
+// is device memory of the caller's. When the CTAs do not all find room on the GPU, no
+// step is taken and kernel_error becomes kNotStarted. resident_ctas: the CTAs, 0 where the
+// problem does not fit.
 int resident_ctas(const Geometry& g, int device);
 size_t resident_scratch_bytes();
 cudaError_t launch_resident(const Buffers& B, const Geometry& g, const SolveConfig& cfg, cudaStream_t s, int ctas,

@@ -7,7 +7,7 @@
 // grouped in chunks of termination_evaluation_frequency iterations; the
 // regular chunk [eval, step x freq] is captured once as a CUDA graph and
 // replayed, or, where the plan fits in the shared memory of the GPU, is an
-// evaluation and one cooperative launch of all its steps (pdot_resident.cu).
+// evaluation and one launch of all its steps (pdot_resident.cu).
 // Two chunks are kept in flight; after each one the host reads the device state
 // record (a 300-byte copy) and the new iteration-stats records, and stops once
 // the device has set `done`. All decisions (step size, restart, primal weight,
@@ -658,6 +658,9 @@ class Solver {
     CK(cudaMemcpy(&status_, st_, sizeof(status_), cudaMemcpyDeviceToHost));
     host_it_ = 1;
     drained_ = 0;
+    resident_from_ = 10;
+    not_started_ = 0;
+    replay_ = 0;
     records_.clear();
     primal_ms_ = dual_ms_ = eval_ms_ = 0.0;
     timed_primal_ = 0;
@@ -682,6 +685,19 @@ class Solver {
       collect_timings(slot);
       ++completed;
       drain();
+      if (status_.kernel_error == pdot::kNotStarted) {
+        // Other work held SMs: no step of that launch ran, nor anything that was enqueued
+        // behind it. Its steps (its evaluation has run) are launched one by one, and the
+        // next chunks as the graph, twice as many after each further time.
+        sync_all(issued, completed);
+        CK(cudaMemsetAsync(&st_->kernel_error, 0, sizeof(int), stream_));
+        status_.kernel_error = 0;
+        replay_ = resident_launch_[slot].steps;
+        remaining += host_it_ - resident_launch_[slot].it;
+        host_it_ = resident_launch_[slot].it;
+        resident_from_ = host_it_ + replay_ + freq_ * (8ll << std::min(not_started_++, 20));
+        continue;
+      }
       if (status_.kernel_error) {
         sync_all(issued, completed);
         fail(PDOT_ERR_CUDA,
@@ -865,7 +881,13 @@ class Solver {
 
   // Enqueues up to `budget` loop bodies starting at host_it_; returns how many.
   int64_t enqueue_chunk(int64_t budget, int slot) {
-    if (resident_ && host_it_ >= 10) {
+    if (replay_ > 0) {
+      const int64_t k = replay_;
+      for (; replay_ > 0; --replay_, ++host_it_)
+        CK(pdot::launch_step(B_, g_, cfg_, stream_, is_eval(host_it_ + 1) ? 1 : 0));
+      return k;
+    }
+    if (resident_ && host_it_ >= resident_from_) {
       // the evaluation due now, then every step up to the next one in one launch (a
       // launch of a few steps would spend more on filling shared memory)
       int64_t k = 1;
@@ -873,6 +895,7 @@ class Solver {
       if (k >= kResidentSteps || host_it_ > limit_) {
         if (is_eval(host_it_)) CK(pdot::launch_eval(B_, g_, cfg_, stream_));
         if (host_it_ <= limit_) CK(pdot::launch_resident(B_, g_, cfg_, stream_, resident_, (int)k, resident_scratch_));
+        resident_launch_[slot] = {host_it_, k};
         host_it_ += k;
         return k;
       }
@@ -896,7 +919,7 @@ class Solver {
       ++k;
       // the evaluation at iteration_limit + 1 ends the solve: nothing after it runs
     } while (k < freq_ && k < budget && host_it_ <= limit_ + 1 && !regular_start(host_it_) &&
-             !(resident_ && host_it_ >= 10));
+             !(resident_ && host_it_ >= resident_from_));
     return k;
   }
 
@@ -962,6 +985,13 @@ class Solver {
   bool persistent_ = false;  // regular chunks run as one persistent launch
   int resident_ = 0;         // CTAs of the resident steps, 0: the problem does not fit
   void* resident_scratch_ = nullptr;
+  struct {
+    long long it;
+    int64_t steps;
+  } resident_launch_[kInFlight] = {};  // of the chunk in each slot, where it is one
+  long long resident_from_ = 10;       // first loop body that may start one
+  int not_started_ = 0;                // launches that found no room since reset()
+  int64_t replay_ = 0;                 // steps of one that are due
   pdot_pdhg_parameters params_;
   pdot::Geometry g_{};
   pdot::SolveConfig cfg_{};

@@ -1,5 +1,5 @@
 // pdot_resident.cu — the iterations between two evaluations of a small problem as one
-// cooperative launch that keeps the plan, its average and the cost in shared memory.
+// launch that keeps the plan, its average and the cost in shared memory.
 //
 // A problem of a few megabytes is bound by latency: an iteration of primal pass and dual
 // step took 17 us at 1000 x 1000 in FP64 and 12 us at 127 x 93 on B200 as two launches of
@@ -31,7 +31,17 @@
 // they can be. Control by one CTA that publishes the result measured 25 % slower.
 //
 // What other CTAs wrote is read through L2 (__ldcg): the L1 of an SM may hold the last
-// iteration's line. The barriers are bounded like those of the persistent chunks.
+// iteration's line.
+//
+// The CTAs take an SM each, and other work on the GPU may hold some. A cooperative launch
+// would wait until all of them are free: a solve of 2.5 ms beside a kernel of one thread
+// that runs for 1.6 s took 1.6 s, where the graph takes 3.7 ms. So the launch is an
+// ordinary one, and its first barrier finds out whether its CTAs are all resident, as the
+// discovery protocol of Sorensen et al. (OOPSLA 2016) does: after kGatherLimitNs without
+// the last arrival the CTAs give up, nothing has been changed but partial sums, and the
+// host runs the steps as launches of their own. Past the first barrier every CTA is on an
+// SM and stays there; the other barriers are bounded by kWaitLimitNs, and a run-out there
+// is an error.
 #include <type_traits>
 
 #include "pdot_device.cuh"
@@ -43,35 +53,46 @@ constexpr int kHalf = 256;            // threads of a CTA range and of a dual bl
 constexpr int kResThreads = 2 * kHalf;
 constexpr int kResSmem = 227 * 1024;  // shared memory of a CTA
 constexpr int kResFixed = 37 * 1024;  // of it, static arrays (row-sum tiles, state)
+// 148 CTAs are through their first primal pass 10 to 20 us after the launch; in 200 us a
+// short kernel of another stream makes room too, and the SMs are not held longer for nothing.
+constexpr unsigned long long kGatherLimitNs = 200000ull;
 static_assert(kHalf == kThreads && kHalf == kVecThreads, "a half runs the other kernels' blocks");
 
 __device__ __forceinline__ void half_sync(int half) { asm volatile("bar.sync %0, %1;" ::"r"(half + 1), "n"(kHalf) : "memory"); }
 
-// Arrives and waits until all CTAs of the grid have arrived `round` times (the counter
-// is zero at the launch). The CTA's writes are released by thread 0 after the CTA's
-// own barrier, and what the others released is visible to the CTA after it. False when
-// the wait ran out or another CTA's did. A CTA that is to `give_up` (test hook) reports
-// a run-out in place of arriving, so that the others' waits end by its error.
-__device__ __forceinline__ bool res_barrier(unsigned* count, unsigned target, const int* abort_flag,
+// Arrives and waits until `target` arrivals are counted (the counter is zero at the
+// launch), but at most `limit_ns`. The CTA's writes are released by thread 0 after the
+// CTA's own barrier, and what the others released is visible to the CTA after it. False
+// when this wait or another CTA's ran out: a CTA gives up by setting the counter's top bit
+// while arrivals are missing, and by nothing else, so either all CTAs pass a barrier or
+// none does. (Each compare-and-swap that fails saw one more arrival.) A CTA that is to
+// `give_up` (test hook) does so in place of arriving.
+constexpr unsigned kGaveUp = 0x80000000u;  // above every target
+__device__ __forceinline__ bool res_barrier(unsigned* count, unsigned target, unsigned long long limit_ns,
                                             bool give_up = false) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     if (!give_up) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
-    int good = give_up ? 0 : 1, it = 0;
+    int it = 0;
     unsigned long long t0 = 0;
-    while (good && ld_acquire_gpu(count) < target) {
-      if ((++it & 255) == 0) {
+    bool late = give_up;
+    for (;;) {
+      const unsigned seen = ld_acquire_gpu(count);
+      if (seen >= target) {
+        ok = (seen & kGaveUp) == 0;
+        break;
+      }
+      if (late && atomicCAS(count, seen, seen | kGaveUp) == seen) {
+        ok = 0;
+        break;
+      }
+      if ((++it & 15) == 0) {
         const unsigned long long t = globaltimer_ns();
         if (t0 == 0) t0 = t;
-        if (t - t0 > kWaitLimitNs || it >= kSpinLimit ||
-            ld_acquire_gpu(reinterpret_cast<const unsigned*>(abort_flag)) != 0u) {
-          good = 0;
-          break;
-        }
+        late |= t - t0 > limit_ns || it >= kSpinLimit;
       }
     }
-    ok = good;
   }
   __syncthreads();
   return ok != 0;
@@ -338,7 +359,8 @@ __global__ void __launch_bounds__(kResThreads, 1)
       else
         primal(std::true_type());
     }
-    if (!(alive = res_barrier(bar, ctas * ++round, &st->kernel_error))) break;
+    ++round;
+    if (!(alive = res_barrier(bar, ctas * round, round == 1 ? kGatherLimitNs : kWaitLimitNs))) break;
 
     if (in_dual) {
       DualArgs A;
@@ -381,7 +403,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
       if (lane == 0) *sqsum = xs[0];
     }
     const bool give_up = g.fail_waits && blockIdx.x == 0;
-    if (!(alive = res_barrier(bar, ctas * ++round, &st->kernel_error, give_up))) break;
+    if (!(alive = res_barrier(bar, ctas * ++round, kWaitLimitNs, give_up))) break;
 
     fetch();
     if (threadIdx.x < 32) {
@@ -413,7 +435,8 @@ __global__ void __launch_bounds__(kResThreads, 1)
     if (loc.numerical_error) break;  // the same in every CTA
   }
   if (!alive) {
-    if (threadIdx.x == 0) atomicExch(&st->kernel_error, 1);
+    // before the first barrier only partial sums were written
+    if (threadIdx.x == 0) atomicExch(&st->kernel_error, round == 1 ? kNotStarted : kWaitRanOut);
     return;
   }
   each_unit([&](unsigned char* s2, int r, int64_t at) {
@@ -480,24 +503,22 @@ size_t resident_smem(const Geometry& g) {
 
 // The CTAs of the resident steps, 0 where they cannot run: the two CTA ranges of a CTA
 // must fit its shared memory (some 1.1 M entries in FP64, 3.6 M with an FP32 plan and
-// coordinate costs), every block of the dual step a half of its own, and all CTAs the
-// device at once.
+// coordinate costs), every block of the dual step a half of its own, and all CTAs an
+// otherwise idle device at once.
 int resident_ctas(const Geometry& g, int device) {
   const int ctas = (g.grid + 1) / 2;
   if (g.dual_row_blocks + g.col_blocks > 2 * ctas) return 0;
   const size_t smem = resident_smem(g);
   if (smem > (size_t)(kResSmem - kResFixed)) return 0;
-  int sms = 0, coop = 0, occ = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess)
-    sms = 0;
+  int sms = 0, occ = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) sms = 0;
   PDOT_RES_VARIANT(g, {
     if (cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem - kResFixed) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kfn, kResThreads, smem) != cudaSuccess)
       occ = 0;
   });
   cudaGetLastError();
-  return coop && (int64_t)occ * sms >= ctas ? ctas : 0;
+  return (int64_t)occ * sms >= ctas ? ctas : 0;
 }
 
 size_t resident_scratch_bytes() { return 64; }
@@ -511,8 +532,8 @@ cudaError_t launch_resident(const Buffers& B, const Geometry& g, const SolveConf
   Geometry gg = g;
   SolveConfig c = cfg;
   void* args[] = {&b, &gg, &c, &steps, &bar};
-  PDOT_RES_VARIANT(g, (e = cudaLaunchCooperativeKernel((const void*)kfn, dim3((unsigned)ctas), dim3(kResThreads), args,
-                                                       resident_smem(g), s)));
+  PDOT_RES_VARIANT(g, (e = cudaLaunchKernel((const void*)kfn, dim3((unsigned)ctas), dim3(kResThreads), args,
+                                            resident_smem(g), s)));
   return e;
 }
 

@@ -33,3 +33,37 @@ def test_a_run_out_barrier_ends_the_call(cuda, m, n, cost):
         assert ei.value.code == _abi.PDOT_ERR_CUDA
         assert "resident steps" in str(ei.value)
     _same(pdot.optimize(params, prob, persistent=False, **kw), pdot.optimize(params, prob, **kw))
+
+
+@pytest.mark.parametrize("m,n,cost", [(600, 500, "f64"), (1216, 900, "f64"), (700, 601, "sqeuclid")])
+def test_a_busy_sm_does_not_hold_a_solve_up(cuda, m, n, cost):
+    """Beside a kernel of another stream that keeps one SM for a second and more, the resident steps find no
+    room for all their CTAs: the solve takes the launches of the graph, ends long before that kernel, and is
+    bit-identical; so it is when the kernel has gone and the resident steps come back."""
+    import torch
+
+    rng = np.random.default_rng(2)
+    prob = instances.uniform_sqeuclid(m, n, seed=2)
+    kw = {}
+    if cost != "f64":
+        kw.update(precision="f32", cost=cost, points=tuple(rng.uniform(0, 1, (k, 2)).astype(np.float32) for k in (m, n)))
+    params = pdot.default_parameters(1e-9, iteration_limit=6000)
+    ref = pdot.optimize(params, prob, persistent=False, **kw)
+    side = torch.cuda.Stream()
+    pdot.optimize(params, prob, **kw)
+    s = pdot.Solver(params, prob, **kw)
+    try:
+        for pieces in ((300, 77, 500), (5, 1000)):
+            s.reset()
+            s.iterate(200)
+            with torch.cuda.stream(side):
+                torch.cuda._sleep(2_500_000_000)  # cycles of one thread
+                over = torch.cuda.Event()
+                over.record()
+            for k in pieces:
+                s.iterate(k)
+            assert not over.query()
+            over.synchronize()
+            _same(ref, s.finish())
+    finally:
+        s.close()
