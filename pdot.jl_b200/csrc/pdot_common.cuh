@@ -228,7 +228,9 @@ cudaError_t launch_chunk(const Buffers& B, const Geometry& g, const SolveConfig&
 // in shared memory (pdot_resident.cu), bit-identical to launch_step so often; `scratch`
 // is device memory of the caller's. When the CTAs do not all find room on the GPU, no
 // step is taken and kernel_error becomes kNotStarted. resident_ctas: the CTAs, 0 where the
-// problem does not fit.
+// problem does not fit. A launch takes up to kMaxResidentSteps steps, some 10 ms and more of
+// every SM; evaluations further apart than that need several.
+constexpr int kMaxResidentSteps = 1024;
 int resident_ctas(const Geometry& g, int device);
 size_t resident_scratch_bytes();
 cudaError_t launch_resident(const Buffers& B, const Geometry& g, const SolveConfig& cfg, cudaStream_t s, int ctas,

@@ -368,7 +368,7 @@ int64_t pass_workspace_bytes(const pdot::Geometry& g) {
 
 constexpr int kRingCap = 4096;
 constexpr int kInFlight = 2;
-constexpr int kResidentSteps = 4;  // fewest steps of a resident launch
+constexpr int kResidentSteps = 4;  // fewest steps of a resident launch (and pdot::kMaxResidentSteps the most)
 
 
 enum TimedKind { kTimedPrimal = 0, kTimedDual = 1, kTimedEval = 2 };
@@ -889,9 +889,11 @@ class Solver {
     }
     if (resident_ && host_it_ >= resident_from_) {
       // the evaluation due now, then every step up to the next one in one launch (a
-      // launch of a few steps would spend more on filling shared memory)
+      // launch of a few steps would spend more on filling shared memory); the next chunk
+      // goes on where the bound on a launch's steps ends it
+      const int64_t most = std::min<int64_t>(budget, pdot::kMaxResidentSteps);
       int64_t k = 1;
-      while (k < budget && !is_eval(host_it_ + k)) ++k;
+      while (k < most && !is_eval(host_it_ + k)) ++k;
       if (k >= kResidentSteps || host_it_ > limit_) {
         if (is_eval(host_it_)) CK(pdot::launch_eval(B_, g_, cfg_, stream_));
         if (host_it_ <= limit_) CK(pdot::launch_resident(B_, g_, cfg_, stream_, resident_, (int)k, resident_scratch_));

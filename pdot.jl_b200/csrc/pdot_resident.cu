@@ -525,6 +525,8 @@ size_t resident_scratch_bytes() { return 64; }
 
 cudaError_t launch_resident(const Buffers& B, const Geometry& g, const SolveConfig& cfg, cudaStream_t s, int ctas,
                             int steps, void* scratch) {
+  // two arrivals of every CTA a step stay below the counter's top bit
+  if (steps < 1 || steps > kMaxResidentSteps || (int64_t)ctas * 2 * steps >= (int64_t)kGaveUp) return cudaErrorInvalidValue;
   unsigned* bar = static_cast<unsigned*>(scratch);
   cudaError_t e = cudaMemsetAsync(bar, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) return e;

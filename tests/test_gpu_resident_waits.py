@@ -67,3 +67,22 @@ def test_a_busy_sm_does_not_hold_a_solve_up(cuda, m, n, cost):
             _same(ref, s.finish())
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("freq,limit", [(3000, 7000), (1027, 2600), (50_000, 2060)])
+def test_evaluations_far_apart_take_several_launches(cuda, freq, limit):
+    """More steps between two evaluations than one launch may take: the next launch goes on, without an
+    evaluation in between; the last steps of an interval may be too few for a launch of their own."""
+    prob = instances.uniform_sqeuclid(300, 200, seed=9)
+    params = pdot.default_parameters(1e-9, iteration_limit=limit)
+    params.termination_evaluation_frequency = freq
+    want, got = (pdot.optimize(params, prob, persistent=p) for p in (False, None))
+    _same(want, got)
+    assert [s.iteration_number for s in want.iteration_stats] == [s.iteration_number for s in got.iteration_stats]
+    s = pdot.Solver(params, prob)
+    try:
+        s.iterate(1500)
+        s.iterate(3)
+        _same(want, s.finish())
+    finally:
+        s.close()
