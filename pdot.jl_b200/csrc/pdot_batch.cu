@@ -1647,9 +1647,9 @@ class BatchSolver {
     fill_config(prm);
     freq_ = prm.termination_evaluation_frequency;
     limit_ = prm.termination_criteria.iteration_limit;
-    void* hp = pdot::pinned_slot_take();
-    if (!hp) BCK(cudaMallocHost(&hp, sizeof(pdot::BatchActive) * 2));
-    host_act_ = static_cast<pdot::BatchActive*>(hp);
+    static_assert(sizeof(pdot::BatchActive) * 2 <= pdot::kPinnedSlot, "the records fit a slot");
+    BCK(act_slot_.take());
+    host_act_ = static_cast<pdot::BatchActive*>(act_slot_.p);
     for (int k = 0; k < 2; ++k) BCK(cudaEventCreateWithFlags(&ev_[k], cudaEventDisableTiming));
     use_graph_ = use_graph_ && !persistent_;
     undo.s = nullptr;
@@ -1662,7 +1662,7 @@ class BatchSolver {
     if (graph_) cudaGraphExecDestroy(graph_);
     for (int k = 0; k < 2; ++k)
       if (ev_[k]) cudaEventDestroy(ev_[k]);
-    if (host_act_ && !pdot::pinned_slot_return(host_act_)) cudaFreeHost(host_act_);
+    act_slot_.release();
     for (void* p : allocs_) cudaFree(p);
     if (stream_) cudaStreamDestroy(stream_);
   }
@@ -1946,6 +1946,7 @@ class BatchSolver {
   cudaStream_t stream_ = nullptr;
   cudaGraphExec_t graph_ = nullptr;
   cudaEvent_t ev_[2] = {};
+  pdot::PinnedSlot act_slot_;
   pdot::BatchActive* host_act_ = nullptr;
 };
 

@@ -308,13 +308,19 @@ cudaError_t copy_to_host(double* dst, size_t count, const ChunkSource& source, c
 // after the work that uses it has ended; cudaFreeAsync a pooled one in stream order.
 constexpr size_t kPoolBlock = size_t(512) << 20;
 cudaError_t device_alloc(void** p, size_t bytes, cudaStream_t s, bool* pooled = nullptr);
+// The id of the current context (made if there is none). No two contexts of a program
+// have the same one, so what is kept with an id is stale when the id is another.
+cudaError_t current_context(unsigned long long* id);
 // kPinnedSlot bytes of page-locked host memory for a solve's status reads, from a
-// block that is kept; null when all slots are taken (or page-locking failed), the
-// caller then locks its own.
+// block that is kept, or its own when all slots are taken.
 constexpr size_t kPinnedSlot = 4096;
-void* pinned_slot_take();
-// Returns a slot; false when `p` is none (the caller's own memory).
-bool pinned_slot_return(void* p);
+struct Kept;
+struct PinnedSlot {
+  void* p = nullptr;
+  Kept* from = nullptr;  // whose block it is in, null: memory of its own
+  cudaError_t take();
+  void release();
+};
 
 // Sets the thread-local text pdot_last_error() returns (pdot_host.cu).
 void set_last_error(const char* msg);

@@ -25,6 +25,8 @@
 #include <thread>
 #include <vector>
 
+#include <cuda.h>
+
 #include "pdot_common.cuh"
 
 namespace {
@@ -71,47 +73,92 @@ void set_last_error(const char* msg) { g_last_error = msg ? msg : ""; }
 // rounding after a synchronisation took 0.5 ms for its scratch.) While a stream is
 // captured the block belongs to the graph. When the pool cannot serve a block it is
 // trimmed and the block taken from cudaMalloc.
-constexpr int kPoolDevices = 64;
+//
+// All of it goes with its context (cudaDeviceReset), so it is kept by the context's id,
+// which the driver gives out once in the life of a program, and another context gets
+// its own.
 constexpr uint64_t kPoolKeep = uint64_t(1) << 30;
 constexpr int kPinnedSlots = 16;
 
-namespace {
-// never destroyed: the driver may be gone by the time static objects are
 struct Kept {
-  std::mutex mu;
-  cudaMemPool_t pool[kPoolDevices] = {};
+  unsigned long long context = 0;
+  cudaMemPool_t pool = nullptr;
   unsigned char* pinned = nullptr;
   bool pinned_tried = false;
   unsigned taken = 0;  // bit k: slot k of `pinned`
 };
-Kept& kept() {
-  static Kept* k = new Kept;
-  return *k;
+
+namespace {
+std::mutex g_kept_mutex;
+// One for each context that was used; never destroyed, as the driver may be gone by the
+// time static objects are.
+std::vector<Kept*>& all_kept() {
+  static auto* v = new std::vector<Kept*>;
+  return *v;
 }
 
-cudaError_t pool_of(int device, cudaMemPool_t* pool) {
-  Kept& k = kept();
-  std::lock_guard<std::mutex> lock(k.mu);
-  if (!k.pool[device]) {
+// What is kept for the current context; null when there is none to be found. The caller
+// holds g_kept_mutex.
+Kept* kept_here() {
+  unsigned long long context = 0;
+  if (current_context(&context) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  for (Kept* k : all_kept())
+    if (k->context == context) return k;
+  Kept* k = new (std::nothrow) Kept;
+  if (!k) return nullptr;
+  k->context = context;
+  all_kept().push_back(k);
+  return k;
+}
+
+cudaError_t pool_here(cudaMemPool_t* pool) {
+  std::lock_guard<std::mutex> lock(g_kept_mutex);
+  Kept* k = kept_here();
+  if (!k) return cudaErrorNotSupported;
+  if (!k->pool) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.handleTypes = cudaMemHandleTypeNone;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = device;
     cudaMemPool_t made = nullptr;
-    cudaError_t e = cudaMemPoolCreate(&made, &props);
-    if (e != cudaSuccess) return e;
+    if ((e = cudaMemPoolCreate(&made, &props)) != cudaSuccess) return e;
     uint64_t keep = kPoolKeep;
     if ((e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
       cudaMemPoolDestroy(made);
       return e;
     }
-    k.pool[device] = made;
+    k->pool = made;
   }
-  *pool = k.pool[device];
+  *pool = k->pool;
   return cudaSuccess;
 }
 }  // namespace
+
+cudaError_t current_context(unsigned long long* id) {
+  using GetId = CUresult (*)(CUcontext, unsigned long long*);
+  static const GetId get = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+    return reinterpret_cast<GetId>(p);
+  }();
+  if (!get) return cudaErrorNotSupported;
+  if (get(nullptr, id) == CUDA_SUCCESS) return cudaSuccess;
+  const cudaError_t e = cudaFree(nullptr);  // no context yet, or none any more: makes one
+  if (e != cudaSuccess) return e;
+  return get(nullptr, id) == CUDA_SUCCESS ? cudaSuccess : cudaErrorNotSupported;
+}
 
 cudaError_t device_alloc(void** p, size_t bytes, cudaStream_t s, bool* pooled) {
   if (pooled) *pooled = true;
@@ -119,11 +166,9 @@ cudaError_t device_alloc(void** p, size_t bytes, cudaStream_t s, bool* pooled) {
   cudaError_t e = cudaStreamIsCapturing(s, &capture);
   if (e != cudaSuccess) return e;
   if (capture != cudaStreamCaptureStatusNone) return cudaMallocAsync(p, bytes, s);
-  int device = 0;
-  if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;
-  if (bytes <= kPoolBlock && device < kPoolDevices) {
+  if (bytes <= kPoolBlock) {
     cudaMemPool_t pool = nullptr;
-    if ((e = pool_of(device, &pool)) == cudaSuccess) {
+    if ((e = pool_here(&pool)) == cudaSuccess) {
       if ((e = cudaMallocFromPoolAsync(p, bytes, pool, s)) == cudaSuccess) return e;
       cudaGetLastError();
       cudaMemPoolTrimTo(pool, 0);
@@ -134,33 +179,39 @@ cudaError_t device_alloc(void** p, size_t bytes, cudaStream_t s, bool* pooled) {
   return cudaMalloc(p, bytes);
 }
 
-void* pinned_slot_take() {
-  Kept& k = kept();
-  std::lock_guard<std::mutex> lock(k.mu);
-  if (!k.pinned_tried) {
-    k.pinned_tried = true;
-    void* q = nullptr;
-    if (cudaHostAlloc(&q, kPinnedSlots * kPinnedSlot, cudaHostAllocPortable) == cudaSuccess)
-      k.pinned = static_cast<unsigned char*>(q);
-    else
-      cudaGetLastError();
-  }
-  if (!k.pinned) return nullptr;
-  for (int i = 0; i < kPinnedSlots; ++i)
-    if (!(k.taken >> i & 1u)) {
-      k.taken |= 1u << i;
-      return k.pinned + i * kPinnedSlot;
+cudaError_t PinnedSlot::take() {
+  {
+    std::lock_guard<std::mutex> lock(g_kept_mutex);
+    if (Kept* k = kept_here()) {
+      if (!k->pinned_tried) {
+        k->pinned_tried = true;
+        void* q = nullptr;
+        if (cudaHostAlloc(&q, kPinnedSlots * kPinnedSlot, cudaHostAllocPortable) == cudaSuccess)
+          k->pinned = static_cast<unsigned char*>(q);
+        else
+          cudaGetLastError();
+      }
+      for (int i = 0; k->pinned && i < kPinnedSlots; ++i)
+        if (!(k->taken >> i & 1u)) {
+          k->taken |= 1u << i;
+          p = k->pinned + i * kPinnedSlot;
+          from = k;
+          return cudaSuccess;
+        }
     }
-  return nullptr;
+  }
+  return cudaMallocHost(&p, kPinnedSlot);
 }
 
-bool pinned_slot_return(void* p) {
-  Kept& k = kept();
-  std::lock_guard<std::mutex> lock(k.mu);
-  const unsigned char* q = static_cast<const unsigned char*>(p);
-  if (!k.pinned || q < k.pinned || q >= k.pinned + kPinnedSlots * kPinnedSlot) return false;
-  k.taken &= ~(1u << ((q - k.pinned) / kPinnedSlot));
-  return true;
+void PinnedSlot::release() {
+  if (from) {
+    std::lock_guard<std::mutex> lock(g_kept_mutex);
+    from->taken &= ~(1u << ((static_cast<unsigned char*>(p) - from->pinned) / kPinnedSlot));
+  } else if (p) {
+    cudaFreeHost(p);
+  }
+  p = nullptr;
+  from = nullptr;
 }
 }  // namespace pdot
 
@@ -528,9 +579,8 @@ class Solver {
     st_ = static_cast<pdot::DevState*>(alloc_bytes(sizeof(pdot::DevState)));
     ring_ = static_cast<pdot_iteration_stats*>(alloc_bytes(sizeof(pdot_iteration_stats) * kRingCap));
     static_assert(sizeof(pdot::DevState) * kInFlight <= pdot::kPinnedSlot, "the status records fit a slot");
-    void* hp = pdot::pinned_slot_take();
-    if (!hp) CK(cudaMallocHost(&hp, sizeof(pdot::DevState) * kInFlight));
-    host_status_ = static_cast<pdot::DevState*>(hp);
+    CK(status_slot_.take());
+    host_status_ = static_cast<pdot::DevState*>(status_slot_.p);
     for (int k = 0; k < kInFlight; ++k) CK(cudaEventCreateWithFlags(&ev_[k], cudaEventDisableTiming));
 
     B_.cost = cost_;
@@ -610,7 +660,7 @@ class Solver {
       cudaEventDestroy(t.start);
       cudaEventDestroy(t.stop);
     }
-    if (host_status_ && !pdot::pinned_slot_return(host_status_)) cudaFreeHost(host_status_);
+    status_slot_.release();
     for (void* p : allocs_) cudaFree(p);
     if (stream_) cudaStreamDestroy(stream_);
   }
@@ -1028,6 +1078,7 @@ class Solver {
   double* work_ = nullptr;
   pdot::DevState* st_ = nullptr;
   pdot_iteration_stats* ring_ = nullptr;
+  pdot::PinnedSlot status_slot_;
   pdot::DevState* host_status_ = nullptr;
   pdot::DevState status_{};
   std::vector<pdot_iteration_stats> records_;

@@ -10,8 +10,9 @@
 // core's memcpy rate (and the first-touch page faults of a fresh output array
 // are spread over the threads).
 //
-// The two 64 MiB staging buffers are allocated once per process on first use
-// and kept; a mutex serialises the staged copies of concurrent solves.
+// The two 64 MiB staging buffers are allocated once per process on first use and
+// kept, until the context that they were allocated in is gone (cudaDeviceReset); a
+// mutex serialises the staged copies of concurrent solves.
 #include <algorithm>
 #include <cstring>
 #include <mutex>
@@ -26,7 +27,9 @@ namespace {
 constexpr size_t kStageBytes = kTransferChunk * sizeof(double);
 constexpr size_t kDirectBelow = size_t(16) << 20;  // smaller copies go by one cudaMemcpy
 std::mutex g_stage_mutex;
-void* g_stage[2] = {nullptr, nullptr};
+unsigned char* g_stage[2] = {nullptr, nullptr};  // two halves of one block
+int g_stage_device = -1;                         // where it was allocated
+unsigned long long g_stage_context = 0;
 
 int copy_workers() {
   const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
@@ -50,15 +53,23 @@ void parallel_memcpy(void* dst, const void* src, size_t bytes, int workers) {
   for (std::thread& t : threads) t.join();
 }
 
+// Where the block was allocated, the context's id tells whether it is still there; on
+// another device, whether it is still page-locked.
 cudaError_t ensure_stage() {
-  for (int k = 0; k < 2; ++k) {
-    if (g_stage[k]) continue;
-    const cudaError_t e = cudaMallocHost(&g_stage[k], kStageBytes);
-    if (e != cudaSuccess) {
-      g_stage[k] = nullptr;
-      return e;
-    }
-  }
+  int device = 0;
+  unsigned long long context = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  if (current_context(&context) != cudaSuccess) cudaGetLastError();  // the id stays 0
+  if (g_stage[0] && (device == g_stage_device ? context == g_stage_context : host_is_pinned(g_stage[0])))
+    return cudaSuccess;
+  void* p = nullptr;
+  g_stage[0] = g_stage[1] = nullptr;
+  if ((e = cudaMallocHost(&p, 2 * kStageBytes)) != cudaSuccess) return e;
+  g_stage[0] = static_cast<unsigned char*>(p);
+  g_stage[1] = g_stage[0] + kStageBytes;
+  g_stage_device = device;
+  g_stage_context = context;
   return cudaSuccess;
 }
 
