@@ -153,7 +153,9 @@ __global__ void __launch_bounds__(kMaxThreads) k_max_sqdist(int64_t m, int64_t n
 // difference by a rounding each; 16 covers D <= 3). A pair whose FP32 value exceeds
 // min(best so far, tile's FP32 minimum + E) + E cannot be the minimum: only the groups
 // whose minima are within that are taken up again, at most two, or the whole tile where
-// a third one is. Where a bound is not finite no pair is left out.
+// a third one is. No pair is left out where a bound is not finite, where a distance may
+// exceed FP32 (the screen's infinity is then a finite value times a small scale), or
+// where the scale is below the normal FP32 numbers and errs by more than a rounding.
 template <int D>
 __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kMinThreads)
     k_c_transform(int64_t np, int64_t nc, const float* __restrict__ pts, const double* __restrict__ centres,
@@ -183,6 +185,7 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kMinThreads)
   }
   const float sc = (float)scale;
   const unsigned long long sc2 = pack2(sc, sc);
+  const bool screened = scale == 0.0 || (fabsf(sc) >= FLT_MIN && fabsf(sc) < INFINITY);
   const int64_t share = (nc + kSplit - 1) / kSplit;
   const int64_t jb = (int64_t)blockIdx.y * share, je = (jb + share < nc) ? jb + share : nc;
   for (int64_t j0 = jb; j0 < je; j0 += kTile) {
@@ -268,7 +271,7 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kMinThreads)
                       fabsf(sc) * 1e-38f + 1e-30f;
       const float have = __double2float_ru(best[q]);
       const float lim = (low[q] + E < have ? low[q] + E : have) + E;
-      const bool all = !(E < INFINITY) || !(fabsf(sc) < INFINITY) || !(fabsf(lim) < INFINITY);
+      const bool all = !screened || !(E < INFINITY) || !(2.0f * (float)D * A * A < INFINITY) || !(fabsf(lim) < INFINITY);
       auto take = [&](int t) {
         double s = 0.0;
 #pragma unroll

@@ -1,0 +1,64 @@
+"""The passes over point pairs that screen in FP32, where FP32 itself gives out: coordinates
+whose squared distances exceed it or fall below its normal numbers, and scales outside
+its range. The FP64 values decide, bit for bit (sums of squares in the order of the
+dimensions, rounded after every operation)."""
+import pytest
+
+from pdot import _abi
+
+pytestmark = pytest.mark.gpu
+
+# magnitude of the coordinates, and the scale that brings a squared distance to about one
+MAGNITUDES = [(1.0, 1.0), (1e18, 1e-36), (1e19, 1e-38), (3e19, 1e-39), (1e20, 1e-40), (3e22, 1e-45), (1e25, 1e-50),
+              (1e37, 1e-74), (1e-10, 1e20), (1e-19, 1e38), (1e-22, 1e44), (1e-30, 1e60)]
+
+
+def _points(torch, count, dim, magnitude, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.rand(count, dim, generator=g, device="cuda", dtype=torch.float64) * magnitude
+    return x.float()
+
+
+def _sqdist(torch, x, y):
+    d = torch.zeros(x.shape[0], y.shape[0], device="cuda", dtype=torch.float64)
+    for k in range(x.shape[1]):
+        e = x[:, k].double()[:, None] - y[:, k].double()[None, :]
+        d += e * e
+    return d
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3])
+@pytest.mark.parametrize("magnitude,scale", MAGNITUDES)
+def test_c_transform_at_the_ends_of_fp32(cuda, magnitude, scale, dim):
+    import torch
+
+    lib = _abi.load()
+    n, centres = 700, 3001
+    p = _points(torch, n, dim, magnitude, 1)
+    c = _points(torch, centres, dim, magnitude, 2).double()
+    v = torch.randn(centres, device="cuda", dtype=torch.float64, generator=torch.Generator(device="cuda").manual_seed(3))
+    for s, dual in ((scale, 1.0), (scale, 0.01), (-scale, 1.0), (0.0, 1.0)):
+        out = torch.empty(n, device="cuda", dtype=torch.float64)
+        w = v * dual
+        rc = lib.pdot_points_c_transform(n, centres, dim, p.data_ptr(), c.data_ptr(), w.data_ptr(), s, out.data_ptr(), None)
+        _abi.check(lib, rc, "pdot_points_c_transform")
+        want = (s * _sqdist(torch, p, c) - w[None, :]).min(1).values
+        assert torch.equal(out, want), (s, dual)
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3])
+@pytest.mark.parametrize("magnitude", [m for m, _ in MAGNITUDES])
+def test_largest_distance_at_the_ends_of_fp32(cuda, magnitude, dim):
+    import torch
+
+    lib = _abi.load()
+    m, n = 2300, 2100  # above the size from which the cost builder screens
+    x, y = _points(torch, m, dim, magnitude, 4), _points(torch, n, dim, magnitude, 5)
+    want = _sqdist(torch, x, y).max()
+    out = torch.empty(1, device="cuda", dtype=torch.float64)
+    _abi.check(lib, lib.pdot_points_max_sqdist(m, n, dim, x.data_ptr(), y.data_ptr(), out.data_ptr(), None), "max")
+    assert torch.equal(out[0], want)
+    x64, y64 = x.double(), y.double()
+    cost = torch.empty(n, m, device="cuda", dtype=torch.float64)  # column-major m x n
+    _abi.check(lib, lib.pdot_sqeuclid_cost_f64(m, n, dim, x64.data_ptr(), y64.data_ptr(), 1, cost.data_ptr(), None), "cost")
+    assert torch.equal(cost.T, _sqdist(torch, x, y) / want)
