@@ -150,7 +150,11 @@ __global__ void __launch_bounds__(kMaxThreads) k_max_sqdist(int64_t m, int64_t n
 //   E = 16 * 2^-24 * (2 |scale| D A^2 + V),  A = |p|_max + |c|_max,  V = |dual|_max
 // of the FP64 one over a tile (each coordinate difference is at most A and errs by at
 // most 2 * 2^-24 A, a square by 5 * 2^-24 A^2, their sum, the product and the
-// difference by a rounding each; 16 covers D <= 3). A pair whose FP32 value exceeds
+// difference by a rounding each; 16 covers D <= 3). The screen's coordinates are taken
+// relative to the first centre, so that A is the extent of the points and not their
+// distance from the origin: for points of a unit square at (1000, 1000) E would let most
+// pairs through (3000 centres, 5000 points: 109 us, 19 this way, 82 in FP64
+// throughout). A pair whose FP32 value exceeds
 // min(best so far, tile's FP32 minimum + E) + E cannot be the minimum: only the groups
 // whose minima are within that are taken up again, at most two, or the whole tile where
 // a third one is. No pair is left out where a bound is not finite, where a distance may
@@ -168,8 +172,10 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kMinThreads)
   __shared__ double part[kMinThreads * kPointsPer];
   float p[kPointsPer][D], reach[kPointsPer];
   unsigned long long minus[kPointsPer][D];
-  double best[kPointsPer];
+  double best[kPointsPer], origin[D];
   bool ok[kPointsPer];
+#pragma unroll
+  for (int d = 0; d < D; ++d) origin[d] = fabs(centres[d]) < INFINITY ? centres[d] : 0.0;
 #pragma unroll
   for (int q = 0; q < kPointsPer; ++q) {
     const int64_t i = ((int64_t)blockIdx.x * kPointsPer + q) * kMinThreads + threadIdx.x;
@@ -179,8 +185,9 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kMinThreads)
 #pragma unroll
     for (int d = 0; d < D; ++d) {
       p[q][d] = ok[q] ? pts[i * D + d] : 0.0f;
-      reach[q] = fmaxf(reach[q], fabsf(p[q][d]));
-      minus[q][d] = pack2(-p[q][d], -p[q][d]);
+      const float f = ok[q] ? (float)((double)p[q][d] - origin[d]) : 0.0f;
+      reach[q] = fmaxf(reach[q], fabsf(f));
+      minus[q][d] = pack2(-f, -f);
     }
   }
   const float sc = (float)scale;
@@ -197,7 +204,10 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kMinThreads)
     bool odd = false;  // a value that FP32 cannot hold or that is not a number
     for (int t = threadIdx.x; t < cnt * D; t += kMinThreads) {
       const double c = centres[j0 * D + t];
-      const float f = (float)c;
+      double o = origin[0];
+#pragma unroll
+      for (int d = 1; d < D; ++d) o = t % D == d ? origin[d] : o;
+      const float f = (float)(c - o);
       tc[t] = c;
       fc[t % D][t / D] = f;
       mc = fmaxf(mc, fabsf(f));
@@ -289,7 +299,7 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kMinThreads)
               float s = 0.0f;
 #pragma unroll
               for (int d = 0; d < D; ++d) {
-                const float e = p[q][d] - fc[d][t];
+                const float e = fc[d][t] + unpack_low(minus[q][d]);
                 s = d == 0 ? e * e : __fmaf_rn(e, e, s);
               }
               if (__fmaf_rn(sc, s, fv[t]) > lim) continue;

@@ -18,6 +18,7 @@ __device__ __forceinline__ unsigned long long pack2(float a, float b) {
 __device__ __forceinline__ void unpack2(unsigned long long r, float& a, float& b) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
 }
+__device__ __forceinline__ float unpack_low(unsigned long long r) { return __uint_as_float((unsigned)r); }
 __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
   unsigned long long r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));

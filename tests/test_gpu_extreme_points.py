@@ -62,3 +62,26 @@ def test_largest_distance_at_the_ends_of_fp32(cuda, magnitude, dim):
     cost = torch.empty(n, m, device="cuda", dtype=torch.float64)  # column-major m x n
     _abi.check(lib, lib.pdot_sqeuclid_cost_f64(m, n, dim, x64.data_ptr(), y64.data_ptr(), 1, cost.data_ptr(), None), "cost")
     assert torch.equal(cost.T, _sqdist(torch, x, y) / want)
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3])
+@pytest.mark.parametrize("shift", [0.5, 1e3, 1e6])
+def test_c_transform_of_points_far_from_the_origin(cuda, shift, dim):
+    """Points of a unit cube at a distance, whose coordinates FP32 holds to fewer digits."""
+    import torch
+
+    lib = _abi.load()
+    n, centres = 1000, 2000
+    p = (_points(torch, n, dim, 1.0, 6).double() + shift).float()
+    c = _points(torch, centres, dim, 1.0, 7).double() + shift
+    v = torch.randn(centres, device="cuda", dtype=torch.float64, generator=torch.Generator(device="cuda").manual_seed(8))
+    for dual in (0.0, 0.1):
+        out = torch.empty(n, device="cuda", dtype=torch.float64)
+        w = v * dual
+        rc = lib.pdot_points_c_transform(n, centres, dim, p.data_ptr(), c.data_ptr(), w.data_ptr(), 1.0, out.data_ptr(), None)
+        _abi.check(lib, rc, "pdot_points_c_transform")
+        d = torch.zeros(n, centres, device="cuda", dtype=torch.float64)
+        for k in range(dim):
+            e = p[:, k].double()[:, None] - c[None, :, k]
+            d += e * e
+        assert torch.equal(out, (d - w[None, :]).min(1).values)
