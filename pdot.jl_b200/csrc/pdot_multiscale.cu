@@ -337,6 +337,110 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kMinThreads)
   cluster.sync();  // no CTA leaves while its shared memory is read
 }
 
+// Both in FP64 throughout, a point of the first set a thread, for a second set of few
+// points: there is little to split over CTAs and a screen has no best value to measure a
+// tile against, so that its passes and barriers only come on top. On B200, this and the
+// screened form, 5000 points: the c-transform in the plane 4.1 and 6.2 us for 32 centres,
+// 6.2 and 8.2 for 128, 10.3 and 8.2 for 256, on the line, where a distance is two
+// operations less, 6.3 and 8.4 for 189; the maximum in the plane 5.2 and 5.7 us for one
+// point, 8.2 and 8.3 for 128, 10.3 and 8.5 for 256, on the line 6.2 and 8.2 for 128, 8.2
+// and 8.2 for 256.
+__host__ __device__ constexpr int few_centres(int dim) { return dim == 1 ? 192 : 128; }
+__host__ __device__ constexpr int few_far(int dim) { return dim == 1 ? 256 : 160; }
+constexpr int kFewThreads = 256;
+template <int D>
+__global__ void __launch_bounds__(kFewThreads) k_max_sqdist_few(int64_t m, int64_t n, const float* __restrict__ xs,
+                                                                const float* __restrict__ ys,
+                                                                unsigned long long* __restrict__ out_bits) {
+  __shared__ float ty[few_far(D) * D];
+  __shared__ double red[kFewThreads / 32];
+  const int64_t i = (int64_t)blockIdx.x * kFewThreads + threadIdx.x;
+  double x[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) x[d] = i < m ? (double)xs[i * D + d] : 0.0;
+  double best = 0.0;
+  for (int t = threadIdx.x; t < n * D; t += kFewThreads) ty[t] = ys[t];
+  __syncthreads();
+  if (i < m)
+    for (int t = 0; t < n; ++t) {
+      double s = 0.0;
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        const double e = x[d] - (double)ty[t * D + d];
+        s += e * e;
+      }
+      best = s > best ? s : best;
+    }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double y = __shfl_xor_sync(0xffffffffu, best, o);
+    best = y > best ? y : best;
+  }
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double b = red[0];
+    for (int w = 1; w < kFewThreads / 32; ++w) b = red[w] > b ? red[w] : b;
+    atomicMax(out_bits, (unsigned long long)__double_as_longlong(b));
+  }
+}
+
+template <int D>
+__global__ void __launch_bounds__(kFewThreads)
+    k_c_transform_few(int64_t np, int64_t nc, const float* __restrict__ pts, const double* __restrict__ centres,
+                      const double* __restrict__ duals, double scale, double* __restrict__ out) {
+  __shared__ double tc[few_centres(D) * D];
+  __shared__ double tv[few_centres(D)];
+  const int64_t i = (int64_t)blockIdx.x * kFewThreads + threadIdx.x;
+  double p[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) p[d] = i < np ? (double)pts[i * D + d] : 0.0;
+  double best = INFINITY;
+  for (int t = threadIdx.x; t < nc * D; t += kFewThreads) tc[t] = centres[t];
+  for (int t = threadIdx.x; t < nc; t += kFewThreads) tv[t] = duals[t];
+  __syncthreads();
+  if (i < np)
+    for (int t = 0; t < nc; ++t) {
+      double s = 0.0;
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        const double e = p[d] - tc[t * D + d];
+        s += e * e;
+      }
+      const double val = scale * s - tv[t];
+      best = val < best ? val : best;
+    }
+  if (i < np) out[i] = best;
+}
+
+template <int D>
+void max_sqdist(int64_t m, int64_t n, const float* xs, const float* ys, unsigned long long* bits, cudaStream_t s) {
+  if (n <= few_far(D)) {
+    k_max_sqdist_few<D><<<(unsigned)((m + kFewThreads - 1) / kFewThreads), kFewThreads, 0, s>>>(m, n, xs, ys, bits);
+    return;
+  }
+  const int64_t blocks = (m + kMaxThreads * kPointsPer - 1) / (kMaxThreads * kPointsPer);
+  // the second set in shares of whole tiles, some 16 CTAs per SM
+  const int64_t tiles = (n + kFarTile - 1) / kFarTile;
+  int64_t shares = (148 * 16 + blocks - 1) / blocks;
+  shares = shares < tiles ? shares : tiles;
+  const int64_t share = (tiles + shares - 1) / shares * kFarTile;
+  const dim3 grid((unsigned)blocks, (unsigned)((n + share - 1) / share));
+  k_max_sqdist<D><<<grid, kMaxThreads, 0, s>>>(m, n, share, xs, ys, bits);
+}
+
+template <int D>
+void c_transform(int64_t np, int64_t nc, const float* pts, const double* centres, const double* duals, double scale,
+                 double* out, cudaStream_t s) {
+  if (nc <= few_centres(D)) {
+    k_c_transform_few<D><<<(unsigned)((np + kFewThreads - 1) / kFewThreads), kFewThreads, 0, s>>>(
+        np, nc, pts, centres, duals, scale, out);
+    return;
+  }
+  const dim3 grid((unsigned)((np + kMinThreads * kPointsPer - 1) / (kMinThreads * kPointsPer)), kSplit);
+  k_c_transform<D><<<grid, kMinThreads, 0, s>>>(np, nc, pts, centres, duals, scale, out);
+}
+
 int report(int code, const char* msg) {
   set_last_error(msg);
   return code;
@@ -355,20 +459,13 @@ extern "C" int pdot_points_max_sqdist(int64_t m, int64_t n, int32_t dim, const f
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaMemsetAsync(out, 0, sizeof(double), s);
   if (e != cudaSuccess) return report(PDOT_ERR_CUDA, cudaGetErrorString(e));
-  const int64_t blocks = (m + kMaxThreads * kPointsPer - 1) / (kMaxThreads * kPointsPer);
-  // the second set in shares of whole tiles, some 16 CTAs per SM
-  const int64_t tiles = (n + kFarTile - 1) / kFarTile;
-  int64_t shares = (148 * 16 + blocks - 1) / blocks;
-  shares = shares < tiles ? shares : tiles;
-  const int64_t share = (tiles + shares - 1) / shares * kFarTile;
-  const dim3 grid((unsigned)blocks, (unsigned)((n + share - 1) / share));
   auto* bits = reinterpret_cast<unsigned long long*>(out);
   if (dim == 1)
-    k_max_sqdist<1><<<grid, kMaxThreads, 0, s>>>(m, n, share, source_points, target_points, bits);
+    max_sqdist<1>(m, n, source_points, target_points, bits, s);
   else if (dim == 2)
-    k_max_sqdist<2><<<grid, kMaxThreads, 0, s>>>(m, n, share, source_points, target_points, bits);
+    max_sqdist<2>(m, n, source_points, target_points, bits, s);
   else
-    k_max_sqdist<3><<<grid, kMaxThreads, 0, s>>>(m, n, share, source_points, target_points, bits);
+    max_sqdist<3>(m, n, source_points, target_points, bits, s);
   e = cudaGetLastError();
   if (e != cudaSuccess) return report(PDOT_ERR_CUDA, cudaGetErrorString(e));
   return PDOT_OK;
@@ -384,13 +481,12 @@ extern "C" int pdot_points_c_transform(int64_t num_points, int64_t num_centres, 
   if (!points || !centres || !duals || !out) return report(PDOT_ERR_INVALID_ARGUMENT, "null pointer argument");
   if (!std::isfinite(scale)) return report(PDOT_ERR_INVALID_ARGUMENT, "scale must be finite");
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const dim3 blocks((unsigned)((num_points + kMinThreads * kPointsPer - 1) / (kMinThreads * kPointsPer)), kSplit);
   if (dim == 1)
-    k_c_transform<1><<<blocks, kMinThreads, 0, s>>>(num_points, num_centres, points, centres, duals, scale, out);
+    c_transform<1>(num_points, num_centres, points, centres, duals, scale, out, s);
   else if (dim == 2)
-    k_c_transform<2><<<blocks, kMinThreads, 0, s>>>(num_points, num_centres, points, centres, duals, scale, out);
+    c_transform<2>(num_points, num_centres, points, centres, duals, scale, out, s);
   else
-    k_c_transform<3><<<blocks, kMinThreads, 0, s>>>(num_points, num_centres, points, centres, duals, scale, out);
+    c_transform<3>(num_points, num_centres, points, centres, duals, scale, out, s);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return report(PDOT_ERR_CUDA, cudaGetErrorString(e));
   return PDOT_OK;

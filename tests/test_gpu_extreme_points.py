@@ -85,3 +85,24 @@ def test_c_transform_of_points_far_from_the_origin(cuda, shift, dim):
             e = p[:, k].double()[:, None] - c[None, :, k]
             d += e * e
         assert torch.equal(out, (d - w[None, :]).min(1).values)
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3])
+@pytest.mark.parametrize("second", [1, 31, 128, 129, 160, 161, 192, 193, 256, 257])
+def test_pair_passes_over_few_points(cuda, second, dim):
+    """Both sides of the size up to which the second set is one tile in FP64."""
+    import torch
+
+    lib = _abi.load()
+    for first in (1, 255, 257, 3000):
+        x, y = _points(torch, first, dim, 1.0, 9), _points(torch, second, dim, 1.0, 10)
+        d = _sqdist(torch, x, y)
+        top = torch.empty(1, device="cuda", dtype=torch.float64)
+        _abi.check(lib, lib.pdot_points_max_sqdist(first, second, dim, x.data_ptr(), y.data_ptr(), top.data_ptr(), None), "max")
+        assert torch.equal(top[0], d.max())
+        c = y.double()
+        v = torch.randn(second, device="cuda", dtype=torch.float64, generator=torch.Generator(device="cuda").manual_seed(11))
+        out = torch.empty(first, device="cuda", dtype=torch.float64)
+        rc = lib.pdot_points_c_transform(first, second, dim, x.data_ptr(), c.data_ptr(), v.data_ptr(), 1.5, out.data_ptr(), None)
+        _abi.check(lib, rc, "pdot_points_c_transform")
+        assert torch.equal(out, (1.5 * d - v[None, :]).min(1).values)
