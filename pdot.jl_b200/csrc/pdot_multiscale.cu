@@ -146,20 +146,26 @@ __global__ void __launch_bounds__(kMaxThreads) k_max_sqdist(int64_t m, int64_t n
 // equal shares; the cluster's first CTA reads the others' minima from their shared
 // memory.
 //
-// The FP32 value of a pair (centre, dual and scale rounded to FP32) is within
-//   E = 16 * 2^-24 * (2 |scale| D A^2 + V),  A = |p|_max + |c|_max,  V = |dual|_max
-// of the FP64 one over a tile (each coordinate difference is at most A and errs by at
-// most 2 * 2^-24 A, a square by 5 * 2^-24 A^2, their sum, the product and the
-// difference by a rounding each; 16 covers D <= 3). The screen's coordinates are taken
-// relative to the first centre, so that A is the extent of the points and not their
-// distance from the origin: for points of a unit square at (1000, 1000) E would let most
-// pairs through (3000 centres, 5000 points: 109 us, 19 this way, 82 in FP64
-// throughout). A pair whose FP32 value exceeds
-// min(best so far, tile's FP32 minimum + E) + E cannot be the minimum: only the groups
-// whose minima are within that are taken up again, at most two, or the whole tile where
-// a third one is. No pair is left out where a bound is not finite, where a distance may
-// exceed FP32 (the screen's infinity is then a finite value times a small scale), or
-// where the scale is below the normal FP32 numbers and errs by more than a rounding.
+// What FP32 makes of a pair (centre, dual and scale rounded to it): with u = 2^-24 and A =
+// |p|_max + |c|_max over the tile, a coordinate difference errs by at most 2 u A, the
+// squared distance s by 4 u A sqrt(D s) + 4 D u^2 A^2 + 4 u s, the value scale s - v by
+// |scale| times that, another 2 u |scale| s and u (|v| + |value|). Where the scale is
+// positive a pair whose value is at most x has scale s <= x + V, V = |dual|_max, so that
+// error(x) below, twice the sum and more, holds for every pair that counts; it is some
+// twenty times less than with the largest distance for s, which let through many more
+// pairs on the line (20000 points and 6000 centres with the duals 0.3 c^2 + 0.1 c: 141 us
+// then, 131 now, 121 in FP64 throughout; with duals of 1e-3 51, 41 and 121). A pair whose FP32 value exceeds
+// M + error(M), M = min(best so far, tile's FP32 minimum + its error), cannot be the
+// minimum: only the groups whose minima are within that are taken up again, at most two,
+// or the whole tile where a third one is.
+//
+// The screen's coordinates are taken relative to the first centre, so that A is the
+// extent of the points and not their distance from the origin: for points of a unit
+// square at (1000, 1000) the error would let most pairs through (3000 centres, 5000
+// points: 109 us, 19 this way, 82 in FP64 throughout). No pair is left out where a bound
+// is not finite, where a distance may exceed FP32 (the screen's infinity is then a finite
+// value times a small scale), or where the scale is below the normal FP32 numbers and
+// errs by more than a rounding.
 template <int D>
 __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kMinThreads)
     k_c_transform(int64_t np, int64_t nc, const float* __restrict__ pts, const double* __restrict__ centres,
@@ -276,12 +282,19 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kMinThreads)
     }
 #pragma unroll
     for (int q = 0; q < kPointsPer; ++q) {
-      const float A = reach[q] + __int_as_float(bound_c);
-      const float E = 16.0f * kUnit * (2.0f * fabsf(sc) * (float)D * A * A + __int_as_float(bound_v)) +
-                      fabsf(sc) * 1e-38f + 1e-30f;
+      const float A = reach[q] + __int_as_float(bound_c), V = __int_as_float(bound_v);
+      const float far = 2.0f * (float)D * A * A;  // no squared distance is larger
+      const float least = fabsf(sc) * (64.0f * kUnit * kUnit * far + 1e-38f) + 1e-30f;
+      // the error of a pair whose value is at most x
+      auto error = [&](float x) {
+        const float t = sc < 0.0f ? fabsf(sc) * far : fminf(fmaxf(x + V, 0.0f), sc * far);
+        return kUnit * (8.0f * A * sqrtf((float)D * fabsf(sc) * t) + 16.0f * t + 4.0f * (V + fabsf(x))) + least;
+      };
       const float have = __double2float_ru(best[q]);
-      const float lim = (low[q] + E < have ? low[q] + E : have) + E;
-      const bool all = !screened || !(E < INFINITY) || !(2.0f * (float)D * A * A < INFINITY) || !(fabsf(lim) < INFINITY);
+      float lim = low[q] + error(low[q]);
+      lim = lim < have ? lim : have;
+      lim += error(lim);
+      const bool all = !screened || !(far < INFINITY) || !(fabsf(lim) < INFINITY);
       auto take = [&](int t) {
         double s = 0.0;
 #pragma unroll
@@ -342,17 +355,16 @@ __global__ void __cluster_dims__(1, kSplit, 1) __launch_bounds__(kMinThreads)
 // tile against, so that its passes and barriers only come on top. On B200, this and the
 // screened form, 5000 points: the c-transform in the plane 4.1 and 6.2 us for 32 centres,
 // 6.2 and 8.2 for 128, 10.3 and 8.2 for 256, on the line, where a distance is two
-// operations less, 6.3 and 8.4 for 189; the maximum in the plane 5.2 and 5.7 us for one
+// operations less, 6.3 and 8.4 for 189, 8.2 and 8.3 for 256; the maximum in the plane 5.2 and 5.7 us for one
 // point, 8.2 and 8.3 for 128, 10.3 and 8.5 for 256, on the line 6.2 and 8.2 for 128, 8.2
 // and 8.2 for 256.
-__host__ __device__ constexpr int few_centres(int dim) { return dim == 1 ? 192 : 128; }
-__host__ __device__ constexpr int few_far(int dim) { return dim == 1 ? 256 : 160; }
+__host__ __device__ constexpr int few_points(int dim) { return dim == 1 ? 256 : 160; }
 constexpr int kFewThreads = 256;
 template <int D>
 __global__ void __launch_bounds__(kFewThreads) k_max_sqdist_few(int64_t m, int64_t n, const float* __restrict__ xs,
                                                                 const float* __restrict__ ys,
                                                                 unsigned long long* __restrict__ out_bits) {
-  __shared__ float ty[few_far(D) * D];
+  __shared__ float ty[few_points(D) * D];
   __shared__ double red[kFewThreads / 32];
   const int64_t i = (int64_t)blockIdx.x * kFewThreads + threadIdx.x;
   double x[D];
@@ -389,8 +401,8 @@ template <int D>
 __global__ void __launch_bounds__(kFewThreads)
     k_c_transform_few(int64_t np, int64_t nc, const float* __restrict__ pts, const double* __restrict__ centres,
                       const double* __restrict__ duals, double scale, double* __restrict__ out) {
-  __shared__ double tc[few_centres(D) * D];
-  __shared__ double tv[few_centres(D)];
+  __shared__ double tc[few_points(D) * D];
+  __shared__ double tv[few_points(D)];
   const int64_t i = (int64_t)blockIdx.x * kFewThreads + threadIdx.x;
   double p[D];
 #pragma unroll
@@ -415,7 +427,7 @@ __global__ void __launch_bounds__(kFewThreads)
 
 template <int D>
 void max_sqdist(int64_t m, int64_t n, const float* xs, const float* ys, unsigned long long* bits, cudaStream_t s) {
-  if (n <= few_far(D)) {
+  if (n <= few_points(D)) {
     k_max_sqdist_few<D><<<(unsigned)((m + kFewThreads - 1) / kFewThreads), kFewThreads, 0, s>>>(m, n, xs, ys, bits);
     return;
   }
@@ -432,7 +444,7 @@ void max_sqdist(int64_t m, int64_t n, const float* xs, const float* ys, unsigned
 template <int D>
 void c_transform(int64_t np, int64_t nc, const float* pts, const double* centres, const double* duals, double scale,
                  double* out, cudaStream_t s) {
-  if (nc <= few_centres(D)) {
+  if (nc <= few_points(D)) {
     k_c_transform_few<D><<<(unsigned)((np + kFewThreads - 1) / kFewThreads), kFewThreads, 0, s>>>(
         np, nc, pts, centres, duals, scale, out);
     return;

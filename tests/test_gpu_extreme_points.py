@@ -106,3 +106,36 @@ def test_pair_passes_over_few_points(cuda, second, dim):
         rc = lib.pdot_points_c_transform(first, second, dim, x.data_ptr(), c.data_ptr(), v.data_ptr(), 1.5, out.data_ptr(), None)
         _abi.check(lib, rc, "pdot_points_c_transform")
         assert torch.equal(out, (1.5 * d - v[None, :]).min(1).values)
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3])
+@pytest.mark.parametrize("kind", ["zero", "smooth", "flat", "own", "twins"])
+def test_c_transform_where_many_centres_nearly_tie(cuda, kind, dim):
+    """Duals under which centres differ by less than FP32 tells apart: none, a smooth potential, one that
+    makes every centre as good as the next, centres that are the points, and centres that coincide."""
+    import torch
+
+    lib = _abi.load()
+    n, centres = 1500, 2500
+    p = _points(torch, n, dim, 1.0, 12)
+    c = _points(torch, centres, dim, 1.0, 13).double()
+    v = torch.zeros(centres, device="cuda", dtype=torch.float64)
+    if kind == "smooth":
+        v = 0.3 * (c * c).sum(1) + 0.1 * c[:, 0]
+    elif kind == "flat":  # |x - c|^2 - |c|^2 hardly depends on c for points near the origin
+        v = (c * c).sum(1)
+        p = p * 1e-6
+    elif kind == "own":
+        c[:n] = p.double()
+    elif kind == "twins":
+        c[1000:] = c[torch.arange(1000, centres, device="cuda") % 7]
+    for scale in (1.0, 0.37, -1.0):
+        w = scale * v
+        out = torch.empty(n, device="cuda", dtype=torch.float64)
+        rc = lib.pdot_points_c_transform(n, centres, dim, p.data_ptr(), c.data_ptr(), w.data_ptr(), scale, out.data_ptr(), None)
+        _abi.check(lib, rc, "pdot_points_c_transform")
+        d = torch.zeros(n, centres, device="cuda", dtype=torch.float64)
+        for k in range(dim):
+            e = p[:, k].double()[:, None] - c[None, :, k]
+            d += e * e
+        assert torch.equal(out, (scale * d - w[None, :]).min(1).values), scale
