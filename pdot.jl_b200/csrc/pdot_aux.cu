@@ -390,13 +390,14 @@ __global__ void __launch_bounds__(kAuxThreads)
 // The same in FP64 throughout: any dimension, and small problems, where the tiles' barriers
 // and second passes cost more than the arithmetic (500 x 500 in one dimension, whole cost:
 // 14.3 us against 17; 3000 x 2500 in two: 30.6 either way).
-constexpr int kSmallRows = 4;  // rows per thread: a column's coordinates serve four distances
+// rows per thread: a column's coordinates serve four distances where they are in registers
+__host__ __device__ constexpr int small_rows(int dim) { return dim > 0 ? 4 : 1; }
 constexpr int64_t kSmallPairs = int64_t(1) << 22;
 template <int DIM>
 __global__ void __launch_bounds__(kAuxThreads)
     k_sqeuclid_max_small(int64_t m, int64_t n, int dim, int64_t chunk, const double* __restrict__ xs,
                    const double* __restrict__ ys, unsigned long long* __restrict__ out) {
-  constexpr int Q = kSmallRows;
+  constexpr int Q = small_rows(DIM);
   constexpr int D = DIM > 0 ? DIM : 1;
   const int64_t i0 = (int64_t)blockIdx.x * kAuxThreads * Q + threadIdx.x;
   double x[Q][D], mx[Q];
@@ -446,34 +447,25 @@ __global__ void __launch_bounds__(kAuxThreads)
 // given and positive. Entry 0, where *top lies, is left to k_sqeuclid_first.
 template <int DIM, int R>
 __global__ void __launch_bounds__(kAuxThreads)
-    k_sqeuclid_write(int64_t m, int64_t n, int dim, int64_t chunk, const double* __restrict__ xs,
-                     const double* __restrict__ ys, const double* top, double* C) {
-  constexpr int D = DIM > 0 ? DIM : 1;
+    k_sqeuclid_write(int64_t m, int64_t n, int64_t chunk, const double* __restrict__ xs, const double* __restrict__ ys,
+                     const double* top, double* C) {
   const double mx = top ? *top : 0.0;
   const DivideBy by(mx);
   const int64_t i = ((int64_t)blockIdx.x * kAuxThreads + threadIdx.x) * R;
   if (i >= m) return;
-  double x[R][D];
-  if constexpr (DIM > 0) {
+  double x[R][DIM];
 #pragma unroll
-    for (int e = 0; e < R; ++e)
+  for (int e = 0; e < R; ++e)
 #pragma unroll
-      for (int d = 0; d < D; ++d) x[e][d] = xs[(i + e) * DIM + d];
-  }
+    for (int d = 0; d < DIM; ++d) x[e][d] = xs[(i + e) * DIM + d];
   const int64_t j0 = (int64_t)blockIdx.y * chunk, j1 = (j0 + chunk < n) ? j0 + chunk : n;
 #pragma unroll 2
   for (int64_t j = j0; j < j1; ++j) {
-    double v[R];
-    if constexpr (DIM > 0) {
-      double y[D];
+    double v[R], y[DIM];
 #pragma unroll
-      for (int d = 0; d < D; ++d) y[d] = __ldg(ys + j * DIM + d);
+    for (int d = 0; d < DIM; ++d) y[d] = __ldg(ys + j * DIM + d);
 #pragma unroll
-      for (int e = 0; e < R; ++e) v[e] = sq_distance<DIM>(x[e], y, dim);
-    } else {
-#pragma unroll
-      for (int e = 0; e < R; ++e) v[e] = sq_distance<0>(xs + (i + e) * dim, ys + j * dim, dim);
-    }
+    for (int e = 0; e < R; ++e) v[e] = sq_distance<DIM>(x[e], y, DIM);
     if (mx > 0.0) {
 #pragma unroll
       for (int e = 0; e < R; ++e) v[e] = by(v[e]);
@@ -483,6 +475,30 @@ __global__ void __launch_bounds__(kAuxThreads)
     } else {
       store_rows<R>(C + j * m + i, v);
     }
+  }
+}
+
+// The same an entry a thread, in the order of the matrix: for dimensions that are not
+// compiled in, whose coordinates come from memory for every entry either way; for fewer
+// than kEntryRows rows, which leave most lanes of the other form without one; and for few
+// entries, which leave it too few CTAs. On B200, this and the other form: 10000 x 10000
+// in six dimensions 548 and 742 us, 1000 x 3000 19 and 31; 8 x 10000 in the plane 4.1
+// and 6.2, 64 x 10000 6.2 either way; 954 x 165 in four dimensions 4.4 and 6.3.
+constexpr int kEntryRows = 64;
+constexpr int64_t kFewEntries = 160000;
+template <int DIM>
+__global__ void __launch_bounds__(kAuxThreads)
+    k_sqeuclid_entries(int64_t m, int64_t n, int dim, const double* __restrict__ xs, const double* __restrict__ ys,
+                       const double* top, double* C) {
+  const double mx = top ? *top : 0.0;
+  const DivideBy by(mx);
+  const int64_t N = m * n;
+  for (int64_t e = (int64_t)blockIdx.x * kAuxThreads + threadIdx.x; e < N; e += (int64_t)gridDim.x * kAuxThreads) {
+    const int64_t j = e / m, i = e - j * m;
+    const int D = DIM > 0 ? DIM : dim;
+    double v = sq_distance<DIM>(xs + i * D, ys + j * D, dim);
+    if (mx > 0.0) v = by(v);
+    if (!top || e != 0) C[e] = v;
   }
 }
 
@@ -591,8 +607,9 @@ cudaError_t sqeuclid_passes(int64_t m, int64_t n, int dim, const double* xs, con
     if (e != cudaSuccess) return e;
     auto* bits = reinterpret_cast<unsigned long long*>(top);
     if (DIM == 0 || m * n <= kSmallPairs) {
-      const int64_t strips = (m + kAuxThreads * kSmallRows - 1) / (kAuxThreads * kSmallRows);
-      const int64_t chunk = column_chunk(n, strips, 148 * 16, 16);
+      constexpr int Q = small_rows(DIM);
+      const int64_t strips = (m + kAuxThreads * Q - 1) / (kAuxThreads * Q);
+      const int64_t chunk = column_chunk(n, strips, 148 * 16, 4 * Q);
       k_sqeuclid_max_small<DIM>
           <<<dim3((unsigned)strips, (unsigned)((n + chunk - 1) / chunk)), kAuxThreads, 0, s>>>(m, n, dim, chunk, xs, ys, bits);
     } else if constexpr (DIM > 0) {
@@ -603,15 +620,20 @@ cudaError_t sqeuclid_passes(int64_t m, int64_t n, int dim, const double* xs, con
           m, n, share, xs, ys, bits);
     }
   }
-  const bool wide = m % kCostRows == 0 && (reinterpret_cast<uintptr_t>(C) & 15u) == 0;
-  const int R = wide ? kCostRows : 1;
-  const int64_t strips = (m + kAuxThreads * R - 1) / (kAuxThreads * R);
-  const int64_t chunk = column_chunk(n, strips, 148 * 32, 8);
-  const dim3 grid((unsigned)strips, (unsigned)((n + chunk - 1) / chunk));
-  if (wide)
-    k_sqeuclid_write<DIM, kCostRows><<<grid, kAuxThreads, 0, s>>>(m, n, dim, chunk, xs, ys, top, C);
-  else
-    k_sqeuclid_write<DIM, 1><<<grid, kAuxThreads, 0, s>>>(m, n, dim, chunk, xs, ys, top, C);
+  if (DIM == 0 || m < kEntryRows || m * n <= kFewEntries) {
+    const int64_t ctas = (m * n + kAuxThreads - 1) / kAuxThreads;
+    k_sqeuclid_entries<DIM><<<(unsigned)(ctas < 148 * 16 ? ctas : 148 * 16), kAuxThreads, 0, s>>>(m, n, dim, xs, ys, top, C);
+  } else if constexpr (DIM > 0) {
+    const bool wide = m % kCostRows == 0 && (reinterpret_cast<uintptr_t>(C) & 15u) == 0;
+    const int R = wide ? kCostRows : 1;
+    const int64_t strips = (m + kAuxThreads * R - 1) / (kAuxThreads * R);
+    const int64_t chunk = column_chunk(n, strips, 148 * 32, 8);
+    const dim3 grid((unsigned)strips, (unsigned)((n + chunk - 1) / chunk));
+    if (wide)
+      k_sqeuclid_write<DIM, kCostRows><<<grid, kAuxThreads, 0, s>>>(m, n, chunk, xs, ys, top, C);
+    else
+      k_sqeuclid_write<DIM, 1><<<grid, kAuxThreads, 0, s>>>(m, n, chunk, xs, ys, top, C);
+  }
   if (normalise) k_sqeuclid_first<<<1, 1, 0, s>>>(dim, xs, ys, C);
   return cudaGetLastError();
 }

@@ -139,3 +139,22 @@ def test_c_transform_where_many_centres_nearly_tie(cuda, kind, dim):
             e = p[:, k].double()[:, None] - c[None, :, k]
             d += e * e
         assert torch.equal(out, (scale * d - w[None, :]).min(1).values), scale
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3, 4, 5, 6, 9])
+@pytest.mark.parametrize("m,n", [(1, 1), (1, 4000), (3000, 1), (2, 300), (63, 500), (64, 500), (65, 33), (513, 260), (1000, 16),
+                                 (400, 400), (401, 400), (402, 400)])
+def test_cost_of_few_rows_and_of_more_dimensions(cuda, m, n, dim):
+    """Both sides of the number of rows up to which a thread takes an entry, and dimensions beyond those
+    that are compiled in; as given and normalised."""
+    import torch
+
+    lib = _abi.load()
+    x, y = _points(torch, m, dim, 1.0, 14).double(), _points(torch, n, dim, 1.0, 15).double()
+    d = _sqdist(torch, x, y)
+    for normalise in (0, 1):
+        cost = torch.full((n * m + 1,), 7.0, device="cuda", dtype=torch.float64)
+        rc = lib.pdot_sqeuclid_cost_f64(m, n, dim, x.data_ptr(), y.data_ptr(), normalise, cost.data_ptr(), None)
+        _abi.check(lib, rc, "pdot_sqeuclid_cost_f64")
+        assert torch.equal(cost[:-1].view(n, m).T, d / d.max() if normalise else d)
+        assert cost[-1] == 7.0
