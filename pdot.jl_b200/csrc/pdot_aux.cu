@@ -242,13 +242,9 @@ __device__ __forceinline__ double sq_distance(const double* xi, const double* yj
   return s;
 }
 
-// v / mx rounded to nearest for one divisor and many v. With y the correctly rounded
-// 1 / mx and q a quotient within one ulp, q + (v - q mx) y, its residual exact by one
-// fused multiply-add, is the correctly rounded quotient (Markstein, IBM J. Res. Dev.
-// 34, 1990). v y can be 1.5 ulp off, so a first such correction makes it a q within
-// one ulp and a second takes the theorem. The bounds on mx and v keep every term in
-// the normal range; everything else, 0 and the entries next to mx and NaNs among it,
-// takes the division itself. Five operations in place of a division an entry.
+// v / mx rounded to nearest for one divisor and many v >= 0 (quotient_of). The bounds on mx
+// and v keep every term in the normal range; everything else, 0 and the entries next to
+// mx and NaNs among it, takes the division itself.
 struct DivideBy {
   double mx, y;
   unsigned low, span;  // high words of the v that take the corrections: low ... low + span
@@ -260,9 +256,7 @@ struct DivideBy {
   }
   __device__ __forceinline__ double operator()(double v) const {
     if ((unsigned)__double2hiint(v) - low < span) {
-      double q = __dmul_rn(v, y);
-      q = __fma_rn(__fma_rn(-q, mx, v), y, q);
-      return __fma_rn(__fma_rn(-q, mx, v), y, q);
+      return quotient_of(v, mx, y);
     }
     return __ddiv_rn(v, mx);
   }

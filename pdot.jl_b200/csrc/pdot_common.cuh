@@ -100,6 +100,18 @@ __host__ __device__ __forceinline__ int64_t cta_of_unit(const Geometry& g, int64
 // the slot is unique. There are at most grid + panels slots.
 __host__ __device__ __forceinline__ int64_t row_slot(int64_t cta, int64_t panel) { return cta + panel; }
 
+// x / d rounded to nearest from y = 1 / d rounded to nearest, for one divisor and many x:
+// five operations in place of a division. With q a quotient within one ulp, q + (x - q d)
+// y, its residual exact by one fused multiply-add, is the correctly rounded quotient
+// (Markstein, IBM J. Res. Dev. 34, 1990). x y can be 1.5 ulp off, so a first such
+// correction makes it a q within one ulp and a second takes the theorem. The caller
+// keeps every term in the normal range.
+__device__ __forceinline__ double quotient_of(double x, double d, double y) {
+  double q = __dmul_rn(x, y);
+  q = __fma_rn(__fma_rn(-q, d, x), y, q);
+  return __fma_rn(__fma_rn(-q, d, x), y, q);
+}
+
 // Solver state in device memory. Every per-iteration decision is taken on the
 // device, so the host only reads this record between replayed chunks.
 struct DevState {

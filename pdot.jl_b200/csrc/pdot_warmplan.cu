@@ -196,10 +196,8 @@ __global__ void __launch_bounds__(kWpGroupThreads) k_wp_balance(WarmPlanArgs A, 
   });
 }
 
-// x / eps rounded to nearest, one divisor for many x: two Markstein corrections of
-// x y with y = 1 / eps rounded to nearest (IBM J. Res. Dev. 34, 1990: a quotient
-// within one ulp is corrected to the nearest; the first correction brings it there).
-// Outside the range that keeps every term normal, the division itself.
+// x / eps rounded to nearest, one divisor for many x of either sign (quotient_of); outside
+// the range that keeps every term normal, the division itself.
 struct OverEps {
   double eps, y;
   bool usable;
@@ -210,9 +208,7 @@ struct OverEps {
   __device__ __forceinline__ double operator()(double x) const {
     const double ax = fabs(x);
     if (usable && ax >= 0x1p-500 && ax <= 0x1p+500) {
-      double q = __dmul_rn(x, y);
-      q = __fma_rn(__fma_rn(-q, eps, x), y, q);
-      return __fma_rn(__fma_rn(-q, eps, x), y, q);
+      return quotient_of(x, eps, y);
     }
     return x / eps;
   }
