@@ -27,8 +27,8 @@ namespace {
 constexpr size_t kStageBytes = kTransferChunk * sizeof(double);
 constexpr size_t kDirectBelow = size_t(16) << 20;  // smaller copies go by one cudaMemcpy
 std::mutex g_stage_mutex;
-unsigned char* g_stage[2] = {nullptr, nullptr};  // two halves of one block
-int g_stage_device = -1;                         // where it was allocated
+void* g_stage[2] = {nullptr, nullptr};  // both or none
+int g_stage_device = -1;                // where they were allocated
 unsigned long long g_stage_context = 0;
 
 int copy_workers() {
@@ -53,8 +53,8 @@ void parallel_memcpy(void* dst, const void* src, size_t bytes, int workers) {
   for (std::thread& t : threads) t.join();
 }
 
-// Where the block was allocated, the context's id tells whether it is still there; on
-// another device, whether it is still page-locked.
+// Where the buffers were allocated, the context's id tells whether they are still there;
+// on another device, whether they are still page-locked.
 cudaError_t ensure_stage() {
   int device = 0;
   unsigned long long context = 0;
@@ -63,11 +63,15 @@ cudaError_t ensure_stage() {
   if (current_context(&context) != cudaSuccess) cudaGetLastError();  // the id stays 0
   if (g_stage[0] && (device == g_stage_device ? context == g_stage_context : host_is_pinned(g_stage[0])))
     return cudaSuccess;
-  void* p = nullptr;
+  void* p[2] = {nullptr, nullptr};
   g_stage[0] = g_stage[1] = nullptr;
-  if ((e = cudaMallocHost(&p, 2 * kStageBytes)) != cudaSuccess) return e;
-  g_stage[0] = static_cast<unsigned char*>(p);
-  g_stage[1] = g_stage[0] + kStageBytes;
+  if ((e = cudaMallocHost(&p[0], kStageBytes)) != cudaSuccess) return e;
+  if ((e = cudaMallocHost(&p[1], kStageBytes)) != cudaSuccess) {
+    cudaFreeHost(p[0]);
+    return e;
+  }
+  g_stage[0] = p[0];
+  g_stage[1] = p[1];
   g_stage_device = device;
   g_stage_context = context;
   return cudaSuccess;
