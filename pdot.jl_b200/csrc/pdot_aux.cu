@@ -52,8 +52,8 @@ __device__ __forceinline__ double scale_of(double dist, double sum) {
 // rounding streams the plan four times in and once out (40 B per entry: the row
 // sums, the column sums of the row-scaled plan, both sums of the scaled plan,
 // the write). With the scaled plans written back in place it was 80 B per entry
-// and 11 launches: 10000 x 10000 took 1.75 ms of device time on B200, now the
-// four passes take 0.64 ms of their 0.61 ms at the copy peak (measured below).
+// and 11 launches: 10000 x 10000 took 1.81 ms on B200, now 0.75 with seven launches,
+// where the five streams alone take 0.61 at the copy peak.
 //
 // CTA (p, c) of a summing pass covers panel p (kRoundRows rows) of column chunk c; a
 // warp takes whole columns of the panel, lane rows in R-wide loads, so a column
@@ -219,8 +219,10 @@ __global__ void __launch_bounds__(kAuxThreads)
 // maximum is taken from the points, nothing stored, and the cost is then written
 // once (8 B per entry); stored first, scanned and divided in place it took 32 B per
 // entry: 0.93 ms at 10000 x 10000 in three dimensions on B200, now 0.20: 39 us for the
-// maximum, 159 for the write, which is bound by FP64 issue (14 operations an entry; the
-// bytes alone would take 122).
+// maximum, 159 for the write, where a plain fill of the same bytes takes 116 to 120. The
+// write is bound by latency, not by a unit: the FP64 pipe, issue and DRAM are each busy
+// for half the time, and of the 13 cycles between two instructions of a warp 5 go to the
+// loads of a column's coordinates and 4 to the chain of its 14 FP64 operations.
 //
 // DIM 1..4 are compiled in, 0 is any dimension (coordinates from global memory).
 constexpr int kCostRows = 2;  // rows per thread of the write

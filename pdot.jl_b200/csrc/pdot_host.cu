@@ -72,7 +72,10 @@ void set_last_error(const char* msg) { g_last_error = msg ? msg : ""; }
 // use. (The device's default pool keeps nothing unless the program says so: a small
 // rounding after a synchronisation took 0.5 ms for its scratch.) While a stream is
 // captured the block belongs to the graph. When the pool cannot serve a block it is
-// trimmed and the block taken from cudaMalloc.
+// trimmed and the block taken from cudaMalloc; and what the pool keeps unused the driver
+// gives to any cudaMalloc that would fail without it (two blocks of 552 MB were had with
+// 498 MB free and 1 GB in the pool). The blocks of large solves, three of 800 MB at
+// 10000 x 10000, cost 1.3 ms to take and 2.4 to give back, of some 130.
 //
 // All of it goes with its context (cudaDeviceReset), so it is kept by the context's id,
 // which the driver gives out once in the life of a program, and another context gets

@@ -8,7 +8,7 @@
 // shared memory with the 128-byte swizzle, one thread issues tcgen05.mma
 // (M = 128, N = 128, K = 16 per instruction) into a TMEM accumulator, each
 // stage of the 4-deep ring is released by tcgen05.commit on its mbarrier, and
-// the four warps read the accumulator back with tcgen05.ld for a fused
+// the eight warps read the accumulator back with tcgen05.ld for a fused
 // epilogue (bias, GELU or the GELU derivative) that also writes the transposed
 // BF16 copy the backward products read. With every operand K-major:
 //
