@@ -1842,14 +1842,15 @@ class BatchSolver {
 
   void enqueue_chunk(long long& it) {
     if (regular_start(it)) {
-      if (persistent_) {
-        launch_persistent_chunk();
-      } else {
-        if (!graph_) capture();  // while the GPU runs the chunk before it
-        BCK(cudaGraphLaunch(graph_, stream_));
+      // (captured while the GPU runs the chunk before it)
+      if (persistent_ || graph_ || capture()) {
+        if (persistent_)
+          launch_persistent_chunk();
+        else
+          BCK(cudaGraphLaunch(graph_, stream_));
+        it += freq_;
+        return;
       }
-      it += freq_;
-      return;
     }
     long long k = 0;
     do {
@@ -1870,15 +1871,28 @@ class BatchSolver {
                                                        args, 0, stream_)));
   }
 
-  void capture() {
+  // False when the capture failed, by a device-wide synchronisation of another thread for
+  // one: the chunk is then launched kernel by kernel and the next one captured.
+  bool capture() {
     cudaGraph_t g = nullptr;
-    BCK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    launch_eval();
-    for (long long k = 0; k < freq_; ++k) launch_step();
-    BCK(cudaStreamEndCapture(stream_, &g));
-    const cudaError_t e = cudaGraphInstantiate(&graph_, g, 0);
-    cudaGraphDestroy(g);
-    BCK(e);
+    cudaError_t e = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+      try {
+        launch_eval();
+        for (long long k = 0; k < freq_; ++k) launch_step();
+      } catch (const BatchFailure&) {
+        e = cudaErrorStreamCaptureInvalidated;
+      }
+    }
+    const cudaError_t e2 = cudaStreamEndCapture(stream_, &g);
+    if (e == cudaSuccess) e = e2;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&graph_, g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      graph_ = nullptr;
+    }
+    return e == cudaSuccess;
   }
 
   void collect(pdot_batch_output* outs) {

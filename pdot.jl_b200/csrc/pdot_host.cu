@@ -956,16 +956,16 @@ class Solver {
       }
     }
     if (regular_start(host_it_) && budget >= freq_) {
-      if (persistent_) {
-        CK(pdot::launch_chunk(B_, g_, cfg_, stream_, (int)freq_));
-      } else {
-        // captured on first use, while the GPU runs the chunk before it: capture,
-        // instantiation and upload take 0.8 ms of host time
-        if (!graph_exec_) capture_regular_chunk();
-        CK(cudaGraphLaunch(graph_exec_, stream_));
+      // the graph is captured on first use, while the GPU runs the chunk before it:
+      // capture, instantiation and upload take 0.8 ms of host time
+      if (persistent_ || graph_exec_ || capture_regular_chunk()) {
+        if (persistent_)
+          CK(pdot::launch_chunk(B_, g_, cfg_, stream_, (int)freq_));
+        else
+          CK(cudaGraphLaunch(graph_exec_, stream_));
+        host_it_ += freq_;
+        return freq_;
       }
-      host_it_ += freq_;
-      return freq_;
     }
     int64_t k = 0;
     do {
@@ -1007,19 +1007,25 @@ class Solver {
     drain();
   }
 
-  void capture_regular_chunk() {
+  // False when the capture failed. A device-wide synchronisation by another thread is
+  // refused while any stream is captured, and spoils the capture: this chunk is then
+  // launched kernel by kernel (which reports any other cause) and the next one captured.
+  bool capture_regular_chunk() {
     cudaGraph_t graph = nullptr;
-    CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = pdot::launch_eval(B_, g_, cfg_, stream_);
+    cudaError_t e = cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) e = pdot::launch_eval(B_, g_, cfg_, stream_);
     // the chunk's last step precedes the next chunk's evaluation
     for (long long k = 0; k < freq_ && e == cudaSuccess; ++k)
       e = pdot::launch_step(B_, g_, cfg_, stream_, k == freq_ - 1 ? 1 : 0);
-    cudaError_t e2 = cudaStreamEndCapture(stream_, &graph);
-    CK(e);
-    CK(e2);
-    cudaError_t e3 = cudaGraphInstantiate(&graph_exec_, graph, 0);
-    cudaGraphDestroy(graph);
-    CK(e3);
+    const cudaError_t e2 = cudaStreamEndCapture(stream_, &graph);
+    if (e == cudaSuccess) e = e2;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&graph_exec_, graph, 0);
+    if (graph) cudaGraphDestroy(graph);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      graph_exec_ = nullptr;
+    }
+    return e == cudaSuccess;
   }
 
   void drain() {
